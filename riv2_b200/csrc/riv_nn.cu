@@ -1000,7 +1000,88 @@ __global__ void __launch_bounds__(PF_THREADS, 5) k_prop_input(const uint8_t* __r
 // Training kernels
 // =====================================================================================
 // im2col^T of a 3x3 convolution: out[k][m] (k = tap * cin + channel, m = MB * hout^2 + position)
-// for k < 9 * cin; rows 9 * cin .. kpad - 1 are zero.  One thread per (k, m) pair, m fastest.
+// for k < 9 * cin; rows 9 * cin .. kpad - 1 are zero.
+//
+// Bound by the bytes written (layer 2 at 4096 MBs: 94 MB).  Both forms below write 16 bytes (eight
+// positions of one row) per store, so they need M, the row length, to be a multiple of 8
+// (then every row starts on a 16-byte boundary); other M take the element form.
+struct Im2colShape {
+    int in_mb, nmb;
+    long long M;
+};
+// 32 input channels: a CTA takes 64 positions, and per tap stages their 64-byte input rows in
+// shared memory and writes them out as 32 rows of 128 bytes.  The tile's rows are 17 words
+// apart, so the column reads of a warp conflict at most two ways.  Layers 2 / 3 / 4 at 4096
+// MBs: 30 / 26 / 9 us; one thread per element (a 64-bit division and a 2-byte store each) took
+// 254 / 253 / 68 us.
+template <int HIN, int HOUT, int STRIDE>
+__global__ void __launch_bounds__(256) k_nn_im2col_t32(const __nv_bfloat16* __restrict__ in, Im2colShape s,
+                                                       __nv_bfloat16* __restrict__ out) {
+    __shared__ __align__(16) uint32_t tile[2][64 * 17];
+    const int t = threadIdx.x;
+    const long long m0 = (long long)blockIdx.x * 64;
+    // load: 16 bytes (8 channels) of one position per thread
+    const int lp = t >> 2, lc = t & 3;
+    const long long lm = m0 + lp;
+    const bool lv = lm < s.M;
+    const int b = lv ? (int)(lm / (HOUT * HOUT)) : 0, p = lv ? (int)(lm % (HOUT * HOUT)) : 0;
+    const int oy = p / HOUT * STRIDE - 1, ox = p % HOUT * STRIDE - 1;
+    const __nv_bfloat16* src = in + (size_t)b * s.in_mb + 8 * lc;
+    // store: 8 positions of one channel per thread
+    const int sc = t >> 3, sg = t & 7;
+    const bool sv = m0 + 8 * sg < s.M;
+    __nv_bfloat16* dst = out + (size_t)sc * s.M + m0 + 8 * sg;
+    auto load = [&](int tap) {
+        const int iy = oy + tap / 3, ix = ox + tap % 3;
+        return lv && iy >= 0 && iy < HIN && ix >= 0 && ix < HIN ? __ldg((const uint4*)(src + (iy * HIN + ix) * 32))
+                                                                : make_uint4(0u, 0u, 0u, 0u);
+    };
+    uint4 v = load(0);
+#pragma unroll
+    for (int tap = 0; tap < 9; tap++) {
+        uint32_t* T = tile[tap & 1];
+        uint32_t* w = T + lp * 17 + 4 * lc;
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        if (tap < 8) v = load(tap + 1);
+        __syncthreads();  // the other tile is rewritten only after the next barrier
+        if (sv) {
+            const uint16_t* h = (const uint16_t*)T + (size_t)(8 * sg) * 34 + sc;
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[j] = (uint32_t)h[68 * j] | ((uint32_t)h[68 * j + 34] << 16);
+            *(uint4*)(dst + (size_t)(32 * tap) * s.M) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+    if (sv) *(uint4*)(dst + (size_t)288 * s.M) = make_uint4(0u, 0u, 0u, 0u);  // rows 288 .. 319
+}
+// Two input channels (layer 1): a thread reads the words of eight positions at one tap and
+// writes both channels' 16 bytes; taps 9 .. 15 are the zero rows 18 .. 31.  15 us at 4096 MBs
+// against 78 us one element per thread.
+__global__ void __launch_bounds__(256) k_nn_im2col_t2(const __nv_bfloat16* __restrict__ in, Im2colShape s,
+                                                      __nv_bfloat16* __restrict__ out) {
+    constexpr int HIN = nn::FEAT, HOUT = 12;
+    const long long m0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    const int tap = blockIdx.y;
+    if (m0 >= s.M) return;
+    uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (tap < 9) {
+        int b = (int)(m0 / (HOUT * HOUT)), p = (int)(m0 % (HOUT * HOUT));  // a multiple of 8: one MB (144 = 18 * 8)
+#pragma unroll
+        for (int j = 0; j < 8; j++, p++) {
+            const int iy = p / HOUT * 2 + tap / 3 - 1, ix = p % HOUT * 2 + tap % 3 - 1;
+            if (iy >= 0 && iy < HIN && ix >= 0 && ix < HIN)
+                w[j] = __ldg((const uint32_t*)(in + (size_t)b * s.in_mb) + iy * HIN + ix);
+        }
+    }
+    uint4 a, c;
+    a.x = __byte_perm(w[0], w[1], 0x5410); a.y = __byte_perm(w[2], w[3], 0x5410);
+    a.z = __byte_perm(w[4], w[5], 0x5410); a.w = __byte_perm(w[6], w[7], 0x5410);
+    c.x = __byte_perm(w[0], w[1], 0x7632); c.y = __byte_perm(w[2], w[3], 0x7632);
+    c.z = __byte_perm(w[4], w[5], 0x7632); c.w = __byte_perm(w[6], w[7], 0x7632);
+    *(uint4*)(out + (size_t)(2 * tap) * s.M + m0) = a;
+    *(uint4*)(out + (size_t)(2 * tap + 1) * s.M + m0) = c;
+}
+// Any M: one thread per (k, m) pair, m fastest.
 __global__ void k_nn_im2col_t(const __nv_bfloat16* __restrict__ in, int in_mb, int cin, int hin, int hout, int stride,
                               int nmb, int kpad, __nv_bfloat16* __restrict__ out) {
     const long long M = (long long)nmb * hout * hout;
@@ -1019,49 +1100,106 @@ __global__ void k_nn_im2col_t(const __nv_bfloat16* __restrict__ in, int in_mb, i
     }
 }
 
-// col2im of the input gradient of a 3x3 convolution (dcol: [m][kpad] f32, k = tap * 32 + channel),
+// A 64-row x 32-column tile of bf16 gradients (row stride 17 words in shared memory) to dzt:
+// column c0 + c, rows r0 .. r0 + 63 of `rows`.  16-byte stores where every column starts on a
+// 16-byte boundary, elements otherwise.  256 threads, after a barrier.
+__device__ __forceinline__ void store_dzt(const uint32_t* tile, __nv_bfloat16* __restrict__ dzt, int c0, long long r0,
+                                          long long rows) {
+    const int c = threadIdx.x >> 3, g = threadIdx.x & 7;
+    const uint16_t* h = (const uint16_t*)tile + (size_t)(8 * g) * 34 + c;
+    uint16_t* dst = (uint16_t*)dzt + (size_t)(c0 + c) * rows + r0 + 8 * g;
+    if ((rows & 7) == 0 && ((uintptr_t)dzt & 15) == 0) {
+        if (r0 + 8 * g >= rows) return;
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) o[j] = (uint32_t)h[68 * j] | ((uint32_t)h[68 * j + 34] << 16);
+        *(uint4*)dst = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (r0 + 8 * g + j < rows) dst[j] = h[34 * j];
+    }
+}
+
+// col2im of the input gradient of a 3x3 convolution (dcol: [m][KC] f32, k = tap * 32 + channel),
 // times the ReLU derivative of the input activation (act, NHWC bf16 with per-MB stride act_mb),
 // written as bf16 in two layouts: dz[mi][32] (mi = MB * hin^2 + position) and dzt[32][Mi].
-__global__ void k_nn_col2im(const float* __restrict__ dcol, int kpad, int hin, int hout, int stride, int nmb,
-                            const __nv_bfloat16* __restrict__ act, int act_mb, __nv_bfloat16* __restrict__ dz,
-                            __nv_bfloat16* __restrict__ dzt) {
-    const long long Mi = (long long)nmb * hin * hin;
-    const long long n = Mi * 32;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
-        const long long mi = idx >> 5;
-        const int c = (int)(idx & 31);
-        const int b = (int)(mi / (hin * hin)), p = (int)(mi % (hin * hin));
-        const int iy = p / hin, ix = p % hin;
-        float g = 0.0f;
+// Bound by dcol (layer 2 at 4096 MBs: 170 MB read once).  A CTA takes 64 input positions, a
+// thread four channels of two of them (16-byte loads where VEC: aligned buffers; the taps summed
+// in tap order), and the transposed layout leaves through a shared tile.  Layers 2 / 3 / 4 at 4096 MBs: 56 / 28 / 17 us;
+// one thread per element, its transposed value stored on its own, took 349 / 133 / 86 us.
+template <int HIN, int HOUT, int STRIDE, bool VEC>
+__global__ void __launch_bounds__(256) k_nn_col2im(const float* __restrict__ dcol, int nmb,
+                                                   const __nv_bfloat16* __restrict__ act, int act_mb,
+                                                   __nv_bfloat16* __restrict__ dz, __nv_bfloat16* __restrict__ dzt) {
+    __shared__ __align__(16) uint32_t tile[64 * 17];
+    const long long Mi = (long long)nmb * (HIN * HIN), r0 = (long long)blockIdx.x * 64;
+    const int c = 4 * (threadIdx.x & 7);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int q = (threadIdx.x >> 3) + 32 * h;
+        const long long mi = r0 + q;
+        if (mi >= Mi) continue;
+        const int b = (int)(mi / (HIN * HIN)), p = (int)(mi % (HIN * HIN));
+        const int iy = p / HIN, ix = p % HIN;
+        float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
         for (int tap = 0; tap < 9; tap++) {
-            const int ny = iy + 1 - tap / 3, nx = ix + 1 - tap % 3;  // = o * stride
-            if (ny < 0 || nx < 0 || ny % stride || nx % stride) continue;
-            const int oy = ny / stride, ox = nx / stride;
-            if (oy >= hout || ox >= hout) continue;
-            const long long m = (long long)b * hout * hout + oy * hout + ox;
-            g += dcol[m * kpad + tap * 32 + c];
+            const int ny = iy + 1 - tap / 3, nx = ix + 1 - tap % 3;  // = o * STRIDE
+            if (ny < 0 || nx < 0 || ny % STRIDE || nx % STRIDE) continue;
+            const int oy = ny / STRIDE, ox = nx / STRIDE;
+            if (oy >= HOUT || ox >= HOUT) continue;
+            const long long m = (long long)b * (HOUT * HOUT) + oy * HOUT + ox;
+            const float* dp = dcol + m * nn::KC + tap * 32 + c;
+            const float4 v = VEC ? __ldcs((const float4*)dp) : make_float4(dp[0], dp[1], dp[2], dp[3]);
+            g.x += v.x; g.y += v.y; g.z += v.z; g.w += v.w;
         }
-        const float a = __bfloat162float(act[(size_t)b * act_mb + (size_t)p * 32 + c]);
-        const float d = a > 0.0f ? g : 0.0f;
-        dz[idx] = __float2bfloat16_rn(d);
-        dzt[(size_t)c * Mi + mi] = __float2bfloat16_rn(d);
+        const __nv_bfloat16* ap = act + (size_t)b * act_mb + (size_t)p * 32 + c;
+        __align__(8) __nv_bfloat16 a[4];
+        if (VEC) *(uint2*)a = *(const uint2*)ap;
+        else a[0] = ap[0], a[1] = ap[1], a[2] = ap[2], a[3] = ap[3];
+        const uint32_t d0 = pack_bf16(__bfloat162float(a[0]) > 0.0f ? g.x : 0.0f, __bfloat162float(a[1]) > 0.0f ? g.y : 0.0f);
+        const uint32_t d1 = pack_bf16(__bfloat162float(a[2]) > 0.0f ? g.z : 0.0f, __bfloat162float(a[3]) > 0.0f ? g.w : 0.0f);
+        if (VEC) {
+            *(uint2*)(dz + mi * 32 + c) = make_uint2(d0, d1);
+        } else {
+            uint16_t* zp = (uint16_t*)(dz + mi * 32 + c);
+            zp[0] = (uint16_t)d0; zp[1] = (uint16_t)(d0 >> 16); zp[2] = (uint16_t)d1; zp[3] = (uint16_t)(d1 >> 16);
+        }
+        tile[q * 17 + (c >> 1)] = d0;
+        tile[q * 17 + (c >> 1) + 1] = d1;
     }
+    __syncthreads();
+    store_dzt(tile, dzt, 0, r0, Mi);
 }
 
 // ReLU derivative of a layer's output: d (f32) times (act > 0) (act bf16), as bf16 rows x n (dz)
 // and n x rows (dzt).  Rows come in groups of grp: row r, column c lies at
 // (r / grp) * ld + (r % grp) * n + c, with ld = ldd for d and lda for act (grp = 1: plain rows).
-__global__ void k_nn_relu_bwd(const float* __restrict__ d, int ldd, const __nv_bfloat16* __restrict__ act, int lda,
-                              int rows, int n, int grp, __nv_bfloat16* __restrict__ dz, __nv_bfloat16* __restrict__ dzt) {
-    const long long total = (long long)rows * n;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(idx / n), c = (int)(idx % n);
-        const int g = r / grp, q = r - g * grp;
-        const float a = __bfloat162float(act[(size_t)g * lda + (size_t)q * n + c]);
-        const float v = a > 0.0f ? d[(size_t)g * ldd + (size_t)q * n + c] : 0.0f;
-        dz[idx] = __float2bfloat16_rn(v);
-        dzt[(size_t)c * rows + r] = __float2bfloat16_rn(v);
+// A CTA takes 64 rows x 32 columns; the transposed layout leaves through a shared tile (stored
+// per element: 18 us at 36864 x 32, now 12; 11 us at 4096 x 128 either way).
+__global__ void __launch_bounds__(256) k_nn_relu_bwd(const float* __restrict__ d, int ldd,
+                                                     const __nv_bfloat16* __restrict__ act, int lda, int rows, int n,
+                                                     int grp, __nv_bfloat16* __restrict__ dz,
+                                                     __nv_bfloat16* __restrict__ dzt) {
+    __shared__ __align__(16) uint32_t tile[64 * 17];
+    const int r0 = (int)blockIdx.x * 64;
+    const int c0 = blockIdx.y * 32, lane = threadIdx.x & 31;
+    const int c = c0 + lane;
+    uint16_t* th = (uint16_t*)tile;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int q = (threadIdx.x >> 5) + 8 * j;
+        const int r = r0 + q;
+        if (q >= rows - r0 || c >= n) continue;
+        const int g = r / grp, k = r - g * grp;
+        const float a = __bfloat162float(act[(size_t)g * lda + (size_t)k * n + c]);
+        const __nv_bfloat16 v = __float2bfloat16_rn(a > 0.0f ? d[(size_t)g * ldd + (size_t)k * n + c] : 0.0f);
+        dz[(size_t)r * n + c] = v;
+        th[q * 34 + lane] = __bfloat16_as_ushort(v);
     }
+    __syncthreads();
+    if (c0 + (int)(threadIdx.x >> 3) < n) store_dzt(tile, dzt, c0, r0, rows);
 }
 
 // bf16 transpose: in rows x cols (pitch ld) -> out cols x rows.
@@ -1081,13 +1219,49 @@ __global__ void k_nn_transpose(const __nv_bfloat16* __restrict__ in, int ld, int
     }
 }
 
-// Column sums of a bf16 matrix (rows x n, pitch ld) added into out[n] (bias gradients).
-__global__ void k_nn_colsum(const __nv_bfloat16* __restrict__ z, int ld, long long rows, int n, float* __restrict__ out) {
-    const int c = threadIdx.x % n, lanes = blockDim.x / n;
-    float acc = 0.0f;
-    for (long long r = (long long)blockIdx.x * lanes + threadIdx.x / n; r < rows; r += (long long)gridDim.x * lanes)
-        acc += __bfloat162float(z[r * ld + c]);
-    if ((int)threadIdx.x < lanes * n) atomicAdd(out + c, acc);
+// Column sums of a bf16 matrix (rows x n, pitch ld) added into out[n] (bias gradients).  A thread
+// sums V adjacent columns over its share of the rows, the CTA's threads of a column are summed in
+// shared memory, and each CTA adds one value per column: the adds to the same n words, not the
+// rows read, bounded the form in which every thread added its own sum (80-88 us at
+// 589,824 x 32, 20 us at 4096 x 128).  V = 8 (16-byte loads) where n, the pitch and the address
+// allow it, else 1.
+template <int V>
+__global__ void __launch_bounds__(256) k_nn_colsum(const __nv_bfloat16* __restrict__ z, int ld, long long rows, int n,
+                                                   float* __restrict__ out) {
+    __shared__ float part[256 * V];
+    const int nv = n / V, c = (int)threadIdx.x % nv, lanes = (int)blockDim.x / nv, l = (int)threadIdx.x / nv;
+    float acc[2][V];
+#pragma unroll
+    for (int k = 0; k < V; k++) acc[0][k] = acc[1][k] = 0.0f;
+    auto add = [&](float (&a)[V], long long r) {
+        const __nv_bfloat16* p = z + r * ld + (long long)c * V;
+        if constexpr (V == 8) {
+            const uint4 w = *(const uint4*)p;
+            const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                a[2 * k] += __uint_as_float(u[k] << 16);
+                a[2 * k + 1] += __uint_as_float(u[k] & 0xffff0000u);
+            }
+        } else {
+            a[0] += __bfloat162float(*p);
+        }
+    };
+    const long long step = (long long)gridDim.x * lanes;
+    long long r = (long long)blockIdx.x * lanes + l;
+    for (; r + step < rows; r += 2 * step) {
+        add(acc[0], r);
+        add(acc[1], r + step);
+    }
+    if (r < rows) add(acc[0], r);
+#pragma unroll
+    for (int k = 0; k < V; k++) part[(l * nv + c) * V + k] = acc[0][k] + acc[1][k];
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        float v = 0.0f;
+        for (int q = 0; q < lanes; q++) v += part[q * n + j];
+        atomicAdd(out + j, v);
+    }
 }
 
 // Loss of the head and its gradient.  o: rows x 16 f32 (fc3 output); target MV (half-pel) and
@@ -1205,29 +1379,53 @@ int riv_nn_front(const uint8_t* cur_y, const uint8_t* ref_y, int W, int H, const
 int riv_nn_im2col_t(int layer, const void* in, int in_mb, int nmb, void* out, void* stream) {
     static const int HIN[5] = {0, 24, 12, 6, 6}, HOUT[5] = {0, 12, 6, 6, 3}, STRIDE[5] = {0, 2, 2, 1, 2};
     if (layer < 1 || layer > 4 || nmb <= 0) return (int)cudaErrorInvalidValue;
-    const int cin = layer == 1 ? 2 : 32, kpad = layer == 1 ? nn::K1 : nn::KC;
-    const long long n = (long long)nmb * HOUT[layer] * HOUT[layer] * kpad;
-    k_nn_im2col_t<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, in_mb, cin, HIN[layer],
-                                                                 HOUT[layer], STRIDE[layer], nmb, kpad,
-                                                                 (__nv_bfloat16*)out);
+    const cudaStream_t st = (cudaStream_t)stream;
+    const __nv_bfloat16* x = (const __nv_bfloat16*)in;
+    __nv_bfloat16* o = (__nv_bfloat16*)out;
+    const Im2colShape s{in_mb, nmb, (long long)nmb * HOUT[layer] * HOUT[layer]};
+    // 16-byte stores need rows that start on 16-byte boundaries, the loads an input of 4-byte
+    // (layer 1) or 16-byte aligned pixels
+    const uintptr_t al = layer == 1 ? 3 : 15;
+    const bool vec = s.M % 8 == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)in & al) == 0 &&
+                     ((uintptr_t)(2 * (long long)in_mb) & al) == 0;
+    if (vec) {
+        const unsigned g = (unsigned)((s.M + 63) / 64);
+        if (layer == 1) k_nn_im2col_t2<<<dim3((unsigned)((s.M / 8 + 255) / 256), 16), 256, 0, st>>>(x, s, o);
+        else if (layer == 2) k_nn_im2col_t32<12, 6, 2><<<g, 256, 0, st>>>(x, s, o);
+        else if (layer == 3) k_nn_im2col_t32<6, 6, 1><<<g, 256, 0, st>>>(x, s, o);
+        else k_nn_im2col_t32<6, 3, 2><<<g, 256, 0, st>>>(x, s, o);
+    } else {
+        const int cin = layer == 1 ? 2 : 32, kpad = layer == 1 ? nn::K1 : nn::KC;
+        k_nn_im2col_t<<<grid_for(s.M * kpad), 256, 0, st>>>(x, in_mb, cin, HIN[layer], HOUT[layer], STRIDE[layer], nmb, kpad,
+                                                            o);
+    }
     return (int)cudaGetLastError();
 }
 
 int riv_nn_col2im(int layer, const float* dcol, int nmb, const void* act, int act_mb, void* dz, void* dzt,
                   void* stream) {
-    static const int HIN[5] = {0, 24, 12, 6, 6}, HOUT[5] = {0, 12, 6, 6, 3}, STRIDE[5] = {0, 2, 2, 1, 2};
+    static const int HIN[5] = {0, 24, 12, 6, 6};
     if (layer < 2 || layer > 4 || nmb <= 0) return (int)cudaErrorInvalidValue;
-    const long long n = (long long)nmb * HIN[layer] * HIN[layer] * 32;
-    k_nn_col2im<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(dcol, nn::KC, HIN[layer], HOUT[layer], STRIDE[layer], nmb,
-                                                               (const __nv_bfloat16*)act, act_mb, (__nv_bfloat16*)dz,
-                                                               (__nv_bfloat16*)dzt);
+    const cudaStream_t st = (cudaStream_t)stream;
+    const __nv_bfloat16* a = (const __nv_bfloat16*)act;
+    __nv_bfloat16 *z = (__nv_bfloat16*)dz, *zt = (__nv_bfloat16*)dzt;
+    const unsigned g = (unsigned)(((long long)nmb * HIN[layer] * HIN[layer] + 63) / 64);
+    const bool vec = (((uintptr_t)dcol & 15) | ((uintptr_t)act & 7) | ((uintptr_t)(2 * (long long)act_mb) & 7) |
+                      ((uintptr_t)dz & 7)) == 0;
+#define RIV_COL2IM(HIN, HOUT, STRIDE)                                                                     \
+    (vec ? k_nn_col2im<HIN, HOUT, STRIDE, true> : k_nn_col2im<HIN, HOUT, STRIDE, false>)<<<g, 256, 0, st>>>( \
+        dcol, nmb, a, act_mb, z, zt)
+    if (layer == 2) RIV_COL2IM(12, 6, 2);
+    else if (layer == 3) RIV_COL2IM(6, 6, 1);
+    else RIV_COL2IM(6, 3, 2);
+#undef RIV_COL2IM
     return (int)cudaGetLastError();
 }
 
 int riv_nn_relu_bwd(const float* d, int ldd, const void* act, int lda, int rows, int n, int grp, void* dz, void* dzt,
                     void* stream) {
     if (grp < 1 || n <= 0 || rows <= 0) return (int)cudaErrorInvalidValue;
-    k_nn_relu_bwd<<<grid_for((long long)rows * n), 256, 0, (cudaStream_t)stream>>>(
+    k_nn_relu_bwd<<<dim3((unsigned)((rows + 63) / 64), (unsigned)((n + 31) / 32)), 256, 0, (cudaStream_t)stream>>>(
         d, ldd, (const __nv_bfloat16*)act, lda, rows, n, grp, (__nv_bfloat16*)dz, (__nv_bfloat16*)dzt);
     return (int)cudaGetLastError();
 }
@@ -1241,8 +1439,13 @@ int riv_nn_transpose(const void* in, int ld, int rows, int cols, void* out, void
 
 int riv_nn_colsum(const void* z, int ld, long long rows, int n, float* out, void* stream) {
     if (n <= 0 || n > 256) return (int)cudaErrorInvalidValue;
-    const int per = 256 / n * n;
-    k_nn_colsum<<<grid_for(rows, per / n), per, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)z, ld, rows, n, out);
+    const bool vec = n % 8 == 0 && ld % 8 == 0 && ((uintptr_t)z & 15) == 0;
+    const int nv = vec ? n / 8 : n, lanes = 256 / nv, per = lanes * nv;
+    // at least 8 rows a thread, at most two CTAs per SM: each CTA ends with n adds to the same n words
+    const long long want = (rows + 8 * lanes - 1) / (8 * lanes);
+    const unsigned g = (unsigned)(want < 1 ? 1 : want < 2 * 148 ? want : 2 * 148);
+    if (vec) k_nn_colsum<8><<<g, per, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)z, ld, rows, n, out);
+    else k_nn_colsum<1><<<g, per, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)z, ld, rows, n, out);
     return (int)cudaGetLastError();
 }
 

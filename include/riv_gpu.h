@@ -307,6 +307,13 @@ void riv_dct_tables(int32_t* t16, int32_t* t8);
  * encoder panics (a magnitude class above 13). */
 riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uint32_t threads, uint8_t* out, size_t cap,
                                size_t* len);
+/* Test hook (no reference counterpart): the coefficient stream as the encoder makes it, with the
+ * symbols and models on the GPU and the rANS batches on the host, of n > 0 dense blocks; P-frames
+ * (intra == 0): blocks with skip[b] != 0 are not coded.  max_symbols: what the GPU's stacks hold
+ * (0: as an encoder's).  *on_gpu = 0 when the frame went to the host coder instead (more symbols,
+ * or a class it refuses: RIV_ERR_ENCODING_FAILED). */
+riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, uint32_t n, int intra, uint32_t max_symbols,
+                                   uint8_t* out, size_t cap, size_t* len, int* on_gpu);
 /* Test hook (host only, no reference counterpart): the decoder's DCT-coefficient decoder on one
  * frame's coefficient stream; n blocks of 384 i16 out, blocks with coded[b] == 0 are not in the
  * stream and stay zero; DC prediction when intra.  RIV_OK, or RIV_ERR_FRAME where the stream is

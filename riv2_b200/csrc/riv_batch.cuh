@@ -28,8 +28,8 @@ __host__ __device__ inline int batch_deblock_tiles(int W, int H, int tw) {
     return ty + 2 * tc;
 }
 
-// CTAs of clip k in stage s (host and device agree through this one function).
-__host__ __device__ inline int batch_ctas(int s, const BatchClip& k, const BatchTune& t) {
+// CTAs of clip k in stage s.
+inline int batch_ctas(int s, const BatchClip& k, const BatchTune& t) {
     const int nmb = k.NMB;
     switch (s) {
         case BS_CONVERT: return k.rgb != nullptr ? ((k.W / 2) * (k.H / 2) + 127) / 128 : 0;
@@ -38,8 +38,7 @@ __host__ __device__ inline int batch_ctas(int s, const BatchClip& k, const Batch
         case BS_AQSUM: return k.intra ? 0 : 1;
         case BS_RESIDUAL: return (nmb + t.res_mbs - 1) / t.res_mbs;
         case BS_DEBLOCK: return k.db_level > 0 ? batch_deblock_tiles(k.W, k.H, t.db_tw) : 0;
-        case BS_SCAN: return 1;
-        case BS_PACK: return (nmb + 7) / 8;
+        case BS_SCAN: case BS_PACK: return sym_part_ctas(nmb);
         default: return 0;
     }
 }
@@ -129,24 +128,31 @@ __global__ void __launch_bounds__(128) kb_deblock(BatchLaunch b) {
                      blockDim.x, 0);
 }
 
-// ---- compaction: the scan (one CTA per clip; it also copies the clip's status word to the
-// mapped header, so no separate copy is needed), then one warp per MB
-__global__ void __launch_bounds__(SC_THREADS) kb_scan(BatchLaunch b) {
-    __shared__ int wsum[SC_THREADS / 32], wsz[SC_THREADS / 32];
+// ---- coefficient symbols (riv_symbols.cuh): counts and their scan (which also copies the clip's
+// status word to the mapped header, so no separate copy is needed), then symbols and models
+__global__ void __launch_bounds__(32 * SY_WARPS, 4) kb_sym_count(BatchLaunch b) {
+    __shared__ unsigned h[SY_WARPS][SYM_ROWS];
     const int* st = b.start + BS_SCAN * (b.nclips + 1);
-    const BatchClip& k = b.clips[batch_clip(st, b.nclips, blockIdx.x)];
-    scan_mbs<SC_THREADS, SC_IPT>(k.rp.opt_skip, k.rp.eobs, k.NMB, k.intra, k.c_index, k.c_offset, k.c_hdr, threadIdx.x,
-                                 1, wsum, wsz);
-    if (threadIdx.x == 0) k.c_hdr[2] = *(volatile const unsigned*)k.status;
+    const int c = batch_clip(st, b.nclips, blockIdx.x);
+    sym_count_cta(b.clips[c].sym, (int)blockIdx.x - st[c], h);
 }
-__global__ void __launch_bounds__(256) kb_pack(BatchLaunch b) {
+__global__ void __launch_bounds__(1024) kb_sym_scan(BatchLaunch b) {
+    sym_scan_rows(b.clips[blockIdx.y].sym, blockIdx.x);
+}
+__global__ void __launch_bounds__(32 * SY_WARPS, 4) kb_sym_emit(BatchLaunch b) {
+    __shared__ unsigned h[SY_WARPS][SYM_ROWS];
     const int* st = b.start + BS_PACK * (b.nclips + 1);
     const int c = batch_clip(st, b.nclips, blockIdx.x);
-    const BatchClip& k = b.clips[c];
-    const int m = ((int)blockIdx.x - st[c]) * 8 + (threadIdx.x >> 5);
-    if (m < k.NMB)
-        pack_mb(m, threadIdx.x & 31, k.rp.opt_skip, k.rp.mb, k.rp.coeffs, k.rp.eobs, k.c_index, k.c_offset, k.intra,
-                k.c_side, k.c_packed, k.c_peobs);
+    sym_emit_cta(b.clips[c].sym, (int)blockIdx.x - st[c], h);
+}
+__global__ void __launch_bounds__(SY_CHAIN_THREADS) kb_sym_chain(BatchLaunch b) {
+    const SymFrame& f = b.clips[blockIdx.y].sym;
+    if (f.work[1] != 0u) sym_chain_cta(f, blockIdx.x);
+}
+constexpr int BATCH_MODEL_CTAS = 64;  // per clip; its warps share the clip's units
+__global__ void __launch_bounds__(SY_MODEL_THREADS, 8) kb_sym_model(BatchLaunch b) {
+    sym_model_units(b.clips[blockIdx.y].sym, (blockIdx.x * SY_MODEL_THREADS + threadIdx.x) >> 5,
+                    BATCH_MODEL_CTAS * (SY_MODEL_THREADS / 32), threadIdx.x & 31);
 }
 
 // ---- the multi-clip search wavefront (per-MB reference windows; see the file comment)
@@ -171,10 +177,10 @@ static size_t batch_stage_smem(int s, int max_sr) {
 static int batch_stage_threads(int s, const BatchTune& t) {
     switch (s) {
         case BS_CONVERT: case BS_TABLE: case BS_DEBLOCK: return 128;
-        case BS_PREDICT: case BS_PACK: return 256;
+        case BS_PREDICT: return 256;
         case BS_AQSUM: return 1024;
         case BS_RESIDUAL: return 64 * t.res_mbs;
-        case BS_SCAN: return SC_THREADS;
+        case BS_SCAN: case BS_PACK: return 32 * SY_WARPS;
         default: return 0;
     }
 }
@@ -209,8 +215,15 @@ int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int tota
             else if (t.db_tw == 256) kb_deblock<256><<<total, nt, 0, st>>>(b);
             else return (int)cudaErrorInvalidValue;
             break;
-        case BS_SCAN: kb_scan<<<total, nt, 0, st>>>(b); break;
-        case BS_PACK: kb_pack<<<total, nt, 0, st>>>(b); break;
+        case BS_SCAN:
+            kb_sym_count<<<total, nt, 0, st>>>(b);
+            kb_sym_scan<<<dim3(SYM_ROWS / 32, b.nclips), 1024, 0, st>>>(b);
+            break;
+        case BS_PACK:
+            kb_sym_emit<<<total, nt, 0, st>>>(b);
+            kb_sym_chain<<<dim3(SY_MODELS, b.nclips), SY_CHAIN_THREADS, 0, st>>>(b);
+            kb_sym_model<<<dim3(BATCH_MODEL_CTAS, b.nclips), SY_MODEL_THREADS, 0, st>>>(b);
+            break;
         default: return (int)cudaErrorInvalidValue;
     }
     return (int)cudaGetLastError();

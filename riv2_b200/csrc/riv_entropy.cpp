@@ -179,6 +179,28 @@ bool RansWriter::ready() {
     return true;
 }
 
+std::unique_ptr<RansWriter> RansWriter::over_stacks(const uint16_t* stacks, size_t n, std::vector<uint8_t>* sink,
+                                                    const BatchSubmit& submit) {
+    std::unique_ptr<RansWriter> w(new RansWriter());
+    w->sink_ = sink;
+    const size_t nb = (n + BATCH - 1) / BATCH;
+    for (size_t k = 0; k < nb; k++) {
+        w->batches_.emplace_back();
+        Batch& b = w->batches_.back();
+        const uint16_t* st = stacks + k * BATCH;
+        b.sp = k + 1 < nb ? 0 : (int)(nb * BATCH - n);
+        std::packaged_task<void()> here;
+        if (k + 1 < nb) {
+            b.done = submit([&b, st] { code_batch(st, b.sp, b.bytes); });
+        } else {
+            here = std::packaged_task<void()>([&b, st] { code_batch(st, b.sp, b.bytes); });
+            b.done = here.get_future();
+            here();
+        }
+    }
+    return w;
+}
+
 void RansWriter::collect() {
     for (Batch& b : batches_) {
         b.done.get();
@@ -537,6 +559,13 @@ void encode_residual_frame(const int16_t* packed, const uint8_t* eobs, int nbloc
     sink.finish();
     if (sink.bad) throw std::runtime_error(MAG_CLASS_ERROR);
     w.finish();
+}
+
+std::unique_ptr<RansWriter> encode_stacks_async(const uint16_t* stacks, size_t n, std::vector<uint8_t>& out,
+                                                const BatchSubmit& submit) {
+    out.clear();
+    if (n == 0) return nullptr;  // no coded block: the reference never instantiates the coder
+    return RansWriter::over_stacks(stacks, n, &out, submit);
 }
 
 std::unique_ptr<RansWriter> encode_residual_frame_async(const int16_t* packed, const uint8_t* eobs, int nblocks,

@@ -42,6 +42,11 @@ public:
     void finish_async();
     void collect();
     bool ready();  // every handed-off batch coded (collect() would not wait)
+    // A writer over n symbols whose (probability, bit) stacks exist already, batch after batch in
+    // this writer's layout (they must outlive it): all batches but the last go to submit, the
+    // last is coded here; collect() appends their words.
+    static std::unique_ptr<RansWriter> over_stacks(const uint16_t* stacks, size_t n, std::vector<uint8_t>* sink,
+                                                   const BatchSubmit& submit);
 
     // The stack in a caller's registers, for symbol loops: start from stack() and depth(),
     // push downwards (stack()[--depth] = entry), call refill() at depth 0 (it hands the full
@@ -56,10 +61,11 @@ public:
 private:
     // out of line and cold: inlined into put it costs the symbol loop its registers
     __attribute__((noinline, cold)) void drain();
-    std::vector<uint8_t>* sink_;
+    RansWriter() = default;
+    std::vector<uint8_t>* sink_ = nullptr;
     std::vector<uint16_t> stack_;  // entry = p | bit << 8; stack_[BATCH-1] is the oldest
-    int sp_;
-    const BatchSubmit* submit_;
+    int sp_ = 0;
+    const BatchSubmit* submit_ = nullptr;
     struct Batch {
         std::vector<uint16_t> stack;
         int sp = 0;
@@ -102,6 +108,10 @@ bool decode_residual_frame(const uint8_t* data, size_t len, const uint8_t* coded
 // Throws std::runtime_error where the reference encoder panics (a magnitude class above 13).
 void encode_residual_frame(const int16_t* packed, const uint8_t* eobs, int nblocks, bool intra,
                            std::vector<uint8_t>& out, const BatchSubmit* submit = nullptr, int parts = 0);
+// The rANS half alone, over the stacks the GPU made of a frame's n symbols (nullptr: n = 0, out
+// empty): the returned writer's collect() appends the bytes to out.
+std::unique_ptr<RansWriter> encode_stacks_async(const uint16_t* stacks, size_t n, std::vector<uint8_t>& out,
+                                                const BatchSubmit& submit);
 // The one-thread form of encode_residual_frame with every rANS batch, the last one included,
 // handed to submit: the returned writer's collect() appends the bytes to out (nullptr: no coded
 // block, out empty).  The modelling thread does not wait for the batches.

@@ -329,10 +329,11 @@ enum { EV_START, EV_YUV, EV_S0, EV_TABLE, EV_SEARCH, EV_PRED, EV_AQ, EV_RES, EV_
 static const int NSTAGE = 8;  // rgb->yuv, table, search, predict, aq, residual, deblock, compact (+ total)
 
 struct Slot {
-    DevBuf rgb, dside, dpacked, dpeobs;        // compacted frame output on the device
+    // frame output on the device; dpacked: rANS stacks, or truncated coefficient blocks
+    DevBuf rgb, dside, dpacked, dpeobs;
     HostBuf side, packed, peobs;               // pinned copies (DMA on the copy stream)
-    MappedBuf hdr;                             // coded MBs, coefficients, device status
-    size_t prefetched = 0;                     // coefficient bytes included in the first copy
+    MappedBuf hdr;                             // coded MBs, coefficients, device status, symbols
+    size_t prefetched = 0;                     // bytes of dpacked included in the first copy
     cudaEvent_t ev_h2d = nullptr, ev_gpu = nullptr, ev_d2h = nullptr;
     cudaEvent_t ev_k[EV_N] = {};  // stage timing (recorded on timed frames only)
     cudaEvent_t ev_yuv = nullptr, ev_recon = nullptr;  // dependencies: input converted / reconstruction done
@@ -353,9 +354,11 @@ struct Job {
     bool want_stats = false, prev_valid = false;
     int prev_buf = 0;
     int ck = 0;             // double-buffer parity of the frame's buffers
+    bool sym = false;       // its symbols were made on the GPU (riv_symbols.cuh)
     uint32_t count = 0;
     std::future<void> fut, fut_mv, fut_prep, fut_asm;
     std::vector<uint8_t> res_bytes, mv_bytes;
+    std::vector<uint16_t> big_stacks;     // rANS stacks that the slot's pinned buffer does not hold
     std::vector<MvCodedBlock> mv_blocks;  // the P-frame's MV coder input
     // host timeline (milliseconds, steady clock), kept when the encoder traces: submitted; MV
     // input assembly started / done; MV listing started / done; MV coding started / done; DCT
@@ -382,6 +385,9 @@ struct riv_encoder {
     size_t yuv_bytes = 0;
     cudaStream_t S = nullptr, C = nullptr, Hs = nullptr;  // main chain, device->host, host->device
     cudaStream_t Y = nullptr, K = nullptr;                // input conversion, compaction
+    // what a frame's first copy left out, copied once the frame is done: on C it would wait for
+    // the copies of every later frame in flight
+    cudaStream_t R = nullptr;
     // cross-stream reuse guards: cur[k] free (its residual is done), mbout[k] and the
     // coefficient buffers free (their compaction is done)
     cudaEvent_t ev_cur_free[NPAR] = {}, ev_mbout_free[NPAR] = {}, ev_coef_free[NPAR] = {};
@@ -403,8 +409,10 @@ struct riv_encoder {
     // device state
     DevBuf curb[NPAR], ref[2], recon_pre, predb[NPAR], mboutb[NPAR], coded[2], rec, varsum, lnvb[NPAR], qs, coeffsb[NPAR], optskipb[NPAR],
         fmaskb[NPAR], eobsb[NPAR], status, wq;
-    DevBuf cindex, coffset, sadtab;
-    DevBuf lcindex, lcoffset;  // the search launch's own compaction scan (never shared with stream K's)
+    DevBuf sadtab;
+    DevBuf lcindex, lcoffset;  // the search launch's compaction scan
+    DevBuf sym_mem;                     // working memory of launch_symbols (one frame at a time, in stream order)
+    unsigned sym_cap = 0;               // symbols a frame may have there, and its slot's stacks
     DevBuf mvbits, logfix, expfix, ytab, ctab, newcost, newcost32;
     bool small_costs = false;
     bool table_ok = false;  // exhaustive SAD table + packed argmin usable (costs < 2^59)
@@ -442,7 +450,8 @@ struct riv_encoder {
     bool have_times = false;
     riv_frame_stats last_stats{};
     double sum_times[NSTAGE + 1] = {0};
-    size_t coef_guess = 0;  // bytes of coefficients copied eagerly per frame
+    // bytes copied eagerly per frame, of key frames and of P-frames: truncated blocks, rANS stacks
+    size_t coef_guess[2] = {0, 0}, sym_guess[2] = {0, 0};
     DevBuf prof;            // optional per-MB phase stamps of the search kernel
     DevBuf tflag;           // fused table: per-MB "table row written" flags (frame tag)
     DevBuf rowdone;         // AQ inside the search: per-row "ln variances written" flags (frame tag)
@@ -521,6 +530,7 @@ static void setup_device(riv_encoder* e) {
     CK(cudaStreamCreateWithFlags(&e->Hs, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&e->Y, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&e->K, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithFlags(&e->R, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&e->N, cudaStreamNonBlocking));
     for (int k = 0; k < 2; k++) {
         CK(cudaEventCreateWithFlags(&e->ev_net_out[k], cudaEventDisableTiming));
@@ -644,6 +654,10 @@ static void setup_device(riv_encoder* e) {
     deblock_thresholds(e->inter_level, false, e->inter_E, e->inter_I, e->inter_H);
     e->intra_level = deblock_level(quant_step(c.intra_quality));
     deblock_thresholds(e->intra_level, true, e->intra_E, e->intra_I, e->intra_H);
+    // Symbols made on the GPU: room for 512 a macroblock (a key frame at quality 95 of a noisy
+    // 1080p clip has 470, a P-frame 25 to 130); a frame with more goes to the host coder.
+    e->sym_cap = (unsigned)(((size_t)N * 512 + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH);
+    e->sym_mem.alloc(sym_workspace(nullptr, N, e->sym_cap, nullptr));
     // pipeline slots
     int nslots = std::max(1u, c.pipeline_depth);
     e->slots.resize(nslots);
@@ -651,7 +665,7 @@ static void setup_device(riv_encoder* e) {
     for (auto& s : e->slots) {
         s.rgb.alloc(std::max(rgb_bytes, e->yuv_bytes));
         s.dside.alloc((size_t)N * 4);
-        s.dpacked.alloc((size_t)N * 384 * 2);
+        s.dpacked.alloc(std::max((size_t)N * 384 * 2, (size_t)e->sym_cap * 2));
         s.dpeobs.alloc((size_t)N * 3);
         s.side.alloc((size_t)N * 4);
         s.packed.alloc((size_t)N * 384 * 2);
@@ -664,13 +678,14 @@ static void setup_device(riv_encoder* e) {
         CK(cudaEventCreateWithFlags(&s.ev_yuv, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&s.ev_recon, cudaEventDisableTiming));
     }
-    e->coef_guess = (size_t)N * 384;  // half the dense size until the first frames are seen
+    for (int k = 0; k < 2; k++) {  // half the room until the first frames are seen
+        e->coef_guess[k] = (size_t)N * 384;
+        e->sym_guess[k] = (size_t)e->sym_cap;
+    }
     if (getenv("RIV_PROFILE_SEARCH")) {
         e->prof.alloc((size_t)N * RIV_PROF_WORDS * sizeof(long long));
         e->prof.zero(e->S);
     }
-    e->cindex.alloc((size_t)N * 4);
-    e->coffset.alloc((size_t)N * 4);
     e->lcindex.alloc((size_t)N * 4);
     e->lcoffset.alloc((size_t)N * 4);
     if (e->table_ok)
@@ -714,34 +729,64 @@ static Job* find_job(riv_encoder* e, uint64_t index) {
     return nullptr;
 }
 
-// Compaction of a frame whose reconstruction is enqueued (it waits for the frame's
-// EV_DEBLOCK; `compacted`: the search launch that reconstructed it compacted it too), then
-// the status and the device->host copies of its side info and coefficients.
+// The buffers of launch_symbols for a frame in rotation ck and pipeline slot s.
+static SymFrame sym_frame(riv_encoder* e, int ck, bool intra, Slot& s) {
+    SymFrame f{};
+    f.opt_skip = e->optskipb[ck].as<uint8_t>();
+    f.eobs = e->eobsb[ck].as<uint8_t>();
+    f.coeffs = e->coeffsb[ck].as<int16_t>();
+    f.mb = e->mboutb[ck].as<MbOut>();
+    f.nmb = e->NMB;
+    f.intra = intra ? 1 : 0;
+    f.cap = e->sym_cap;
+    sym_workspace(&f, e->NMB, e->sym_cap, e->sym_mem.p);
+    f.side = s.dside.as<uint32_t>();
+    f.stack = s.dpacked.as<uint16_t>();
+    f.packed = s.dpacked.as<int16_t>();
+    f.peobs = s.dpeobs.as<uint8_t>();
+    f.hdr = s.hdr.dev<uint32_t>();
+    return f;
+}
+
+// The first copy of a frame's rANS stacks to the host: whole batches, as many bytes as the last
+// frame of its type had and a quarter more, as far as the pinned buffer holds; its exact size is
+// only known once the frame is done.
+static void copy_stacks(riv_encoder* e, const Job& j, Slot& s, cudaStream_t st) {
+    const size_t batch = (size_t)SYM_BATCH * 2, room = std::min((size_t)e->sym_cap * 2, (size_t)e->NMB * 384 * 2);
+    s.prefetched = std::min((e->sym_guess[j.type - 1] + batch - 1) / batch * batch, room);
+    CK(cudaMemcpyAsync(s.packed.p, s.dpacked.p, s.prefetched, cudaMemcpyDeviceToHost, st));
+}
+
+// The tail of a frame whose reconstruction is enqueued (it waits for the frame's EV_DEBLOCK):
+// its coefficient symbols -- nothing, `compacted`, when the search launch that reconstructed it
+// packed its blocks for the host coder -- then the status and the device->host copies.
 static void frame_tail(riv_encoder* e, Job& j, bool compacted = false) {
     Slot& s = e->slots[j.slot];
     const int N = e->NMB, ck = j.ck;
     cudaStream_t K = e->K;
     CK(cudaStreamWaitEvent(K, s.ev_recon, 0));
     mark(e, j, EV_K0, K);
+    j.sym = false;
     if (!compacted) {
-        e->launches += 2;  // scan + pack
-        CK(launch_compact(e->optskipb[ck].as<uint8_t>(), e->mboutb[ck].as<MbOut>(), e->coeffsb[ck].as<int16_t>(),
-                          e->eobsb[ck].as<uint8_t>(), N, j.type == 1 ? 1 : 0, e->cindex.as<int32_t>(),
-                          e->coffset.as<int32_t>(), s.dside.as<uint32_t>(), s.dpacked.as<int16_t>(),
-                          s.dpeobs.as<uint8_t>(), s.hdr.dev<uint32_t>(), K));
+        e->launches += 5;
+        CK(launch_symbols(sym_frame(e, ck, j.type == 1, s), K));
+        j.sym = true;
     }
     CK(cudaEventRecord(e->ev_coef_free[ck], K));
     CK(cudaEventRecord(e->ev_mbout_free[ck], K));
     mark(e, j, EV_COMPACT, K);
     CK(cudaMemcpyAsync(s.hdr.host<uint32_t>() + 2, e->status.p, 4, cudaMemcpyDeviceToHost, K));
     CK(cudaEventRecord(s.ev_gpu, K));
-    // DMA the side info, EOBs and (a bounded prefix of) the coefficients on the copy
-    // stream; the exact size is only known once the frame is done.
+    // DMA the side info and (a bounded prefix of) the stacks or coefficients on the copy stream
     CK(cudaStreamWaitEvent(e->C, s.ev_gpu, 0));
     CK(cudaMemcpyAsync(s.side.p, s.dside.p, (size_t)N * 4, cudaMemcpyDeviceToHost, e->C));
-    CK(cudaMemcpyAsync(s.peobs.p, s.dpeobs.p, (size_t)N * 3, cudaMemcpyDeviceToHost, e->C));
-    s.prefetched = std::min(e->coef_guess, (size_t)N * 384 * 2);
-    CK(cudaMemcpyAsync(s.packed.p, s.dpacked.p, s.prefetched, cudaMemcpyDeviceToHost, e->C));
+    if (j.sym) {
+        copy_stacks(e, j, s, e->C);
+    } else {
+        CK(cudaMemcpyAsync(s.peobs.p, s.dpeobs.p, (size_t)N * 3, cudaMemcpyDeviceToHost, e->C));
+        s.prefetched = std::min(e->coef_guess[j.type - 1], (size_t)N * 384 * 2);
+        CK(cudaMemcpyAsync(s.packed.p, s.dpacked.p, s.prefetched, cudaMemcpyDeviceToHost, e->C));
+    }
     CK(cudaEventRecord(s.ev_d2h, e->C));
     j.tail_done = true;
 }
@@ -1207,15 +1252,29 @@ static riv_status retire(riv_encoder* e, Job& j) {
                     (st & ST_WAIT_TIMEOUT) ? "device-side wavefront wait timed out" : "device search iteration cap hit");
     }
     j.count = hdr[0];
-    const size_t coef_bytes = (size_t)hdr[1] * 2;
-    if (coef_bytes > s.prefetched) {  // the eager copy fell short: fetch the rest now
-        CK(cudaMemcpyAsync((char*)s.packed.p + s.prefetched, (const char*)s.dpacked.p + s.prefetched,
-                           coef_bytes - s.prefetched, cudaMemcpyDeviceToHost, e->C));
-        CK(cudaStreamSynchronize(e->C));
+    const size_t nsym = j.sym ? hdr[3] : 0;
+    if (j.sym && hdr[3] == SYM_FAIL) {  // more symbols than the stacks hold, or a class that cannot be coded
+        j.sym = false;
+        s.prefetched = 0;
+        CK(cudaMemcpyAsync(s.peobs.p, s.dpeobs.p, (size_t)e->NMB * 3, cudaMemcpyDeviceToHost, e->R));
+        CK(cudaStreamSynchronize(e->R));
     }
-    // next frames: copy 25% + 64 KiB more than this frame needed
-    e->coef_guess = coef_bytes + coef_bytes / 4 + 65536;
-    e->d2h_bytes += (uint64_t)e->NMB * 7 + 12 + std::max(coef_bytes, s.prefetched);
+    // what the host coder reads: whole rANS batches, or the truncated blocks
+    const size_t coef_bytes = j.sym ? (nsym + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH * 2 : (size_t)hdr[1] * 2;
+    const uint16_t* stacks = s.packed.as<uint16_t>();
+    if (j.sym && coef_bytes > (size_t)e->NMB * 384 * 2) {  // more than the pinned buffer holds (rare: high-quality key frames)
+        j.big_stacks.resize(coef_bytes / 2);
+        CK(cudaMemcpyAsync(j.big_stacks.data(), s.dpacked.p, coef_bytes, cudaMemcpyDeviceToHost, e->R));
+        CK(cudaStreamSynchronize(e->R));
+        stacks = j.big_stacks.data();
+    } else if (coef_bytes > s.prefetched) {  // the eager copy fell short: fetch the rest now
+        CK(cudaMemcpyAsync((char*)s.packed.p + s.prefetched, (const char*)s.dpacked.p + s.prefetched,
+                           coef_bytes - s.prefetched, cudaMemcpyDeviceToHost, e->R));
+        CK(cudaStreamSynchronize(e->R));
+    }
+    // next frames of this type: copy 25% + 64 KiB more than this frame needed
+    (j.sym ? e->sym_guess : e->coef_guess)[j.type - 1] = coef_bytes + coef_bytes / 4 + 65536;
+    e->d2h_bytes += (uint64_t)e->NMB * (j.sym ? 4 : 7) + 16 + std::max(coef_bytes, s.prefetched);
     float t[NSTAGE + 1] = {0};
     if (!j.xev) CK(cudaEventSynchronize(s.ev_recon));  // the D2H did not wait for the deblock
     // stage 1 of the learned form is its network, on stream N
@@ -1307,7 +1366,23 @@ static riv_status retire(riv_encoder* e, Job& j) {
     // batches to rans_pool, which keeps the CPU cost per frame lowest while frames overlap
     // (splitting every drained frame measured slower on a 16-core host: the split coder's
     // extra work then competes with the frames beside it).
-    const int parts = e->draining && &j == &e->jobs.back() ? e->rans_parts : 1;
+    // Frames whose symbols the GPU modelled need only their rANS batches coded.
+    const bool newest = e->draining && &j == &e->jobs.back();
+    if (j.sym) {
+        j.fut = e->pool->submit([jp, ep, stacks, nsym, newest] {
+            double d0 = now_ms();
+            jp->tr[7] = d0;
+            jp->res_writer = encode_stacks_async(stacks, nsym, jp->res_bytes, newest ? ep->rans_submit_urgent : ep->rans_submit);
+            jp->tr[8] = now_ms();
+            double dt = jp->tr[8] - d0;
+            std::lock_guard<std::mutex> g(ep->stat_mu);
+            ep->host_ms[3] += dt;
+        }, newest);
+        j.state = 1;
+        e->host_ms[1] += now_ms() - t0;
+        return RIV_OK;
+    }
+    const int parts = newest ? e->rans_parts : 1;
     j.fut = e->pool->submit([jp, ep, packed, peobs, count, intra, parts] {
         double d0 = now_ms();
         jp->tr[7] = d0;
@@ -1424,7 +1499,28 @@ static riv_status pump(riv_encoder* e, bool block_front, bool block_write) {
     return RIV_OK;
 }
 
+// At a drain no further search launch follows, and the GPU is idle once the launches in flight end,
+// while the host needs about 2 ms to model each 1080p frame: the last frames are the tail of the
+// drain.  Those that a search launch reconstructed and packed, and whose coefficients are still in
+// the rotation, get a second tail with their symbols made on the GPU, behind the last launch (their
+// kernels would delay it) and behind the first tail's copies (their stacks take the packed blocks'
+// place): 16 frames of 1080p took 13.3 ms without, 11.7 ms with this.
+static void retail_last_frames(riv_encoder* e) {
+    if (!e->pend.active) return;
+    for (auto& j : e->jobs) {
+        if (j.index + NPAR <= e->pend.index || j.state != 0 || !j.tail_done || !j.deferred || j.sym) continue;
+        Slot& s = e->slots[j.slot];
+        CK(cudaStreamWaitEvent(e->K, e->ev_search_done, 0));
+        CK(cudaStreamWaitEvent(e->K, s.ev_d2h, 0));
+        const bool timed = j.timed;  // its stage marks are the first tail's
+        j.timed = false;
+        frame_tail(e, j);
+        j.timed = timed;
+    }
+}
+
 static riv_status drain_all(riv_encoder* e) {
+    retail_last_frames(e);
     flush_pending(e);  // no later launch is coming: reconstruct now, before the host work queued ahead of it
     struct Draining {
         riv_encoder* e;
@@ -1719,6 +1815,7 @@ void riv_encoder_free(riv_encoder* e) {
     if (e->Hs) cudaStreamSynchronize(e->Hs);
     if (e->Y) cudaStreamSynchronize(e->Y);
     if (e->K) cudaStreamSynchronize(e->K);
+    if (e->R) cudaStreamSynchronize(e->R);
     for (auto& s : e->slots) {
         s.rgb.release(); s.dside.release(); s.dpacked.release(); s.dpeobs.release();
         s.side.release(); s.packed.release(); s.peobs.release(); s.hdr.release();
@@ -1736,7 +1833,7 @@ void riv_encoder_free(riv_encoder* e) {
             b->release();
     DevBuf* bufs[] = {&e->ref[0], &e->ref[1], &e->recon_pre, &e->wq, &e->coded[0], &e->coded[1], &e->rec,
                       &e->varsum, &e->qs, &e->status,
-                      &e->mvbits, &e->logfix, &e->expfix, &e->ytab, &e->ctab, &e->cindex, &e->coffset, &e->lcindex, &e->lcoffset, &e->sadtab, &e->prof, &e->tflag, &e->rowdone, &e->newcost, &e->newcost32,
+                      &e->mvbits, &e->logfix, &e->expfix, &e->ytab, &e->ctab, &e->sym_mem, &e->lcindex, &e->lcoffset, &e->sadtab, &e->prof, &e->tflag, &e->rowdone, &e->newcost, &e->newcost32,
                       &e->nn_w, &e->nn_b, &e->nn_feat, &e->nn_a1, &e->nn_a2, &e->nn_a3, &e->nn_x1, &e->nn_h1, &e->nn_h2,
                       &e->nn_o[0], &e->nn_o[1], &e->lmv, &e->lcount, &e->lrowcnt};
     for (DevBuf* b : bufs) b->release();
@@ -1753,6 +1850,7 @@ void riv_encoder_free(riv_encoder* e) {
     if (e->Hs) cudaStreamDestroy(e->Hs);
     if (e->Y) cudaStreamDestroy(e->Y);
     if (e->K) cudaStreamDestroy(e->K);
+    if (e->R) cudaStreamDestroy(e->R);
     for (int k = 0; k < NPAR; k++) {
         if (e->ev_cur_free[k]) cudaEventDestroy(e->ev_cur_free[k]);
         if (e->ev_mbout_free[k]) cudaEventDestroy(e->ev_mbout_free[k]);
@@ -2284,6 +2382,84 @@ riv_status riv_test_dct_decode(const uint8_t* data, size_t len, const uint8_t* c
     if ((len > 0 && !data) || (n > 0 && (!coded || !out))) return RIV_ERR_FRAME;
     entropy_init();
     return decode_residual_frame(data, len, coded, (int)n, intra != 0, out) ? RIV_OK : RIV_ERR_FRAME;
+}
+
+riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, uint32_t n, int intra, uint32_t max_symbols,
+                                   uint8_t* out, size_t cap, size_t* len, int* on_gpu) {
+    if (n == 0 || !blocks || !len || !on_gpu || (!intra && !skip)) return RIV_ERR_FRAME;
+    entropy_init();
+    static const int base[3] = {0, 256, 320}, len3[3] = {256, 64, 64};
+    std::vector<uint8_t> eobs((size_t)n * 3);
+    for (uint32_t b = 0; b < n; b++)
+        for (int pl = 0; pl < 3; pl++) {
+            const int16_t* p = blocks + (size_t)b * 384 + base[pl];
+            int last = 0;
+            for (int i = len3[pl] - 1; i >= (intra ? 1 : 0); i--)
+                if (p[i] != 0) { last = i; break; }
+            eobs[(size_t)b * 3 + pl] = (uint8_t)last;
+        }
+    struct Bufs {
+        DevBuf co, sk, eo, mb, work, side, packed, peobs;
+        MappedBuf hdr;
+        ~Bufs() {
+            for (DevBuf* b : {&co, &sk, &eo, &mb, &work, &side, &packed, &peobs}) b->release();
+            hdr.release();
+        }
+    } B;
+    std::vector<uint8_t> stream;
+    try {
+        SymFrame f{};
+        f.cap = (unsigned)(((max_symbols ? (size_t)max_symbols : (size_t)n * 512) + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH);
+        B.co.alloc((size_t)n * 384 * 2);
+        B.sk.alloc(n);
+        B.eo.alloc((size_t)n * 3);
+        B.mb.alloc((size_t)n * sizeof(MbOut));
+        B.work.alloc(sym_workspace(nullptr, (int)n, f.cap, nullptr));
+        B.side.alloc((size_t)n * 4);
+        B.packed.alloc(std::max((size_t)f.cap * 2, (size_t)n * 384 * 2));
+        B.peobs.alloc((size_t)n * 3);
+        B.hdr.alloc(16);
+        CK(cudaMemcpy(B.co.p, blocks, (size_t)n * 384 * 2, cudaMemcpyHostToDevice));
+        if (skip) CK(cudaMemcpy(B.sk.p, skip, n, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(B.eo.p, eobs.data(), (size_t)n * 3, cudaMemcpyHostToDevice));
+        CK(cudaMemset(B.mb.p, 0, (size_t)n * sizeof(MbOut)));
+        f.opt_skip = B.sk.as<uint8_t>();
+        f.eobs = B.eo.as<uint8_t>();
+        f.coeffs = B.co.as<int16_t>();
+        f.mb = B.mb.as<MbOut>();
+        f.nmb = (int)n;
+        f.intra = intra ? 1 : 0;
+        sym_workspace(&f, (int)n, f.cap, B.work.p);
+        f.side = B.side.as<uint32_t>();
+        f.stack = B.packed.as<uint16_t>();
+        f.packed = B.packed.as<int16_t>();
+        f.peobs = B.peobs.as<uint8_t>();
+        f.hdr = B.hdr.dev<uint32_t>();
+        CK(launch_symbols(f, nullptr));
+        CK(cudaDeviceSynchronize());
+        const uint32_t* h = B.hdr.host<uint32_t>();
+        *on_gpu = h[3] != SYM_FAIL ? 1 : 0;
+        ThreadPool pool(2);
+        BatchSubmit sub = [&pool](std::function<void()> g) { return pool.submit(std::move(g)); };
+        if (*on_gpu) {
+            std::vector<uint16_t> st(((size_t)h[3] + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH);
+            CK(cudaMemcpy(st.data(), B.packed.p, st.size() * 2, cudaMemcpyDeviceToHost));
+            if (auto w = encode_stacks_async(st.data(), h[3], stream, sub)) w->collect();
+        } else {
+            std::vector<int16_t> pk(h[1]);
+            std::vector<uint8_t> pe((size_t)h[0] * 3);
+            CK(cudaMemcpy(pk.data(), B.packed.p, pk.size() * 2, cudaMemcpyDeviceToHost));
+            CK(cudaMemcpy(pe.data(), B.peobs.p, pe.size(), cudaMemcpyDeviceToHost));
+            encode_residual_frame(pk.data(), pe.data(), (int)h[0], intra != 0, stream, &sub, 3);
+        }
+    } catch (const CudaError&) {
+        return RIV_ERR_CUDA;
+    } catch (const std::exception&) {
+        return RIV_ERR_ENCODING_FAILED;
+    }
+    *len = stream.size();
+    if (out && cap) memcpy(out, stream.data(), std::min(cap, stream.size()));
+    return RIV_OK;
 }
 
 riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uint32_t threads, uint8_t* out, size_t cap,
@@ -2910,13 +3086,9 @@ static void batch_collect(riv_encoder* e, Job& j, int src, const void* frame, cu
         e->has_prev2_mvs = e->has_prev_mvs;
         e->has_prev_mvs = true;
     }
-    k.c_index = e->cindex.as<int32_t>();
-    k.c_offset = e->coffset.as<int32_t>();
-    k.c_side = s.dside.as<uint32_t>();
-    k.c_packed = s.dpacked.as<int16_t>();
-    k.c_peobs = s.dpeobs.as<uint8_t>();
-    k.c_hdr = s.hdr.dev<uint32_t>();
-    k.status = e->status.as<unsigned>();
+    k.sym = sym_frame(e, ck, j.type == 1, s);
+    k.sym.status = e->status.as<unsigned>();
+    j.sym = true;
     e->ref_cur = nxt;
     e->has_ref = true;
     e->last_par = ck;
@@ -3119,7 +3291,7 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         const double h1 = now_ms();
         b->host_ms[0] += room;
         b->host_ms[1] += h1 - h0 - room;
-        // ---- copies back: side info, EOBs and a bounded prefix of the coefficients per clip
+        // ---- copies back: side info and a bounded prefix of the rANS stacks per clip
         cudaEvent_t xev = b->ev_step[b->steps % b->ev_step.size()];
         CK(cudaStreamWaitEvent(b->C, b->ev_gpu, 0));
         for (int a = 0; a < m; a++) {
@@ -3127,10 +3299,8 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
             Slot& s = e->slots[jobs[a]->slot];
             const int N = e->NMB;
             CK(cudaMemcpyAsync(s.side.p, s.dside.p, (size_t)N * 4, cudaMemcpyDeviceToHost, b->C));
-            CK(cudaMemcpyAsync(s.peobs.p, s.dpeobs.p, (size_t)N * 3, cudaMemcpyDeviceToHost, b->C));
-            s.prefetched = std::min(e->coef_guess, (size_t)N * 384 * 2);
-            CK(cudaMemcpyAsync(s.packed.p, s.dpacked.p, s.prefetched, cudaMemcpyDeviceToHost, b->C));
-            b->d2h_bytes += (uint64_t)N * 7 + s.prefetched;
+            copy_stacks(e, *jobs[a], s, b->C);
+            b->d2h_bytes += (uint64_t)N * 4 + s.prefetched;
         }
         CK(cudaEventRecord(xev, b->C));
         if (src == 0) {

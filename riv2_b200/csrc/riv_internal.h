@@ -94,7 +94,7 @@ struct SearchParams {
     int nlog;
     // Residual and deblock of the previous P-frame, run by the table workers of this launch
     // ahead of the table rows that need them (defer != 0), then (compact != 0) its compaction
-    // (scan + pack, as k_scan / k_pack) at the end of the queue.  wq: [0] task counter,
+    // (scan + pack) at the end of the queue.  wq: [0] task counter,
     // [1 .. BH] residual MBs done per MB row, [BH+1 .. 2BH] deblock tiles done per band,
     // [2BH+1] scan done.  Launches alternate between two such arrays: each zeroes the other
     // (wq_next, wq_words words) for the next launch, its own having been zeroed by the last.
@@ -116,6 +116,34 @@ struct SearchParams {
     uint32_t* c_hdr;
 };
 
+
+// One frame's coefficients on their way to the host's rANS coder (riv_symbols.cuh).
+constexpr unsigned SYM_BATCH = 16386;       // symbols of a rANS batch (com/rans.rs:201)
+constexpr int SYM_ROWS = 448;               // rows of the count table: models, totals, padding to whole lines
+constexpr int SYM_TAB = 2;                  // work: [0] list cursor, [1] symbols made here, then (base, length) per model
+constexpr int SYM_WORK_WORDS = SYM_TAB + 2 * 427;
+constexpr unsigned SYM_UNIT = 128;          // symbols of a model whose probabilities one warp computes
+constexpr unsigned SYM_OCC_SLACK = (SYM_UNIT - 1) * 427;  // each model's list starts on a unit
+constexpr unsigned SYM_FAIL = 0xffffffffu;  // header word 3: the host coder takes the frame
+struct SymFrame {
+    const uint8_t* opt_skip;
+    const uint8_t* eobs;
+    const int16_t* coeffs;
+    const MbOut* mb;  // P-frames
+    int nmb, intra;
+    unsigned cap;     // symbols that `stack` and `occ` hold (a multiple of SYM_BATCH)
+    uint16_t* cnt;    // counts of each part, [SYM_ROWS] (riv_symbols.cuh)
+    unsigned* tot;    // and of each CTA
+    unsigned* occ;    // cap + SYM_OCC_SLACK: per model, its symbols' stack positions | bit << 31
+    uint32_t* ustate; // per unit of occ: the model's counts at its start and the model
+    unsigned* work;   // SYM_WORK_WORDS
+    uint32_t* side;
+    uint16_t* stack;  // cap (probability | bit << 8); the same memory as packed
+    int16_t* packed;  // when the host coder takes the frame: truncated blocks and their EOBs
+    uint8_t* peobs;
+    uint32_t* hdr;    // mapped host words: coded MBs, coefficients, [2] = *status (not nullptr), symbols
+    const unsigned* status;
+};
 
 // ---- multi-clip steps (riv_batch): one launch per stage over every clip of the step.
 // One clip's frame in a step.
@@ -142,15 +170,7 @@ struct BatchClip {
     const uint8_t* db_src;
     uint8_t* db_dst;
     const uint8_t* db_mask;
-    // compaction into the slot's buffers; c_hdr = mapped host words (coded MBs, coefficients,
-    // status)
-    int32_t* c_index;
-    int32_t* c_offset;
-    uint32_t* c_side;
-    int16_t* c_packed;
-    uint8_t* c_peobs;
-    uint32_t* c_hdr;
-    const unsigned* status;
+    SymFrame sym;  // symbols into the slot's buffers
 };
 enum BatchStage { BS_CONVERT, BS_TABLE, BS_PREDICT, BS_AQSUM, BS_RESIDUAL, BS_DEBLOCK, BS_SCAN, BS_PACK, BS_N };
 // Tile shapes of a step (chosen by the batch's autotuner; the output does not depend on them).
@@ -211,11 +231,11 @@ int launch_deblock_tiled(const uint8_t* src, uint8_t* dst, int W, int H, int E, 
 // DEBLOCK_NOALLOC_MAX_BYTES bytes); the address is valid on the current device.
 constexpr size_t DEBLOCK_NOALLOC_MAX_BYTES = (size_t)4 << 20;
 int deblock_scratch_address(void** out);
-// k_scan writes {coded MBs, coefficients} to hhdr (mapped host memory); k_pack fills the
-// device-side side info / EOB / coefficient buffers, copied back by DMA afterwards.
-int launch_compact(const uint8_t* opt_skip, const MbOut* mb, const int16_t* coeffs, const uint8_t* eobs, int nmb,
-                   int intra, int32_t* index, int32_t* offset, uint32_t* dside, int16_t* dpacked, uint8_t* dpeobs,
-                   uint32_t* hhdr, void* stream);
+// Side info and rANS stacks of a reconstructed frame (riv_symbols.cuh), copied back by DMA
+// afterwards.
+int launch_symbols(const SymFrame& f, void* stream);
+// Bytes of a frame's cnt, tot, occ, ustate and work; with f, lays them out at p (256-byte aligned).
+size_t sym_workspace(SymFrame* f, int nmb, unsigned cap, void* p);
 // libm device helpers exposed for the exhaustive check
 int launch_libm_eval(int which, const float* in, float* out, size_t n, const uint32_t* fix, int nfix, void* stream);
 // Learned-proposal form of the P-frame search and mode decision (riv_kernels.cu): lmv holds 8

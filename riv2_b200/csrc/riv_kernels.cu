@@ -1205,7 +1205,6 @@ __device__ __forceinline__ bool wait_ref_rows(const SearchParams& p, int r, int 
 // Scan by NT threads (named barrier `bar`): each thread owns IPT consecutive MBs of an
 // NT * IPT chunk (all their loads are issued together), then one scan of the thread totals
 // per chunk.  wsum / wsz: NT / 32 ints of shared memory each.
-constexpr int SC_THREADS = 256, SC_IPT = 32;
 template <int NT, int IPT>
 __device__ __forceinline__ void scan_mbs(const uint8_t* opt_skip, const uint8_t* eobs, int nmb, int intra,
                                          int32_t* index, int32_t* offset, uint32_t* hdr, int tid, int bar, int* wsum,
@@ -1257,22 +1256,17 @@ __device__ __forceinline__ void scan_mbs(const uint8_t* opt_skip, const uint8_t*
     }
     if (tid == 0) { hdr[0] = (uint32_t)carry; hdr[1] = (uint32_t)carry_sz; }
 }
-// Pack MB m with one warp: side info, EOBs and the truncated coefficient blocks.
-__device__ __forceinline__ void pack_mb(int m, int lane, const uint8_t* opt_skip, const MbOut* mb,
-                                        const int16_t* coeffs, const uint8_t* eobs, const int32_t* index,
-                                        const int32_t* offset, int intra, uint32_t* side, int16_t* packed,
-                                        uint8_t* peobs) {
-    const int k = index[m];
-    const int e0 = eobs[3 * m], e1 = eobs[3 * m + 1], e2 = eobs[3 * m + 2];
+__device__ __forceinline__ uint32_t side_word(const MbOut& o, unsigned skip) {
+    return (uint32_t)o.mode | ((uint32_t)o.base << 3) | ((uint32_t)(o.raw[2] & 1) << 6) | ((uint32_t)(o.raw[3] & 1) << 7) |
+           ((uint32_t)(uint8_t)o.rdelta[0] << 8) | ((uint32_t)(uint8_t)o.rdelta[1] << 16) | ((skip & 1u) << 24);
+}
+// Pack MB m with one warp: side info, EOBs and the truncated coefficient blocks.  k: its index
+// among the coded MBs (negative: not coded), off: its first coefficient's place.
+__device__ __forceinline__ void pack_mb_at(int m, int lane, int k, int off, const uint8_t* opt_skip, const MbOut* mb,
+                                           const int16_t* coeffs, int e0, int e1, int e2, int intra, uint32_t* side,
+                                           int16_t* packed, uint8_t* peobs) {
     if (lane == 0) {
-        uint32_t s = 0;
-        if (!intra) {
-            const MbOut o = mb[m];
-            s = (uint32_t)o.mode | ((uint32_t)o.base << 3) | ((uint32_t)(o.raw[2] & 1) << 6) |
-                ((uint32_t)(o.raw[3] & 1) << 7) | ((uint32_t)(uint8_t)o.rdelta[0] << 8) |
-                ((uint32_t)(uint8_t)o.rdelta[1] << 16) | ((uint32_t)(opt_skip[m] & 1) << 24);
-        }
-        side[m] = s;
+        side[m] = intra ? 0u : side_word(mb[m], opt_skip[m]);
         if (k >= 0) {
             peobs[3 * k] = (uint8_t)e0;
             peobs[3 * k + 1] = (uint8_t)e1;
@@ -1282,7 +1276,7 @@ __device__ __forceinline__ void pack_mb(int m, int lane, const uint8_t* opt_skip
     if (k < 0) return;
     const int n0 = e0 + 1, n1 = e1 + 1, n2 = e2 + 1;
     const int16_t* src = coeffs + (size_t)m * 384;
-    int16_t* dst = packed + offset[m];
+    int16_t* dst = packed + off;
     for (int i = lane; i < n0 + n1 + n2; i += 32) {
         const int si = i < n0 ? i : (i < n0 + n1 ? 256 + (i - n0) : 320 + (i - n0 - n1));
         dst[i] = src[si];
@@ -1432,8 +1426,12 @@ __device__ __forceinline__ void worker_loop(const SearchParams& p, uint8_t* regi
             group_sync(bar, TW_GROUP);
             if (!*gok) return;
             for (int x = tid >> 5; x < p.BW; x += TW_GROUP / 32)
-                pack_mb(row * p.BW + x, tid & 31, p.dres.opt_skip, p.dres.mb, p.dres.coeffs, p.dres.eobs, p.c_index,
-                        p.c_offset, 0, p.c_side, p.c_packed, p.c_peobs);
+            {
+                const int m = row * p.BW + x;
+                const uint8_t* eb = p.dres.eobs + 3 * (size_t)m;
+                pack_mb_at(m, tid & 31, p.c_index[m], p.c_offset[m], p.dres.opt_skip, p.dres.mb, p.dres.coeffs, eb[0], eb[1],
+                           eb[2], 0, p.c_side, p.c_packed, p.c_peobs);
+            }
         } else {  // SAD-table row of MB (row, idx)
             if (tid == 0) {
                 RIV_GSTAMP(row * p.BW + idx, 23);
@@ -3486,31 +3484,9 @@ static __device__ __align__(256) uint8_t g_deblock_scratch[DEBLOCK_NOALLOC_MAX_B
 int deblock_scratch_address(void** out) { return (int)cudaGetSymbolAddress(out, g_deblock_scratch); }
 
 // ---------------------------------------------------------------------------------
-// K8 kernels (compaction of a frame reconstructed outside a search launch; the layout is
-// described at scan_mbs / pack_mb).
+// K8: side info and coefficient symbols of a frame reconstructed outside a search launch.
 // ---------------------------------------------------------------------------------
-// Scan: one CTA of SC_THREADS threads (scan_mbs), small enough to run beside the search kernel.
-__global__ void __launch_bounds__(SC_THREADS) k_scan(const uint8_t* opt_skip, const uint8_t* eobs, int nmb, int intra,
-                                                     int32_t* index, int32_t* offset, uint32_t* hdr) {
-    __shared__ int wsum[SC_THREADS / 32], wsz[SC_THREADS / 32];
-    scan_mbs<SC_THREADS, SC_IPT>(opt_skip, eobs, nmb, intra, index, offset, hdr, threadIdx.x, 1, wsum, wsz);
-}
-// Pack: one warp per MB.
-__global__ void __launch_bounds__(256) k_pack(const uint8_t* opt_skip, const MbOut* mb, const int16_t* coeffs,
-                                              const uint8_t* eobs, const int32_t* index, const int32_t* offset,
-                                              int intra, int nmb, uint32_t* side, int16_t* packed, uint8_t* peobs) {
-    const int m = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (m < nmb) pack_mb(m, threadIdx.x & 31, opt_skip, mb, coeffs, eobs, index, offset, intra, side, packed, peobs);
-}
-
-int launch_compact(const uint8_t* opt_skip, const MbOut* mb, const int16_t* coeffs, const uint8_t* eobs, int nmb,
-                   int intra, int32_t* index, int32_t* offset, uint32_t* dside, int16_t* dpacked, uint8_t* dpeobs,
-                   uint32_t* hhdr, void* stream) {
-    cudaStream_t st = (cudaStream_t)stream;
-    k_scan<<<1, SC_THREADS, 0, st>>>(opt_skip, eobs, nmb, intra, index, offset, hhdr);
-    k_pack<<<(nmb + 7) / 8, 256, 0, st>>>(opt_skip, mb, coeffs, eobs, index, offset, intra, nmb, dside, dpacked, dpeobs);
-    return (int)cudaGetLastError();
-}
+#include "riv_symbols.cuh"
 
 // Multi-clip launches of the stages above (riv_batch).
 #include "riv_batch.cuh"

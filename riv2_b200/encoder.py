@@ -122,7 +122,7 @@ EXPORTED_SYMBOLS = (
     "riv_stage_rgb_to_yuv", "riv_stage_deblock", "riv_stage_libm", "riv_libm_fixup_counts", "riv_dct_tables",
     "riv_debug_frame_state", "riv_counters", "riv_host_times", "riv_stage_deblock_noalloc",
     "riv_decoder_new", "riv_decoder_info", "riv_decode_frame_yuv", "riv_decode_frame_rgb", "riv_decoder_current_frame",
-    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_decode", "riv_test_mv_encode",
+    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_encode_gpu", "riv_test_dct_decode", "riv_test_mv_encode",
     "riv_test_mv_decode", "riv_test_delta_bias", "riv_test_worker_queue", "riv_test_libm_range",
     "riv_stage_predict", "riv_stage_residual", "riv_test_wait_expiry", "riv_encoder_set_proposal",
     "riv_learned_counters", "riv_test_mv_encode_threads",
@@ -144,6 +144,8 @@ def lib() -> C.CDLL:
     L.riv_encode_frame_yuv.argtypes = [P, U8P, U8P, U8P, C.c_uint64, C.POINTER(RivFrameStats)]
     L.riv_finish.argtypes = [P]
     L.riv_test_dct_encode.argtypes = [P, C.c_uint32, C.c_int, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t)]
+    L.riv_test_dct_encode_gpu.argtypes = [P, P, C.c_uint32, C.c_int, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t),
+                                          C.POINTER(C.c_int)]
     L.riv_test_dct_decode.argtypes = [P, C.c_size_t, P, C.c_uint32, C.c_int, P]
     L.riv_test_mv_encode.argtypes = [P, P, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t), P]
     L.riv_test_mv_decode.argtypes = [P, P, P, C.c_uint32, P]
@@ -676,6 +678,22 @@ def dct_encode_host(blocks: np.ndarray, intra: bool, threads: int = 0) -> bytes:
     out = np.zeros(max(n.value, 1), np.uint8)
     lib().riv_test_dct_encode(b.ctypes.data, b.shape[0], int(intra), threads, out.ctypes.data, n.value, C.byref(n))
     return out[:n.value].tobytes()
+
+
+def dct_encode_gpu(blocks: np.ndarray, intra: bool, skip: Optional[np.ndarray] = None, max_symbols: int = 0):
+    """The encoder's coefficient stream with symbols and models made on the GPU (test hook):
+    (bytes, whether the GPU made them) of dense (n, 384) int16 blocks; skip: per-block flags of a
+    P-frame.  Raises EncodingFailed where the reference encoder panics."""
+    b = np.ascontiguousarray(blocks, dtype=np.int16)
+    k = np.ascontiguousarray(np.zeros(b.shape[0]) if skip is None else skip, dtype=np.uint8)
+    n, g = C.c_size_t(0), C.c_int(0)
+    cap = 64 + b.size * 4
+    out = np.zeros(cap, np.uint8)
+    st = lib().riv_test_dct_encode_gpu(b.ctypes.data, k.ctypes.data, b.shape[0], int(intra), max_symbols, out.ctypes.data,
+                                       cap, C.byref(n), C.byref(g))
+    if st != 0:
+        raise _ERRORS.get(st, EncodeError)(f"riv_test_dct_encode_gpu failed (status {st})")
+    return out[:n.value].tobytes(), bool(g.value)
 
 
 def dct_decode_host(data: bytes, coded: np.ndarray, intra: bool):

@@ -162,10 +162,13 @@ __global__ void __maxnreg__(120) k_search_multi(const SearchParams* __restrict__
     search_body<false, TABLE, SMALL>(ps[batch_clip(start, nclips, blockIdx.x)]);
 }
 
-static const void* search_multi_fn(bool table, bool small) {
-    if (table && small) return (const void*)k_search_multi<true, true>;
-    if (table) return (const void*)k_search_multi<true, false>;
-    return (const void*)k_search_multi<false, false>;
+static const void* search_multi_fn(SearchKind k) {
+    switch (k) {
+        case SK_TABLE_SMALL: return (const void*)k_search_multi<true, true>;
+        case SK_TABLE: return (const void*)k_search_multi<true, false>;
+        case SK_DIRECT: return (const void*)k_search_multi<false, true>;
+        default: return (const void*)k_search_multi<false, false>;
+    }
 }
 
 static size_t batch_stage_smem(int s, int max_sr) {
@@ -229,10 +232,15 @@ int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int tota
     return (int)cudaGetLastError();
 }
 
-int search_multi_capacity(bool table, bool small, int max_sr, int* per_sm, size_t* smem, int* threads) {
-    const void* fn = search_multi_fn(table, small);
-    const size_t sm = search_smem(max_sr, 0, false, table);
-    const int nt = search_threads(false, table);
+int search_multi_kind(bool table, bool small) {
+    return table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN;
+}
+bool search_multi_table(int kind) { return kind == SK_TABLE_SMALL || kind == SK_TABLE; }
+
+int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* threads) {
+    const void* fn = search_multi_fn((SearchKind)kind);
+    const size_t sm = search_smem(max_sr, 0, false, (SearchKind)kind);
+    const int nt = search_threads(false);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nt, sm);
     *smem = sm;
@@ -240,12 +248,12 @@ int search_multi_capacity(bool table, bool small, int max_sr, int* per_sm, size_
     return (int)e;
 }
 
-int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total, bool table, bool small,
-                        size_t smem, int threads, void* stream) {
+int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total, int kind, size_t smem,
+                        int threads, void* stream) {
     if (total <= 0) return 0;
     void* args[] = {(void*)&dparams, (void*)&dstart, (void*)&nclips};
     // cooperative: every clip's row CTAs are co-resident, so each row's wait on the row above
     // (a CTA of the same clip) can always make progress
-    return (int)cudaLaunchCooperativeKernel(search_multi_fn(table, small), dim3(total), dim3(threads), args, smem,
+    return (int)cudaLaunchCooperativeKernel(search_multi_fn((SearchKind)kind), dim3(total), dim3(threads), args, smem,
                                             (cudaStream_t)stream);
 }

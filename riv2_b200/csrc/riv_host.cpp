@@ -618,7 +618,7 @@ static void setup_device(riv_encoder* e) {
     if (e->splan.grid <= 0) throw std::runtime_error("search kernel cannot be made resident");
     // P-frame reconstruction folded into the next P-frame's search launch (its worker CTAs)
     e->learned = c.encode_form != RIV_FORM_PLAIN;
-    e->defer_ok = !e->learned && e->splan.fused && e->splan.fast && e->table_ok && c.pipeline_depth > 1;
+    e->defer_ok = !e->learned && e->splan.fused && e->splan.fast && c.pipeline_depth > 1;
     if (e->learned) {
         e->lmv.alloc((size_t)N * 8);
         e->lcount.alloc(2 * sizeof(unsigned));
@@ -894,7 +894,7 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
     if (j.type == 1) flush_pending(e);  // key frames reconstruct immediately
     // kernels per frame: rgb->yuv, (search, predict, 3 x aq), residual, deblock, scan + pack
     const int p_launches = e->learned ? (c.encode_form == RIV_FORM_LEARNED ? 8 : 0) + 3
-                                      : 1 + (e->table_ok && !e->splan.fused ? 1 : 0) + (e->splan.fast && e->table_ok ? 0 : 4);
+                                      : 1 + (e->splan.table && !e->splan.fused ? 1 : 0) + (e->splan.fast ? 0 : 4);
     e->launches += (src == 2 ? 0 : 1) + (j.type == 2 ? p_launches : 0);  // + residual / deblock / compaction below
     if (src == 0) e->h2d_bytes += (uint64_t)c.display_width * c.display_height * 3;
     if (src == 2) e->h2d_bytes += e->yuv_bytes;
@@ -977,7 +977,7 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
             CK(cudaEventRecord(e->ev_net_cur[e->last_par], Nn));     // cur of the previous frame read
             CK(cudaStreamWaitEvent(S, e->ev_net_out[nbuf], 0));
         }
-        if (e->table_ok && !e->learned) {
+        if (e->splan.table && !e->learned) {
             sp.tstride = sad_table_stride(c.search_range);
             sp.tab = e->sadtab.as<uint16_t>();
             if (e->splan.fused) sp.tflag = e->tflag.as<unsigned>();  // computed inside the search launch
@@ -990,7 +990,7 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
         sp.coded_out = e->coded[cn].as<int8_t>();
         // prediction, variances and ln inside the search launch (plain fused form), or inside the
         // learned forms' parallel search (their launch also folds the mean)
-        const bool aq_in_search = (e->splan.fast && e->table_ok) || e->learned;
+        const bool aq_in_search = e->splan.fast || e->learned;
         if (aq_in_search) {  // prediction, variances and ln inside the search launch
             sp.pred = e->predb[ck].as<uint8_t>();
             sp.varsum = e->varsum.as<uint2>();
@@ -2942,9 +2942,9 @@ struct riv_batch {
     size_t off_sp = 0, off_start = 0, off_sstart = 0, desc_bytes = 0;
     int dpar = 0;
     int max_sr = 0;
-    // search capacity per variant: 0 table + small costs, 1 table, 2 no table
-    int cap[3] = {0, 0, 0}, sthreads[3] = {0, 0, 0};
-    size_t ssmem[3] = {0, 0, 0};
+    // search capacity per kind of launch (search_multi_kind)
+    int cap[SEARCH_KINDS] = {}, sthreads[SEARCH_KINDS] = {};
+    size_t ssmem[SEARCH_KINDS] = {};
     // tile shapes and the autotuner
     BatchTune tune{4, 128, 100, 1};
     bool fixed = false, tuned = false;
@@ -2964,7 +2964,7 @@ struct riv_batch {
 
 namespace {
 
-static int search_variant(const riv_encoder* e) { return e->table_ok ? (e->small_costs ? 0 : 1) : 2; }
+static int search_variant(const riv_encoder* e, bool table) { return search_multi_kind(table && e->table_ok, e->small_costs); }
 
 // Row CTAs of each clip of one search launch: about proportional to its MBs, at least one, at
 // most its MB rows, `total` in all (>= the number of clips).
@@ -3213,7 +3213,7 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
                     sps[a].tstride = 0;
                     kc[a].tab = nullptr;
                 }
-                pvar[a] = t.table ? search_variant(e) : 2;
+                pvar[a] = search_variant(e, t.table != 0);
                 step_pmbs += (uint64_t)e->NMB;
             }
         }
@@ -3227,9 +3227,9 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         }
         // search launches, one per variant present; each variant's parameters contiguous in kp,
         // its row CTAs spread over its clips
-        int stot[3] = {0, 0, 0}, sfirst[3] = {0, 0, 0}, scount[3] = {0, 0, 0};
+        int stot[SEARCH_KINDS] = {}, sfirst[SEARCH_KINDS] = {}, scount[SEARCH_KINDS] = {};
         int pos = 0;
-        for (int v = 0; v < 3; v++) {
+        for (int v = 0; v < SEARCH_KINDS; v++) {
             std::vector<int> mem, nmb, bh, rows;
             for (int a = 0; a < m; a++)
                 if (pvar[a] == v) { mem.push_back(a); nmb.push_back(kc[a].NMB); bh.push_back(kc[a].H / 16); }
@@ -3273,11 +3273,11 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         mark(TB_START);
         stage(BS_CONVERT, TB_CONVERT);
         stage(BS_TABLE, TB_TABLE);
-        for (int v = 0; v < 3; v++) {
+        for (int v = 0; v < SEARCH_KINDS; v++) {
             if (!stot[v]) continue;
             const SearchParams* dps = (const SearchParams*)(dd + b->off_sp) + sfirst[v];
             const int* dss = (const int*)(dd + b->off_sstart) + v * (n + 1);
-            CK(launch_search_multi(dps, dss, scount[v], stot[v], v < 2, v == 0, b->ssmem[v], b->sthreads[v], B));
+            CK(launch_search_multi(dps, dss, scount[v], stot[v], v, b->ssmem[v], b->sthreads[v], B));
             b->launches++;
         }
         mark(TB_SEARCH);
@@ -3420,7 +3420,7 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
         b->off_sp = al((size_t)n * sizeof(BatchClip));
         b->off_start = b->off_sp + al((size_t)n * sizeof(SearchParams));
         b->off_sstart = b->off_start + al((size_t)BS_N * (n + 1) * sizeof(int));
-        b->desc_bytes = b->off_sstart + al((size_t)3 * (n + 1) * sizeof(int));
+        b->desc_bytes = b->off_sstart + al((size_t)SEARCH_KINDS * (n + 1) * sizeof(int));
         for (int k = 0; k < 2; k++) {
             b->hdesc[k].alloc(b->desc_bytes);
             memset(b->hdesc[k].p, 0, b->desc_bytes);
@@ -3429,9 +3429,9 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
         int dev = 0, nsm = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        for (int v = 0; v < 3; v++) {
+        for (int v = 0; v < SEARCH_KINDS; v++) {
             int per_sm = 0;
-            CK(search_multi_capacity(v < 2, v == 0, b->max_sr, &per_sm, &b->ssmem[v], &b->sthreads[v]));
+            CK(search_multi_capacity(v, b->max_sr, &per_sm, &b->ssmem[v], &b->sthreads[v]));
             b->cap[v] = per_sm * nsm;
         }
         CK(cudaStreamSynchronize(b->B));

@@ -82,6 +82,7 @@ struct SearchParams {
     long long* prof;  // optional: RIV_PROF_WORDS words per MB (phase stamps, hexagon rounds), nullptr = off
     int nrow_ctas;    // CTAs that own MB rows (row stride); the rest of the grid are table workers
     int cta0;         // first CTA of this clip in a multi-clip launch (0 for a single clip)
+    int fused;        // the grid's CTAs beyond the row CTAs are workers
     int row_helpers;  // row CTAs run worker groups before their row starts and after it ends
     unsigned* tflag;  // fused table: per-MB flag = tag once its table row is written; nullptr = precomputed
     // Prediction and AQ inside the search launch (band + table instantiations): nullptr lnv =
@@ -187,9 +188,14 @@ struct BatchLaunch {
 };
 int batch_ctas_host(int stage, const BatchClip& k, const BatchTune& t);
 int launch_batch_stage(int stage, const BatchLaunch& b, const BatchTune& t, int total_ctas, int max_sr, void* stream);
-int search_multi_capacity(bool table, bool small, int max_sr, int* per_sm, size_t* smem, int* threads);
-int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total_ctas, bool table,
-                        bool small, size_t smem, int threads, void* stream);
+// Kinds of multi-clip search launches: 64- or 32-bit costs, with an exhaustive SAD table or with
+// the SADs computed on the way.
+constexpr int SEARCH_KINDS = 4;
+int search_multi_kind(bool table, bool small);
+bool search_multi_table(int kind);
+int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* threads);
+int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total_ctas, int kind, size_t smem,
+                        int threads, void* stream);
 
 enum StatusBits : unsigned {
     ST_WAIT_TIMEOUT = 1u,
@@ -199,10 +205,13 @@ enum StatusBits : unsigned {
 // Launchers (riv_kernels.cu).  All are asynchronous on `stream`.
 int launch_rgb_to_yuv(const uint8_t* rgb, int dw, int dh, uint8_t* yuv, int W, int H, void* stream, bool beside = false);
 int launch_yuv_to_rgb(const uint8_t* yuv, int W, int H, int dw, int dh, uint8_t* rgb, void* stream);
-// Launch plan of the search wavefront (chosen once per encoder).  fused: the SAD table is
-// computed inside the same cooperative launch by `grid - nrow` worker CTAs.
+// Launch plan of the search wavefront (chosen once per encoder).  fused: the SAD table (if any) and
+// the previous frame's reconstruction are worked on inside the same cooperative launch by
+// `grid - nrow` worker CTAs.
 struct SearchPlan {
-    bool fast;   // band + table instantiation: loader and AQ warps (prediction and AQ in the launch)
+    const void* fn;
+    bool fast;   // loader and AQ warps (prediction and AQ in the launch)
+    bool table;  // searches an exhaustive SAD table
     bool fused;
     bool helpers;  // fused: row CTAs' spare threads and finished row CTAs take worker tasks
     int grid, nrow, threads;
@@ -214,7 +223,6 @@ bool search_use_table(int sr);
 int sad_table_stride(int sr);
 int launch_sad_table(const uint8_t* ref, const uint8_t* cur, int W, int H, int sr, uint16_t* tab, int tstride,
                      void* stream);
-size_t search_smem_bytes(int sr);
 int launch_predict(const uint8_t* ref, const MbOut* mb, uint8_t* pred, uint2* varsum, int W, int H, void* stream);
 int launch_aq(const uint2* varsum, int n, float base, const uint32_t* logfix, int nlog, const uint32_t* expfix,
               int nexp, float* lnv_scratch, float* qs, void* stream);

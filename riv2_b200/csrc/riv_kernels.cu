@@ -238,6 +238,15 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// Row stride of the band: the frame's width and both margins, as an odd number of 16-byte chunks.
+// Then eight adjacent rows lie on eight different groups of four banks, and a load of one word of
+// each of 8 rows (the direct SADs) or 16 (half-pel, prediction) conflicts at most two ways; at
+// 1920 columns and a search range of 31 the plain width put every other row on the same banks
+// (seed round 1167 cycles, then 986; hexagon 2233, then 1917).
+__host__ __device__ inline int band_stride(int W, int sr) {
+    const int chunks = (W >> 4) + 2 * ((sr + 1 + 15) >> 4);
+    return 16 * (chunks | 1);
+}
 // Band layout (BAND mode): the reference rows y0-sr-1 .. y0+16+sr of the whole MB row,
 // columns -MARGIN .. W+MARGIN-1, MARGIN = round_up(sr+1, 16), filled 16-column chunk by
 // chunk with cp.async one MB ahead of use.
@@ -251,6 +260,26 @@ __device__ __forceinline__ void fill_chunk(uint8_t* band, int BWB, int WS, int c
             cp_async16(dst, ref + (size_t)gy * W + fx0);
         } else {
             uint32_t v = ref[(size_t)gy * W + (fx0 < 0 ? 0 : W - 1)] * 0x01010101u;
+            *(uint4*)dst = make_uint4(v, v, v, v);
+        }
+    }
+}
+
+
+// Per-MB window (DIRECT, no band): rows wy0 .. wy0 + WS - 1, columns fx0 .. fx0 + stride - 1 with
+// fx0 = x0 - MARGIN, a multiple of 16, in 16-byte chunks (cp.async; replicated borders by value).
+__host__ __device__ inline int search_window_stride(int sr) { return 16 + 2 * ((sr + 1 + 15) & ~15); }
+__device__ __forceinline__ void fill_window(uint8_t* win, int stride, int WS, int MARGIN, int fx0, int wy0,
+                                           const uint8_t* __restrict__ ref, int W, int H, int lane) {
+    const int nc = stride >> 4;
+    for (int i = lane; i < WS * nc; i += 32) {
+        const int r = i / nc, c = i - r * nc, fx = fx0 + 16 * c;
+        const uint8_t* src = ref + (size_t)min(max(wy0 + r, 0), H - 1) * W;
+        uint8_t* dst = win + r * stride + 16 * c;
+        if (fx >= 0 && fx < W) {
+            cp_async16(dst, src + fx);
+        } else {
+            const uint32_t v = src[fx < 0 ? 0 : W - 1] * 0x01010101u;
             *(uint4*)dst = make_uint4(v, v, v, v);
         }
     }
@@ -1184,10 +1213,12 @@ __device__ __forceinline__ bool wait_at_least(const unsigned* c, unsigned target
     return true;
 }
 // The rows / bands MB row r depends on before its reference samples may be read: the
-// previous frame's deblocked bands r-1 .. r+1 (or its residual rows when it has no deblock).
+// previous frame's deblocked bands (or its residual rows when it has no deblock) that its search
+// window of sr + 1 rows above and below touches, r-1 .. r+1 up to a search range of 15.
 __device__ __forceinline__ bool wait_ref_rows(const SearchParams& p, int r, int tiles_per_band) {
     if (!p.defer) return true;
-    for (int b = max(r - 1, 0); b <= min(r + 1, p.BH - 1); b++) {
+    const int k = (p.sr + 16) >> 4;
+    for (int b = max(r - k, 0); b <= min(r + k, p.BH - 1); b++) {
         const bool ok = p.db_level > 0 ? wait_at_least(p.wq + 1 + p.BH + b, (unsigned)tiles_per_band, p.spin_limit)
                                        : wait_at_least(p.wq + 1 + b, (unsigned)p.BW, p.spin_limit);
         if (!ok) return false;
@@ -1552,7 +1583,7 @@ __host__ __device__ inline int ld_slot_bytes(int tstride) { return 2 * tstride +
 __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long long* fullb, unsigned long long* bandb,
                                             volatile int* ctl, uint8_t* slots, uint8_t* band, volatile int* row_live) {
     const int lane = threadIdx.x & 31;
-    const int sr = p.sr, WS = 18 + 2 * sr, MARGIN = (sr + 1 + 15) & ~15, BWB = p.W + 2 * MARGIN;
+    const int sr = p.sr, WS = 18 + 2 * sr, MARGIN = (sr + 1 + 15) & ~15, BWB = band_stride(p.W, sr);
     const int SLOT = ld_slot_bytes(p.tstride);
     const unsigned tab_bytes = 2u * (unsigned)p.tstride;
     int n = 0, rows = 0;
@@ -1620,7 +1651,7 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
             if (lane < 16)
                 bulk_g2s(slot + tab_bytes + lane * 16, p.cur_y + (size_t)(r * 16 + lane) * p.W + bx * 16, 16u, fullb + s);
             if (lane == 0) {
-                bulk_g2s(slot, p.tab + (size_t)idx * p.tstride, tab_bytes, fullb + s);
+                if (tab_bytes != 0) bulk_g2s(slot, p.tab + (size_t)idx * p.tstride, tab_bytes, fullb + s);
                 const int tm = p.prev_coded ? *(const int*)(p.prev_coded + 4 * (size_t)idx) : 0;
                 *(int*)(slot + tab_bytes + 256) = tm;
                 mbar_arrive_tx(fullb + s, tab_bytes + 256u);
@@ -1656,7 +1687,7 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
 __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned long long* hand, volatile int* hand_done,
                                         volatile int* ctl, const uint8_t* band, unsigned long long* bandb) {
     const int lane = threadIdx.x & 31;
-    const int sr = p.sr, MARGIN = (sr + 1 + 15) & ~15, BWB = p.W + 2 * MARGIN;
+    const int sr = p.sr, MARGIN = (sr + 1 + 15) & ~15, BWB = band_stride(p.W, sr);
     const int W = p.W;
     uint8_t* PY = p.pred;
     const int yy = lane >> 1, xoff = (lane & 1) * 8;  // luma: row, 8-pixel half
@@ -1793,13 +1824,84 @@ __device__ __forceinline__ void aq_fold(const SearchParams& p, volatile int* ctl
     if (lane == 0) p.lnv[(size_t)p.BW * p.BH] = __fdiv_rn(part, (float)(p.BW * p.BH));
 }
 
+// Four positions at once: lane group g (lanes 8g .. 8g + 7) scores its own position, lane i of
+// the group rows 2i and 2i + 1 (16 samples each, current samples in cw: row 2i in cw[0..3], row
+// 2i + 1 in cw[4..7]); the group's sum ends in every lane of the group.  Five aligned words per
+// row cover the 16 unaligned bytes; `w(k, sh)` is the word at byte 4k + sh / 8 of them.
+__device__ __forceinline__ uint32_t ls_word(const uint32_t (&w)[5], int k, uint32_t sh) {
+    return sh >= 32u ? w[k + 1] : __funnelshift_r(w[k], w[k + 1], sh);
+}
+__device__ __forceinline__ void ls_row5(const uint8_t* win, int off, uint32_t (&w)[5], uint32_t& sh) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(win + off);
+    const uint32_t b = a & ~3u;
+    sh = (a & 3u) * 8u;
+#pragma unroll
+    for (int k = 0; k < 5; k++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[k]) : "r"(b + 4u * k));
+}
+__device__ __forceinline__ unsigned group_sum8(unsigned s) {
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    return s;
+}
+// A lane's part of a position's SAD over a search window or band: rows li and li + 8 of the block
+// at (x0, y0) (current samples cw), at position (dx, dy).  INSIDE: every position of the block's
+// search range lies in the frame, else the reference origin of each 4x4 sub-block is clamped
+// (sad_int_part's rule).  Plain loads and no reduction here, so that the loads and sums of several
+// batches overlap; a part is at most 32 * 255, so the sums of two batches share a word.
+// org: the view's origin as an offset into the CTA's shared memory (so that these are shared loads).
+template <bool INSIDE>
+__device__ __forceinline__ unsigned sad_part(const RefView& v, int org, int x0, int y0, int W, int H, int dx,
+                                             int dy, int li, const uint32_t (&cw)[8]) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    unsigned s = 0;
+    if (INSIDE) {
+        const int at = org + (y0 + li + dy - v.wy0) * v.stride + dx;
+        const uint32_t sh = ((uint32_t)at & 3u) * 8u;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t* q = (const uint32_t*)(smem + (at & ~3) + 8 * h * v.stride);  // strides are multiples of 16
+            const uint32_t w[5] = {q[0], q[1], q[2], q[3], q[4]};
+#pragma unroll
+            for (int k = 0; k < 4; k++) s += __vsadu4(__funnelshift_r(w[k], w[k + 1], sh), cw[4 * h + k]);
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int ry = min(max(y0 + ((li + 8 * h) & ~3) + dy, 0), H - 4) + (li & 3) - v.wy0;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                s += __vsadu4(lds_u32(smem + org + ry * v.stride + min(max(x0 + 4 * k + dx, 0), W - 4) - x0), cw[4 * h + k]);
+        }
+    }
+    return s;
+}
+// NB positions a group, a position a batch: straight-line code behind one branch, so that the
+// batches' loads and sums overlap (a branch a batch cost about 300 cycles each).
+template <int NB>
+__device__ __forceinline__ void sad_parts(const RefView& v, int org, bool inside, int x0, int y0, int W, int H,
+                                          const int (&dx)[NB], const int (&dy)[NB], int li, const uint32_t (&cw)[8],
+                                          unsigned (&sums)[NB]) {
+    if (inside) {
+#pragma unroll
+        for (int b = 0; b < NB; b++) sums[b] = sad_part<true>(v, org, x0, y0, W, H, dx[b], dy[b], li, cw);
+    } else {
+#pragma unroll
+        for (int b = 0; b < NB; b++) sums[b] = sad_part<false>(v, org, x0, y0, W, H, dx[b], dy[b], li, cw);
+    }
+}
+
 template <bool BAND, bool TABLE, bool SMALL>
 __device__ __forceinline__ void search_body(const SearchParams& p) {
-    // FAST (band + table): three warps -- search chain, mode decision, loader.  Otherwise the
-    // search warp stages its own data with cp.async and the third warp is not launched.
-    constexpr bool FAST = BAND && TABLE;
+    // FAST (band + 32-bit costs or table): search chain, mode decision, loader and AQ warps.
+    // Otherwise the search warp stages its own data with cp.async and only the mode warp runs
+    // beside it.  DIRECT (32-bit costs, no table): the integer SADs are computed on the chain, four
+    // positions at a time (8 lanes each).  1080p at search range 31: 0.99 ms a frame with the
+    // previous frame's reconstruction in the launch, where one position at a time on 64-bit costs,
+    // its prediction, AQ, residual and deblock in kernels of their own, took 1.60 ms.
+    constexpr bool FAST = BAND && (TABLE || SMALL), DIRECT = SMALL && !TABLE;
     extern __shared__ __align__(16) uint8_t smem[];
-    if (FAST && p.tflag != nullptr && row_cta(p) >= p.nrow_ctas) {
+    if (FAST && p.fused && row_cta(p) >= p.nrow_ctas) {
         frame_worker(p, smem);
         return;
     }
@@ -1824,7 +1926,8 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     const int sr = p.sr;
     const int WS = 18 + 2 * sr;
     const int MARGIN = (sr + 1 + 15) & ~15;
-    const int BWB = p.W + 2 * MARGIN;
+    const int BWB = band_stride(p.W, sr);
+    const int WSB = search_window_stride(sr);  // per-MB window (DIRECT, no band): row stride
     for (int i = threadIdx.x; i < 256; i += blockDim.x) bits[i] = p.mvbits[i];
     const int* nc32 = nc32s;
     if (SMALL)
@@ -1833,7 +1936,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     // Fused launch: threads 128-511 of a row CTA are worker groups 1-3 until the row starts
     // (region after the row layout: a live flag, then a 3-group worker region), and the
     // whole CTA joins the worker queue once its rows are done.
-    const bool helpers = FAST && p.tflag != nullptr && p.row_helpers;
+    const bool helpers = FAST && p.fused && p.row_helpers;
     uint8_t* pre = smem + (((size_t)(refmem - smem) + (size_t)WS * BWB + 16 + 15) & ~(size_t)15);
     volatile int* row_live = (volatile int*)pre;
     uint8_t* preg = pre + 16;
@@ -1877,6 +1980,15 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     const int xoff = (lane & 1) * 8;  // and its 8-pixel half
     bool failed = false;
     int hn = 0;  // MBs handed to the mode warp so far
+    // DIRECT: offsets of the candidates (g, 4 + g, 8 + g) that lane group g scores in a first round,
+    // hexagon 0-5 then diamond 6-9, a byte each
+    uint32_t round_x = 0, round_y = 0;
+    if (DIRECT)
+        for (int b = 0; b < 3; b++) {
+            const int k = 4 * b + (lane >> 3);
+            round_x |= (uint32_t)(k < 6 ? (0x01FFFEFF0102ull >> (8 * k)) & 255u : k < 10 ? (0x0000FF01u >> (8 * (k - 6))) & 255u : 0u) << (8 * b);
+            round_y |= (uint32_t)(k < 6 ? (0xFEFE00020200ull >> (8 * k)) & 255u : k < 10 ? (0xFF010000u >> (8 * (k - 6))) & 255u : 0u) << (8 * b);
+        }
 
     for (int r = row_cta(p); r < p.BH; r += p.nrow_ctas) {
         const int y0 = r * 16;
@@ -1898,6 +2010,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             for (int c = 0; c <= c_hi(0); c++) fill_chunk(refmem, BWB, WS, c, MARGIN, wy0, p.ref_y, p.W, p.H, lane);
             c_done = c_hi(0);
         }
+        if (DIRECT && !BAND) fill_window(refmem, WSB, WS, MARGIN, -MARGIN, wy0, p.ref_y, p.W, p.H, lane);
         if (!FAST) {
             if (lane < 16) cp_async16(curbuf + lane * 16, p.cur_y + (size_t)(y0 + lane) * p.W);
             if (TABLE)
@@ -1937,6 +2050,8 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                         fill_chunk(refmem, BWB, WS, c, MARGIN, wy0, p.ref_y, p.W, p.H, lane);
                     c_done = hi;
                 }
+                if (DIRECT && !BAND)
+                    fill_window(refmem + ((bx + 1) & 1) * (WS * WSB), WSB, WS, MARGIN, x0 + 16 - MARGIN, wy0, p.ref_y, p.W, p.H, lane);
                 RIV_STAMP(10);
                 if (lane < 16)
                     cp_async16(curbuf + ((bx + 1) & 1) * 256 + lane * 16, p.cur_y + (size_t)(y0 + lane) * p.W + x0 + 16);
@@ -1954,6 +2069,9 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             if (BAND) {
                 view.org = refmem + x0 + MARGIN;
                 view.stride = BWB;
+            } else if (DIRECT) {  // per-MB window, filled one MB ahead
+                view.org = refmem + (bx & 1) * (WS * WSB) + MARGIN;
+                view.stride = WSB;
             } else {
                 // per-MB window (large search ranges / very wide frames): rows wy0.., cols x0-sr-1..
                 const int wx0 = x0 - sr - 1;
@@ -2042,11 +2160,21 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                 Tmx = Tm_cod.dx; Tmy = Tm_cod.dy;
             }
             int sdx = 0, sdy = 0;
-            if constexpr (TABLE && SMALL) {
+            if constexpr (SMALL) {
                 // ---- seeds and nearest/near/median (enc/motion/scalar.rs:56-156) in a flat form:
                 // predictor slots 0..4 = left, top, top-right, top-left, temporal; lane 0 holds
                 // the (0,0) seed, lane 1+i predictor i when push_candidate keeps it.
-                const uint16_t* tb = FAST ? (const uint16_t*)lslot : tabbuf + (bx & 1) * p.tstride;
+                const uint16_t* tb = !TABLE ? nullptr : FAST ? (const uint16_t*)lslot : tabbuf + (bx & 1) * p.tstride;
+                // DIRECT: lane group g scores position g of a batch, lane li of it rows li and li + 8
+                const int g = lane >> 3, li = lane & 7;
+                const bool inside = x0 - sr >= 0 && y0 - sr >= 0 && x0 + 15 + sr < p.W && y0 + 15 + sr < p.H;
+                uint32_t cw[8];
+                if (DIRECT) {
+                    const uint4 r0 = *(const uint4*)(cb + 16 * li), r1 = *(const uint4*)(cb + 16 * (li + 8));
+                    cw[0] = r0.x; cw[1] = r0.y; cw[2] = r0.z; cw[3] = r0.w;
+                    cw[4] = r1.x; cw[5] = r1.y; cw[6] = r1.z; cw[7] = r1.w;
+                }
+                const int org = (int)(view.org - smem);
                 const int QX[5] = {L_raw.dx, Tx, TRx, TLx, Tmx}, QY[5] = {L_raw.dy, Ty, TRy, TLy, Tmy};
                 const unsigned pvm = (has_l ? 1u : 0u) | (has_t ? 2u : 0u) | (has_tr ? 4u : 0u) | (has_tl ? 8u : 0u) |
                                      (has_tm ? 16u : 0u);
@@ -2103,17 +2231,31 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                 };
                 RIV_STAMP(12);
                 // seed round: the in-order strict-'<' scan = argmin with the lowest slot winning ties
-                const int t0 = kv ? (int)tb[(ky + sr) * side + kx + sr] + cost(kx, ky) : 0;
+                int ksad = 0;  // this lane's candidate's SAD
+                if (TABLE) {
+                    if (kv) ksad = (int)tb[(ky + sr) * side + kx + sr];
+                } else {  // (a slot not kept scores (0,0): its position may lie outside the window)
+                    const int vx = kv ? kx : 0, vy = kv ? ky : 0;
+                    const int gx[2] = {__shfl_sync(0xffffffffu, vx, g), __shfl_sync(0xffffffffu, vx, 4 + g)};
+                    const int gy[2] = {__shfl_sync(0xffffffffu, vy, g), __shfl_sync(0xffffffffu, vy, 4 + g)};
+                    unsigned s2[2];
+                    sad_parts<2>(view, org, inside, x0, y0, p.W, p.H, gx, gy, li, cw, s2);
+                    const unsigned sums = group_sum8(s2[0] | (s2[1] << 16));
+                    const unsigned r = __shfl_sync(0xffffffffu, sums, 8 * (lane & 3));
+                    ksad = (int)(lane < 4 ? r & 0xffffu : r >> 16);
+                }
+                const int t0 = kv ? ksad + cost(kx, ky) : 0;
                 const uint32_t k0 = __reduce_min_sync(0xffffffffu, kv ? ((uint32_t)t0 << 3) | (uint32_t)lane : 0xffffffffu);
                 RIV_STAMP(13);
-                const int zero_sad = (int)tb[sr * side + sr];
+                const int zero_sad = TABLE ? (int)tb[sr * side + sr] : __shfl_sync(0xffffffffu, ksad, 0);
                 if (!(p.zthr > 0 && zero_sad <= p.zthr)) {  // else stay at (0,0)
                     int scost = (int)(k0 >> 3);
                     const int w0 = (int)(k0 & 7u);
                     sdx = w0 == 0 ? 0 : qx(w0 - 1);
                     sdy = w0 == 0 ? 0 : qy(w0 - 1);
                     RIV_STAMP(9);
-                    if (!(p.pthr > 0 && (int)tb[(sdy + sr) * side + sdx + sr] <= p.pthr)) {
+                    const int seed_sad = TABLE ? (int)tb[(sdy + sr) * side + sdx + sr] : __shfl_sync(0xffffffffu, ksad, w0);
+                    if (!(p.pthr > 0 && seed_sad <= p.pthr)) {
                         // hexagon (lanes 0-5, enc/motion/scalar.rs:694-729) and the small diamond
                         // around the same centre (lanes 6-9, :731-756) in one round: the diamond
                         // result is used when the hexagon does not improve.
@@ -2123,10 +2265,67 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                         const int oy = lane < 6 ? (int)(int8_t)(0xFEFE00020200ull >> (8 * ol))
                                                 : (lane < 10 ? (int)(int8_t)(0xFF010000u >> (8 * ol)) : 0);
                         int iter = 0;
+                        int moved = -1;  // DIRECT: the hexagon direction that led here
                         for (;;) {
                             const int cx = sdx + ox, cy = sdy + oy;
-                            const bool v = lane < 10 && abs(cx) <= sr && abs(cy) <= sr;
-                            const int t = v ? (int)tb[(cy + sr) * side + cx + sr] + cost(cx, cy) : 0;
+                            bool v = lane < 10 && abs(cx) <= sr && abs(cy) <= sr;
+                            int vsad = 0;
+                            if (TABLE) {
+                                if (v) vsad = (int)tb[(cy + sr) * side + cx + sr];
+                            } else {
+                                // After a move in direction m the points m + 2 .. m + 4 are the last
+                                // centre and two points of its round: they cost at least this centre's
+                                // cost, so the strict comparison never takes them and they are not
+                                // scored: three batches of four positions in the first round, two in
+                                // the next ones.
+                                const bool first = moved < 0;
+                                int idx = lane;  // this lane's candidate's place in the batches
+                                if (!first) {
+                                    const int d = lane + 1 - moved;  // hexagon: directions m - 1, m, m + 1
+                                    idx = lane >= 6 ? lane - 3 : d < 0 ? d + 6 : d >= 6 ? d - 6 : d;
+                                    v = v && (lane >= 6 || idx < 3);
+                                }
+                                // positions out of range score the centre (never used)
+                                auto clip = [&](int& gx, int& gy) {
+                                    const bool in = abs(sdx + gx) <= sr && abs(sdy + gy) <= sr;
+                                    gx = in ? sdx + gx : sdx;
+                                    gy = in ? sdy + gy : sdy;
+                                };
+                                if (first) {
+                                    int gx[3], gy[3];
+                                    unsigned sums[3];
+#pragma unroll
+                                    for (int b = 0; b < 3; b++) {
+                                        gx[b] = (int)(int8_t)(round_x >> (8 * b));
+                                        gy[b] = (int)(int8_t)(round_y >> (8 * b));
+                                        clip(gx[b], gy[b]);
+                                    }
+                                    sad_parts<3>(view, org, inside, x0, y0, p.W, p.H, gx, gy, li, cw, sums);
+                                    const unsigned s01 = group_sum8(sums[0] | (sums[1] << 16)), s2 = group_sum8(sums[2]);
+                                    const unsigned r01 = __shfl_sync(0xffffffffu, s01, 8 * (lane & 3));
+                                    const unsigned r2 = __shfl_sync(0xffffffffu, s2, 8 * (lane & 3));
+                                    vsad = (int)(lane < 4 ? r01 & 0xffffu : lane < 8 ? r01 >> 16 : r2);
+                                } else {
+                                    int gx[2], gy[2];
+                                    unsigned sums[2];
+#pragma unroll
+                                    for (int b = 0; b < 2; b++) {  // this group's candidate of the batch, as a lane's
+                                        const int c = 4 * b + g;
+                                        int k = moved + 5 + c;
+                                        k = c >= 3 ? c + 3 : k >= 12 ? k - 12 : k >= 6 ? k - 6 : k;
+                                        gx[b] = k < 6 ? (int)(int8_t)(0x01FFFEFF0102ull >> (8 * k))
+                                                      : k < 10 ? (int)(int8_t)(0x0000FF01u >> (8 * (k - 6))) : 0;
+                                        gy[b] = k < 6 ? (int)(int8_t)(0xFEFE00020200ull >> (8 * k))
+                                                      : k < 10 ? (int)(int8_t)(0xFF010000u >> (8 * (k - 6))) : 0;
+                                        clip(gx[b], gy[b]);
+                                    }
+                                    sad_parts<2>(view, org, inside, x0, y0, p.W, p.H, gx, gy, li, cw, sums);
+                                    const unsigned s01 = group_sum8(sums[0] | (sums[1] << 16));
+                                    const unsigned r01 = __shfl_sync(0xffffffffu, s01, 8 * (idx & 3));
+                                    vsad = (int)(idx < 4 ? r01 & 0xffffu : r01 >> 16);
+                                }
+                            }
+                            const int t = v ? vsad + cost(cx, cy) : 0;
                             const uint32_t kh = __reduce_min_sync(
                                 0xffffffffu, v && lane < 6 ? ((uint32_t)t << 3) | (uint32_t)lane : 0xffffffffu);
                             const uint32_t kd = __reduce_min_sync(
@@ -2136,6 +2335,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                                 scost = (int)(kh >> 3);
                                 sdx += (int)(int8_t)(0x01FFFEFF0102ull >> (8 * w));
                                 sdy += (int)(int8_t)(0xFEFE00020200ull >> (8 * w));
+                                moved = w;
                                 if (++iter > 4096) {  // cost strictly decreases, so this is never reached
                                     if (lane == 0) atomicOr(p.status, ST_HEX_CAP);
                                     break;
@@ -2503,95 +2703,107 @@ __global__ void __maxnreg__(120) k_search(SearchParams p) {
 }
 
 // Shared memory of the search kernel; BAND when the whole MB-row band fits, TABLE when
-// the exhaustive SAD table is used (search ranges up to 15).
+// the exhaustive SAD table is used (search ranges up to 15), DIRECT when the SADs are computed
+// on the chain (32-bit costs).
 int sad_table_stride(int sr) { return ((2 * sr + 1) * (2 * sr + 1) + 7) & ~7; }
 bool search_use_table(int sr) { return sr <= 15; }
-static size_t search_smem(int sr, int W, bool band, bool table) {
+// A fused launch without a table needs fewer CTAs beside the rows: the row CTAs' spare warps take
+// worker tasks too until their row starts (2160 rows of MBs leave 13).
+constexpr int SEARCH_DIRECT_WORKERS = 8;
+enum SearchKind { SK_TABLE_SMALL, SK_TABLE, SK_DIRECT, SK_PLAIN };  // PLAIN: 64-bit costs, no table
+static bool search_fast(bool band, SearchKind k) { return band && k != SK_PLAIN; }
+static size_t search_smem(int sr, int W, bool band, SearchKind k) {
+    const bool table = k == SK_TABLE_SMALL || k == SK_TABLE;
     size_t ws = 18 + 2 * (size_t)sr;
-    size_t margin = ((size_t)sr + 1 + 15) & ~(size_t)15;
-    size_t ref = band ? ws * ((size_t)W + 2 * margin) : ws * ws;
+    size_t ref = band ? ws * (size_t)band_stride(W, sr) : k == SK_DIRECT ? 2 * ws * search_window_stride(sr) : ws * ws;
     size_t head = 256 * sizeof(double) + 64 * 64 * 4 + HAND_RING * 8 + 16;
-    if (band && table) return head + 64 + 1024 + LD_RING * (size_t)ld_slot_bytes(sad_table_stride(sr)) + ref + 16;
-    return head + 512 + (table ? 4 * (size_t)sad_table_stride(sr) : 0) + ref + 16;
+    const int stride = table ? sad_table_stride(sr) : 0;
+    if (search_fast(band, k)) return head + 64 + 1024 + LD_RING * (size_t)ld_slot_bytes(stride) + ref + 16;
+    return head + 512 + 4 * (size_t)stride + ref + 16;
 }
-static int search_threads(bool band, bool table) { return band && table ? 128 : 64; }
+static int search_threads(bool fast) { return fast ? 128 : 64; }
 static const size_t SEARCH_SMEM_MAX = 200 * 1024;
-static bool search_use_band(int sr, int W) {
-    return search_smem(sr, W, true, search_use_table(sr)) <= SEARCH_SMEM_MAX;
+static const void* search_fn(bool band, SearchKind k) {
+    switch (k) {
+        case SK_TABLE_SMALL: return band ? (const void*)k_search<true, true, true> : (const void*)k_search<false, true, true>;
+        case SK_TABLE: return band ? (const void*)k_search<true, true, false> : (const void*)k_search<false, true, false>;
+        case SK_DIRECT: return band ? (const void*)k_search<true, false, true> : (const void*)k_search<false, false, true>;
+        default: return band ? (const void*)k_search<true, false, false> : (const void*)k_search<false, false, false>;
+    }
 }
-static const void* search_fn(bool band, bool table, bool small) {
-    if (table && small) return band ? (const void*)k_search<true, true, true> : (const void*)k_search<false, true, true>;
-    if (table) return band ? (const void*)k_search<true, true, false> : (const void*)k_search<false, true, false>;
-    return band ? (const void*)k_search<true, false, false> : (const void*)k_search<false, false, false>;
-}
-
-size_t search_smem_bytes(int sr) { return search_smem(sr, 0, false, search_use_table(sr)); }
 
 int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) {
-    const bool band = search_use_band(sr, W);
-    const void* fn = search_fn(band, table, table && small);
-    const int threads = search_threads(band, table);
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
+    const void* fn = nullptr;
     auto resident = [&](size_t sm, int nthreads, int* per_sm) {
         cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nthreads, sm);
         return r;
     };
-    const size_t sm = search_smem(sr, W, band, table);
-    SearchPlan pl{};
-    pl.threads = threads;
-    pl.fast = band && table;
-    if (band && table) {
-        // fused: one CTA per SM (the shared-memory request rules out a second), rows first,
-        // table workers on the SMs the rows leave free -- used when enough of them remain
-        // row CTAs' helper region (live flag + three worker groups) after the row layout,
-        // where the per-CTA maximum allows it
-        const size_t with_helpers = ((sm + 15) & ~(size_t)15) + 16 + (size_t)worker_region_bytes(3);
-        const bool helpers = with_helpers <= (size_t)227 * 1024;
-        const size_t need = helpers ? with_helpers : sm;
-        const size_t smf = need > (size_t)116 * 1024 ? need : (size_t)116 * 1024;
+    auto use_band = [&](SearchKind k) { return search_smem(sr, W, true, k) <= SEARCH_SMEM_MAX; };
+    // The plan of one kind: fused when it can be, else one CTA per MB row (as many as fit).
+    // fused: one CTA per SM (the shared-memory request rules out a second), rows first, workers on
+    // the SMs the rows leave free; a table's MBs need at least 32 of those.
+    auto plan = [&](SearchKind k, SearchPlan& pl) -> cudaError_t {
+        const bool band = use_band(k), tab = k == SK_TABLE_SMALL || k == SK_TABLE;
+        const size_t sm = search_smem(sr, W, band, k);
+        fn = search_fn(band, k);
+        pl = SearchPlan{};
+        pl.fn = fn;
+        pl.fast = search_fast(band, k);
+        pl.table = tab;
         int per_sm = 0;
-        e = resident(smf, 4 * 128, &per_sm);
-        if (e != cudaSuccess) return (int)e;
-        const int total = per_sm * nsm;
-        const int nrow = BH < total ? BH : total;
-        const size_t gsm = ((size_t)sad_table_smem(sr) + 15) & ~(size_t)15;
-        if (per_sm == 1 && total - nrow >= 32 && 4 * gsm <= smf) {
-            pl.fused = true;
-            pl.helpers = helpers;
-            pl.threads = 4 * 128;  // row CTAs use three warps; table workers four groups of 128
-            pl.smem = smf;
-            pl.nrow = nrow;
-            pl.grid = total;
-            *out = pl;
-            return 0;
+        if (pl.fast) {
+            // row CTAs' helper region (live flag + three worker groups) after the row layout,
+            // where the per-CTA maximum allows it
+            const size_t with_helpers = ((sm + 15) & ~(size_t)15) + 16 + (size_t)worker_region_bytes(3);
+            const bool helpers = with_helpers <= (size_t)227 * 1024;
+            const size_t need = helpers ? with_helpers : sm;
+            const size_t smf = need > (size_t)116 * 1024 ? need : (size_t)116 * 1024;
+            cudaError_t r = resident(smf, 4 * 128, &per_sm);
+            if (r != cudaSuccess) return r;
+            const int total = per_sm * nsm;
+            const int nrow = BH < total ? BH : total;
+            const size_t gsm = tab ? ((size_t)sad_table_smem(sr) + 15) & ~(size_t)15 : 0;
+            if (per_sm == 1 && total - nrow >= (tab ? 32 : SEARCH_DIRECT_WORKERS) && 4 * gsm <= smf) {
+                pl.fused = true;
+                pl.helpers = helpers;
+                pl.threads = 4 * 128;  // row CTAs use four warps; workers four groups of 128
+                pl.smem = smf;
+                pl.nrow = nrow;
+                pl.grid = total;
+                return cudaSuccess;
+            }
         }
-    }
-    int per_sm = 0;
-    e = resident(sm, threads, &per_sm);
-    if (e != cudaSuccess) return (int)e;
-    pl.fused = false;
-    pl.smem = sm;
-    pl.grid = pl.nrow = BH < per_sm * nsm ? BH : per_sm * nsm;
-    *out = pl;
-    return 0;
+        pl.threads = search_threads(pl.fast);
+        cudaError_t r = resident(sm, pl.threads, &per_sm);
+        if (r != cudaSuccess) return r;
+        pl.smem = sm;
+        pl.grid = pl.nrow = BH < per_sm * nsm ? BH : per_sm * nsm;
+        return cudaSuccess;
+    };
+    // A table wherever there is one: its chain is 1100 cycles a MB shorter (at 2160 rows a table
+    // kernel, the search, the residual and the deblock take 1.9 ms a frame, a fused direct launch
+    // 2.4 ms; at 1080 rows 0.63 ms against 0.99).
+    e = plan(table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN, *out);
+    return (int)e;
 }
 
 int launch_search(const SearchParams& p, const SearchPlan& plan, void* stream) {
-    const bool band = search_use_band(p.sr, p.W), table = p.tab != nullptr;
     SearchParams q = p;
     q.nrow_ctas = plan.nrow;
+    q.fused = plan.fused ? 1 : 0;
     q.row_helpers = plan.fused && plan.helpers ? 1 : 0;
     if (!plan.fused) q.tflag = nullptr;
     void* args[] = {&q};
     // Cooperative launch: every CTA of the grid is co-resident, so the row-to-row waits
     // and the waits for table rows can always make progress.
-    cudaError_t e = cudaLaunchCooperativeKernel(search_fn(band, table, table && p.small), dim3(plan.grid),
-                                                dim3(plan.threads), args, plan.smem, (cudaStream_t)stream);
+    cudaError_t e = cudaLaunchCooperativeKernel(plan.fn, dim3(plan.grid), dim3(plan.threads), args, plan.smem,
+                                                (cudaStream_t)stream);
     return (int)e;
 }
 
@@ -2721,26 +2933,6 @@ __device__ __forceinline__ unsigned ls_sad_hp(const uint8_t* win, int ws, int ox
     return __reduce_add_sync(0xffffffffu, s);
 }
 
-// Four positions at once: lane group g (lanes 8g .. 8g + 7) scores its own position, lane i of
-// the group rows 2i and 2i + 1 (16 samples each, current samples in cw: row 2i in cw[0..3], row
-// 2i + 1 in cw[4..7]); the group's sum ends in every lane of the group.  Five aligned words per
-// row cover the 16 unaligned bytes; `w(k, sh)` is the word at byte 4k + sh / 8 of them.
-__device__ __forceinline__ uint32_t ls_word(const uint32_t (&w)[5], int k, uint32_t sh) {
-    return sh >= 32u ? w[k + 1] : __funnelshift_r(w[k], w[k + 1], sh);
-}
-__device__ __forceinline__ void ls_row5(const uint8_t* win, int off, uint32_t (&w)[5], uint32_t& sh) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(win + off);
-    const uint32_t b = a & ~3u;
-    sh = (a & 3u) * 8u;
-#pragma unroll
-    for (int k = 0; k < 5; k++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[k]) : "r"(b + 4u * k));
-}
-__device__ __forceinline__ unsigned group_sum8(unsigned s) {
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    return s;
-}
 // whole-pixel offset (dx, dy)
 __device__ __forceinline__ unsigned ls_sad_g(const uint8_t* win, int ws, int ox, int oy, int dx, int dy, int li,
                                              const uint32_t (&cw)[8]) {

@@ -1979,7 +1979,19 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     const int yy = lane >> 1;         // this lane's row inside the MB
     const int xoff = (lane & 1) * 8;  // and its 8-pixel half
     bool failed = false;
-    int hn = 0;  // MBs handed to the mode warp so far
+    int hn = 0;     // MBs handed to the mode warp so far
+    int taken = 0;  // MBs that the mode and AQ warps had taken when the ring was last looked at
+    // half-pel: lane q < 9 holds candidate q = (sy + 1) * 3 + sx + 1; which pair sum it takes and from
+    // which half, its offsets and its place in the scan order (the centre first)
+    const uint32_t hp_m[5] = {lane < 2 ? ~0u : 0u, lane == 2 || lane == 3 ? ~0u : 0u, lane == 4 || lane == 5 || lane > 8 ? ~0u : 0u,
+                              lane == 6 || lane == 7 ? ~0u : 0u, lane == 8 ? ~0u : 0u};
+    const int hp_shift = (lane & 1) * 16, hp_sx = lane % 3 - 1, hp_sy = lane / 3 - 1;
+    const uint32_t hp_ord = lane == 4 ? 0u : lane < 4 ? (uint32_t)lane + 1u : (uint32_t)lane & 15u;
+    // the seed of lanes 1 .. 4 (left, top, top-right, top-left) as two bytes of two words, lane 5's
+    // (temporal) as a mask: written as a choice by lane number it became a switch of divergent
+    // branches, 450 cycles of the chain
+    const uint32_t seed_sel = 0x10u + 0x22u * (uint32_t)((lane - 1) & 3), seed_mask = lane >= 1 && lane <= 4 ? 0xffffu : 0u,
+                   temp_mask = lane == 5 ? 0xffffu : 0u;
     // DIRECT: offsets of the candidates (g, 4 + g, 8 + g) that lane group g scores in a first round,
     // hexagon 0-5 then diamond 6-9, a byte each
     uint32_t round_x = 0, round_y = 0;
@@ -2019,18 +2031,15 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             cp_async_commit();
         }
 
-        MvT L_raw{0, 0, 0, 0};
-        unsigned long long recT = 0, recTL = 0, pref = 0;
+        // raw MVs of the left, top and top-left neighbours as dx << 8 | dy (bytes; 0 when there is
+        // none), as in the records' bits 47 .. 32
+        uint32_t pL = 0, pT = 0, pTL = 0;
+        unsigned long long pref = 0;
         for (int bx = 0; bx < p.BW; bx++) {
             const int x0 = bx * 16;
             const int idx = r * p.BW + bx;
             RIV_STAMP(0);
             if (lane == 0) RIV_GSTAMP(idx, 16);
-            // Refresh the prefetched top-right record now if it was not published yet when it
-            // was first read: the load's latency then overlaps the slot wait below instead of
-            // sitting on the chain at the wait for the row above.
-            if (r > 0 && lane == 0 && (pref & 0xffff000000000000ull) != tagbits)
-                pref = ld_rec(p.rec + (r - 1) * p.BW + min(bx + 1, p.BW - 1));
             // ---- FAST: wait for the loader's slot; otherwise prefetch MB bx+1 (columns, current
             // block, table row) and wait for MB bx's data
             const uint8_t* lslot = slots + (size_t)(ln & (LD_RING - 1)) * ld_slot_bytes(p.tstride);
@@ -2101,37 +2110,29 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             const uint32_t c1 = *(const uint32_t*)(cb + yy * 16 + xoff + 4);
 
             RIV_STAMP(1);
-            // ---- wait for the row above (top-right, or top at the last column).  The record
-            // of the next MB's top-right was requested one MB earlier (pref); it is polled
-            // again only if it had not been published yet.
-            unsigned long long recTR = 0;
-            bool has_tr = false;
+            // ---- wait for the row above (top-right, or top at the last column).  The record was
+            // requested when the MB before was published (pref); it is polled again only if it had
+            // not been published yet.  Requested earlier, right after the last wait, it was rarely
+            // there yet and had to be asked for again: 1080p 583 us a frame, 549 like this (a request
+            // before the half-pel search: 559).
+            uint32_t pTR = 0;
+            const bool has_tr = r > 0 && bx + 1 < p.BW;
             if (r > 0) {
-                int wi = (r - 1) * p.BW + min(bx + 1, p.BW - 1);
-                unsigned long long v = 0;
-                if (lane == 0) {
-                    long long spins = 0;
-                    v = pref;
-                    if ((v & 0xffff000000000000ull) != tagbits) v = ld_rec(p.rec + wi);
-                    while ((v & 0xffff000000000000ull) != tagbits) {
-                        if (++spins > p.spin_limit || failed) { failed = true; break; }
-                        __nanosleep(20);
-                        v = ld_rec(p.rec + wi);
-                    }
-                    if (bx == 0 && !failed) {  // the top record, checked like every other
-                        recT = ld_rec(p.rec + (r - 1) * p.BW);
-                        while ((recT & 0xffff000000000000ull) != tagbits) {
-                            if (++spins > p.spin_limit) { failed = true; break; }
-                            __nanosleep(20);
-                            recT = ld_rec(p.rec + (r - 1) * p.BW);
-                        }
-                    }
-                    pref = bx + 1 < p.BW ? ld_rec(p.rec + (r - 1) * p.BW + min(bx + 2, p.BW - 1)) : 0ull;
+                // Every lane loads the record (one request), so that in the usual case, when it is
+                // there, nothing diverges and nothing is passed from lane to lane.
+                unsigned long long v = pref;
+                if (!__all_sync(0xffffffffu, (v & 0xffff000000000000ull) == tagbits)) {
+                    // lane 0 polls; at the row's first MB (no record prefetched) lane 1 polls the top
+                    // record beside it
+                    if (lane < (bx == 0 ? 2 : 1) &&
+                        !rec_wait(p.rec + (r - 1) * p.BW + (lane == 0 ? min(bx + 1, p.BW - 1) : 0), tagbits, v, p.spin_limit))
+                        failed = true;
+                    failed = __any_sync(0xffffffffu, failed);
+                    if (bx == 0) pT = __shfl_sync(0xffffffffu, (uint32_t)(v >> 32) & 0xffffu, 1);
+                    v = __shfl_sync(0xffffffffu, v, 0);
                 }
-                failed = __shfl_sync(0xffffffffu, (int)failed, 0) != 0;
-                v = __shfl_sync(0xffffffffu, v, 0);
-                recT = __shfl_sync(0xffffffffu, recT, 0);
-                if (bx + 1 < p.BW) { recTR = v; has_tr = true; }
+                const uint32_t got = (uint32_t)(v >> 32) & 0xffffu;
+                if (has_tr) pTR = got;
             }
             if (failed) {
                 if (lane == 0) {
@@ -2144,26 +2145,19 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             }
             RIV_STAMP(2);
             const bool has_t = r > 0, has_l = bx > 0, has_tl = r > 0 && bx > 0;
-            auto rec_raw = [](unsigned long long v, int& dx, int& dy) {
-                dx = (int)(int8_t)(v >> 40); dy = (int)(int8_t)(v >> 32);
-            };
-            int Tx = 0, Ty = 0, TRx = 0, TRy = 0, TLx = 0, TLy = 0;
-            if (has_t) rec_raw(recT, Tx, Ty);
-            if (has_tr) rec_raw(recTR, TRx, TRy);
-            if (has_tl) rec_raw(recTL, TLx, TLy);
             const bool has_tm = p.prev_coded != nullptr;
-            int Tmx = 0, Tmy = 0;
-            MvT Tm_cod{0, 0, 0, 0};
+            auto px = [](uint32_t q) { return (int)(int8_t)(q >> 8); };
+            auto py = [](uint32_t q) { return (int)(int8_t)q; };
+            uint32_t pTm = 0;
             if (has_tm) {
                 const char4 pc = FAST ? *(const char4*)(lslot + 2 * p.tstride + 256) : *(const char4*)(p.prev_coded + 4 * idx);
-                Tm_cod = MvT{pc.x, pc.y, pc.z, pc.w};
-                Tmx = Tm_cod.dx; Tmy = Tm_cod.dy;
+                pTm = (uint32_t)(uint8_t)pc.x << 8 | (uint32_t)(uint8_t)pc.y;
             }
             int sdx = 0, sdy = 0;
             if constexpr (SMALL) {
-                // ---- seeds and nearest/near/median (enc/motion/scalar.rs:56-156) in a flat form:
-                // predictor slots 0..4 = left, top, top-right, top-left, temporal; lane 0 holds
-                // the (0,0) seed, lane 1+i predictor i when push_candidate keeps it.
+                // ---- seeds and nearest/near/median (enc/motion/scalar.rs:56-156) on packed MVs: lane 0
+                // holds the (0,0) seed, lanes 1 .. 5 the left, top, top-right, top-left and temporal
+                // predictors: 255 cycles, with its stamps, of the chain.
                 const uint16_t* tb = !TABLE ? nullptr : FAST ? (const uint16_t*)lslot : tabbuf + (bx & 1) * p.tstride;
                 // DIRECT: lane group g scores position g of a batch, lane li of it rows li and li + 8
                 const int g = lane >> 3, li = lane & 7;
@@ -2175,51 +2169,32 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                     cw[4] = r1.x; cw[5] = r1.y; cw[6] = r1.z; cw[7] = r1.w;
                 }
                 const int org = (int)(view.org - smem);
-                const int QX[5] = {L_raw.dx, Tx, TRx, TLx, Tmx}, QY[5] = {L_raw.dy, Ty, TRy, TLy, Tmy};
-                const unsigned pvm = (has_l ? 1u : 0u) | (has_t ? 2u : 0u) | (has_tr ? 4u : 0u) | (has_tl ? 8u : 0u) |
-                                     (has_tm ? 16u : 0u);
-                unsigned long long X5 = 0, Y5 = 0;
-                unsigned okm = 0;
-#pragma unroll
-                for (int i = 0; i < 5; i++) {
-                    X5 |= (unsigned long long)(uint8_t)QX[i] << (8 * i);
-                    Y5 |= (unsigned long long)(uint8_t)QY[i] << (8 * i);
-                    const bool ok = ((pvm >> i) & 1u) && abs(QX[i]) <= sr && abs(QY[i]) <= sr && (QX[i] | QY[i]) != 0;
-                    okm |= ok ? (1u << i) : 0u;
-                }
-                auto qx = [&](int i) { return (int)(int8_t)(X5 >> (8 * i)); };
-                auto qy = [&](int i) { return (int)(int8_t)(Y5 >> (8 * i)); };
-                int nix = 0, niy = 0, rix = 0, riy = 0;
-                if (pvm) {  // nearest = first available; near = first later one that differs
-                    const int ni = __ffs(pvm) - 1;
-                    nix = qx(ni);
-                    niy = qy(ni);
-                    unsigned dm = 0;
-#pragma unroll
-                    for (int i = 0; i < 5; i++) dm |= (QX[i] != nix || QY[i] != niy) ? (1u << i) : 0u;
-                    const unsigned rm = pvm & dm & ~((2u << ni) - 1u);
-                    if (rm) {
-                        const int ri = __ffs(rm) - 1;
-                        rix = qx(ri);
-                        riy = qy(ri);
-                    }
-                }
-                const int mdx = median3(L_raw.dx, Tx, has_tr ? TRx : TLx), mdy = median3(L_raw.dy, Ty, has_tr ? TRy : TLy);
-                int kx = 0, ky = 0;
-                bool kv = lane == 0;
-                if (lane >= 1 && lane <= 5) {
-                    const int ci = lane - 1;
-                    kx = qx(ci);
-                    ky = qy(ci);
-                    unsigned eq = 0;
-#pragma unroll
-                    for (int j = 0; j < 5; j++) eq |= (QX[j] == kx && QY[j] == ky) ? (1u << j) : 0u;
-                    kv = ((okm >> ci) & 1u) && (eq & okm & ((1u << ci) - 1u)) == 0;
-                }
+                // nearest = first available; near = first other one that differs (all lanes alike).  By
+                // masks: conditions that are the same in every lane become branches otherwise, and
+                // a dozen of those cost 200 cycles here.
+                const uint32_t mL = has_l ? ~0u : 0u, mT = has_t ? ~0u : 0u, mTR = has_tr ? ~0u : 0u, mTL = mL & mT,
+                               mTm = has_tm ? ~0u : 0u;
+                auto sel = [](uint32_t m, uint32_t a, uint32_t b) { return (a & m) | (b & ~m); };
+                auto differs = [](uint32_t a, uint32_t b) { return (uint32_t)((int32_t)(0u - (a ^ b)) >> 31); };  // 16-bit values
+                const uint32_t pn = sel(mL, pL, sel(mT, pT, sel(mTR, pTR, sel(mTL, pTL, pTm))));
+                const uint32_t pr = sel(mT & differs(pT, pn), pT, sel(mTR & differs(pTR, pn), pTR,
+                                        sel(mTL & differs(pTL, pn), pTL, pTm & mTm & differs(pTm, pn))));
+                const int nix = px(pn), niy = py(pn), rix = px(pr), riy = py(pr);
+                auto med = [](int a, int b, int c) { return max(min(a, b), min(max(a, b), c)); };
+                const uint32_t pq = sel(mTR, pTR, pTL);
+                const int mdx = med(px(pL), px(pT), px(pq)), mdy = med(py(pL), py(pT), py(pq));
+                // this lane's seed, and whether push_candidate keeps it: available, in range, not zero
+                // and not equal to one kept before
+                const uint32_t mine = (__byte_perm(pL | pT << 16, pTR | pTL << 16, seed_sel) & seed_mask) | (pTm & temp_mask);
+                const int kx = px(mine), ky = py(mine);
+                const unsigned pvm = (mL & 2u) | (mT & 4u) | (mTR & 8u) | (mTL & 16u) | (mTm & 32u);
+                const unsigned okm = __ballot_sync(0xffffffffu, ((pvm >> lane) & 1u) != 0u && mine != 0u && abs(kx) <= sr && abs(ky) <= sr);
+                const unsigned same = (pL == mine ? 2u : 0u) | (pT == mine ? 4u : 0u) | (pTR == mine ? 8u : 0u) | (pTL == mine ? 16u : 0u);
+                const bool kv = lane == 0 || (((okm >> lane) & 1u) != 0u && (same & okm & ((1u << lane) - 1u)) == 0u);
                 const int c15i = (int)p.c15, c05i = (int)p.c05;
                 // estimate_mv_cost (enc/motion/scalar.rs:453-544), every term below 2^27 here
+                // (with lambda 0 all of them are 0)
                 auto cost = [&](int cx, int cy) -> int {
-                    if (p.lambda_zero) return 0;
                     int best = INT_MAX;
                     if ((cx == nix && cy == niy) || (cx == rix && cy == riy) || (cx == mdx && cy == mdy)) best = c15i;
                     if ((cx | cy) == 0) best = min(best, c05i);
@@ -2251,8 +2226,9 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                 if (!(p.zthr > 0 && zero_sad <= p.zthr)) {  // else stay at (0,0)
                     int scost = (int)(k0 >> 3);
                     const int w0 = (int)(k0 & 7u);
-                    sdx = w0 == 0 ? 0 : qx(w0 - 1);
-                    sdy = w0 == 0 ? 0 : qy(w0 - 1);
+                    const uint32_t seed = __shfl_sync(0xffffffffu, mine, w0);
+                    sdx = px(seed);
+                    sdy = py(seed);
                     RIV_STAMP(9);
                     const int seed_sad = TABLE ? (int)tb[(sdy + sr) * side + sdx + sr] : __shfl_sync(0xffffffffu, ksad, w0);
                     if (!(p.pthr > 0 && seed_sad <= p.pthr)) {
@@ -2356,7 +2332,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             } else {
                 // ---- seeds, nearest/near/median (enc/motion/scalar.rs:56-156).  Predictor slots in
                 // the reference's order: left, top, top-right, top-left, temporal.
-                const int PX[5] = {L_raw.dx, Tx, TRx, TLx, Tmx}, PY[5] = {L_raw.dy, Ty, TRy, TLy, Tmy};
+                const int PX[5] = {px(pL), px(pT), px(pTR), px(pTL), px(pTm)}, PY[5] = {py(pL), py(pT), py(pTR), py(pTL), py(pTm)};
                 const bool PV[5] = {has_l, has_t, has_tr, has_tl, has_tm};
                 CostCtx cc;
                 cc.nx = cc.ny = cc.rx = cc.ry = 0;
@@ -2369,11 +2345,9 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                         else if (take && nu == 1) { cc.rx = PX[i]; cc.ry = PY[i]; }
                         nu += take ? 1 : 0;
                     }
-                    int lx = has_l ? L_raw.dx : 0, ly = has_l ? L_raw.dy : 0;
-                    int tx = has_t ? Tx : 0, ty = has_t ? Ty : 0;
-                    int qx = has_tr ? TRx : (has_tl ? TLx : 0), qy = has_tr ? TRy : (has_tl ? TLy : 0);
-                    cc.mx = median3(lx, tx, qx);
-                    cc.my = median3(ly, ty, qy);
+                    const uint32_t pq = has_tr ? pTR : pTL;
+                    cc.mx = median3(px(pL), px(pT), px(pq));
+                    cc.my = median3(py(pL), py(pT), py(pq));
                 }
                 // seed slots: 0 = (0,0), 1..5 = predictors kept if within range and not already
                 // pushed (push_candidate, enc/motion/scalar.rs:46-53)
@@ -2563,30 +2537,42 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                     uint32_t al = sa & ~3u, o = sa & 3u;
                     uint32_t w0 = lds_aligned(al), w1 = lds_aligned(al + 4), w2 = lds_aligned(al + 8),
                              w3 = lds_aligned(al + 12);
-                    // byte offsets o, o+1, o+2 into w0..w3
-                    uint32_t sh = o * 8;
-                    A[j][0] = __funnelshift_r(w0, w1, sh);
-                    A[j][1] = __funnelshift_r(w1, w2, sh);
-                    uint32_t ob = o + 1, shb = (ob & 3) * 8;
-                    B[j][0] = ob < 4 ? __funnelshift_r(w0, w1, shb) : __funnelshift_r(w1, w2, shb);
-                    B[j][1] = ob < 4 ? __funnelshift_r(w1, w2, shb) : __funnelshift_r(w2, w3, shb);
-                    uint32_t oc = o + 2, shc = (oc & 3) * 8;
-                    Cq[j][0] = oc < 4 ? __funnelshift_r(w0, w1, shc) : __funnelshift_r(w1, w2, shc);
-                    Cq[j][1] = oc < 4 ? __funnelshift_r(w1, w2, shc) : __funnelshift_r(w2, w3, shc);
+                    // the samples left of, at and right of the centre's columns
+                    const uint32_t sh = o * 8, q0 = __funnelshift_r(w0, w1, sh), q1 = __funnelshift_r(w1, w2, sh),
+                                   q2 = __funnelshift_r(w2, w3, sh);
+                    A[j][0] = q0;
+                    A[j][1] = q1;
+                    B[j][0] = __byte_perm(q0, q1, 0x4321);
+                    B[j][1] = __byte_perm(q1, q2, 0x4321);
+                    Cq[j][0] = __byte_perm(q0, q1, 0x5432);
+                    Cq[j][1] = __byte_perm(q1, q2, 0x5432);
                 }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t cw = h ? c1 : c0;
+                    // four-tap floor averages from sums of two adjacent columns (even and odd bytes in
+                    // 16-bit lanes), each row's sums used for the row above and the row below
+                    const uint32_t M = 0x00FF00FFu;
+                    uint32_t sl[3], sh2[3], tl[3], th[3];
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        const uint32_t bl = B[j][h] & M, bh = (B[j][h] >> 8) & M;
+                        sl[j] = (A[j][h] & M) + bl;
+                        sh2[j] = ((A[j][h] >> 8) & M) + bh;
+                        tl[j] = bl + (Cq[j][h] & M);
+                        th[j] = bh + ((Cq[j][h] >> 8) & M);
+                    }
+                    auto avg4 = [&](uint32_t l, uint32_t hh) { return ((l >> 2) & M) | ((hh << 6) & ~M); };
                     uint32_t v[9];
-                    v[0] = favg4(A[0][h], B[0][h], A[1][h], B[1][h]);
+                    v[0] = avg4(sl[0] + sl[1], sh2[0] + sh2[1]);
                     v[1] = favg(B[0][h], B[1][h]);
-                    v[2] = favg4(B[0][h], Cq[0][h], B[1][h], Cq[1][h]);
+                    v[2] = avg4(tl[0] + tl[1], th[0] + th[1]);
                     v[3] = favg(A[1][h], B[1][h]);
                     v[4] = B[1][h];
                     v[5] = favg(B[1][h], Cq[1][h]);
-                    v[6] = favg4(A[1][h], B[1][h], A[2][h], B[2][h]);
+                    v[6] = avg4(sl[1] + sl[2], sh2[1] + sh2[2]);
                     v[7] = favg(B[1][h], B[2][h]);
-                    v[8] = favg4(B[1][h], Cq[1][h], B[2][h], Cq[2][h]);
+                    v[8] = avg4(tl[1] + tl[2], th[1] + th[2]);
 #pragma unroll
                     for (int q = 0; q < 9; q++) hpart[q] = (h ? hpart[q] : 0u) + __vsadu4(cw, v[q]);
                 }
@@ -2603,20 +2589,18 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                 const unsigned w45 = __reduce_add_sync(0xffffffffu, hpart[4] | (hpart[5] << 16));
                 const unsigned w67 = __reduce_add_sync(0xffffffffu, hpart[6] | (hpart[7] << 16));
                 const unsigned w8 = __reduce_add_sync(0xffffffffu, hpart[8]);
-                const int q = lane < 9 ? lane : 4;
-                const unsigned wq = q < 2 ? w01 : q < 4 ? w23 : q < 6 ? w45 : q < 8 ? w67 : w8;
-                const int hsq = (int)((wq >> ((q & 1) * 16)) & 0xffffu);
-                const int sxq = q % 3 - 1, syq = q / 3 - 1;
-                const bool vq = lane < 9 && !((sdx == -128 && sxq == -1) || (sdy == -128 && syq == -1));
+                // (lane constants and masks, computed before the rows: choices by lane would be branches)
+                const unsigned wq = (w01 & hp_m[0]) | (w23 & hp_m[1]) | (w45 & hp_m[2]) | (w67 & hp_m[3]) | (w8 & hp_m[4]);
+                const int hsq = (int)((wq >> hp_shift) & 0xffffu);
+                const bool vq = lane < 9 && !((sdx == -128 && hp_sx == -1) || (sdy == -128 && hp_sy == -1));
                 const int c15i = (int)p.c15;  // every neighbour is fractional in at least one axis
-                const int ord = q == 4 ? 0 : (q < 4 ? q + 1 : q);
-                const int tot = hsq + (q == 4 ? 0 : c15i);
-                const uint32_t key = __reduce_min_sync(0xffffffffu, vq ? ((uint32_t)tot << 4) | (uint32_t)ord : 0xffffffffu);
+                const int tot = hsq + (lane == 4 ? 0 : c15i);
+                const uint32_t key = __reduce_min_sync(0xffffffffu, vq ? ((uint32_t)tot << 4) | hp_ord : 0xffffffffu);
                 const int ow = (int)(key & 15u);
-                const int qw = ow == 0 ? 4 : (ow <= 4 ? ow - 1 : ow);
-                bsx = qw % 3 - 1;
-                bsy = qw / 3 - 1;
-                best_sad = (long long)((int)(key >> 4) - (qw == 4 ? 0 : c15i));
+                // column and row offsets + 1 of the candidates in that order (4, 0, 1, 2, 3, 5, 6, 7, 8)
+                bsx = (int)((0x24891u >> (2 * ow)) & 3u) - 1;
+                bsy = (int)((0x2A501u >> (2 * ow)) & 3u) - 1;
+                best_sad = (long long)((int)(key >> 4) - (ow == 0 ? 0 : c15i));
             } else {
                 long long hs[9];
 #pragma unroll
@@ -2633,15 +2617,14 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                     if (hs[q] + pen < best_total) { best_total = hs[q] + pen; best_sad = hs[q]; bsx = sx; bsy = sy; }
                 }
             }
-            int dxh = min(max(2 * sdx + bsx, -255), 255), dyh = min(max(2 * sdy + bsy, -255), 255);
-            // MotionVector::new(dx_hp/2, dy_hp/2, dx_hp%2, dy_hp%2).as_canonicalized()
-            MvT raw{sat8(dxh / 2), sat8(dyh / 2), dxh % 2, dyh % 2};
-            if (raw.dx == -128 && raw.sx == -1) raw.sx = 0;
-            if (raw.dy == -128 && raw.sy == -1) raw.sy = 0;
-            if (raw.sx == -1) { raw.sx = 1; raw.dx = max(-128, raw.dx - 1); }
-            if (raw.sy == -1) { raw.sy = 1; raw.dy = max(-128, raw.dy - 1); }
+            // MotionVector::new(dx_hp/2, dy_hp/2, dx_hp%2, dy_hp%2).as_canonicalized(): a -1/2 component
+            // becomes +1/2 of the whole sample below, which is the half-pel value split by a floor
+            const int dxh = min(max(2 * sdx + bsx, -255), 255), dyh = min(max(2 * sdy + bsy, -255), 255);
+            const MvT raw{dxh >> 1, dyh >> 1, dxh & 1, dyh & 1};
 
             RIV_STAMP(4);
+            // the next MB's top-right record
+            if (r > 0) pref = ld_rec(p.rec + (r - 1) * p.BW + min(bx + 2, p.BW - 1));
             // ---- publish the raw MV for the next row's search; hand the MB (raw MV, best SAD)
             // to the mode warp, which runs the RDO skip and the mode decision off this chain
             if (lane == 0) {
@@ -2651,19 +2634,24 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                                                (unsigned long long)((uint32_t)(uint8_t)raw.dx | ((uint32_t)(uint8_t)raw.dy << 8) |
                                                                     ((uint32_t)(uint8_t)raw.sx << 16) |
                                                                     ((uint32_t)(uint8_t)raw.sy << 24));
-                if (!hand_put(hand, hand_done, hn, pay, p.spin_limit)) failed = true;
+                if (hn - taken < HAND_RING)  // room for it when the ring was last looked at
+                    *(volatile unsigned long long*)(hand + (hn & (HAND_RING - 1))) = ((unsigned long long)((hn + 1) & 0x7fff) << 49) | pay;
+                else if (!hand_put(hand, hand_done, hn, pay, p.spin_limit)) failed = true;
+            }
+            if (hn - taken >= HAND_RING) {  // (the same in every lane)
+                taken = __shfl_sync(0xffffffffu, min(hand_done[0], hand_done[1]), 0);
+                failed = __shfl_sync(0xffffffffu, (int)failed, 0) != 0;
             }
             hn++;
-            failed = __shfl_sync(0xffffffffu, (int)failed, 0) != 0;
             if (failed) {
                 if (lane == 0) atomicOr(p.status, ST_WAIT_TIMEOUT);
                 abort_loader();
                 if (!FAST) cp_async_wait0();
                 return;
             }
-            L_raw = MvT{raw.dx, raw.dy, 0, 0};
-            recTL = recT;
-            recT = recTR;
+            pL = (uint32_t)(uint8_t)raw.dx << 8 | (uint32_t)(uint8_t)raw.dy;
+            pTL = pT;
+            pT = pTR;
         }
         if (FAST) {  // the band of this row is no longer read
             __syncwarp();

@@ -34,7 +34,7 @@ inline int batch_ctas(int s, const BatchClip& k, const BatchTune& t) {
     switch (s) {
         case BS_CONVERT: return k.rgb != nullptr ? ((k.W / 2) * (k.H / 2) + 127) / 128 : 0;
         case BS_TABLE: return k.intra || k.tab == nullptr ? 0 : nmb;
-        case BS_PREDICT: return k.intra ? 0 : nmb;
+        case BS_PREDICT: return k.intra || k.predicted ? 0 : nmb;
         case BS_AQSUM: return k.intra ? 0 : 1;
         case BS_RESIDUAL: return (nmb + t.res_mbs - 1) / t.res_mbs;
         case BS_DEBLOCK: return k.db_level > 0 ? batch_deblock_tiles(k.W, k.H, t.db_tw) : 0;
@@ -155,11 +155,13 @@ __global__ void __launch_bounds__(SY_MODEL_THREADS, 8) kb_sym_model(BatchLaunch 
                     BATCH_MODEL_CTAS * (SY_MODEL_THREADS / 32), threadIdx.x & 31);
 }
 
-// ---- the multi-clip search wavefront (per-MB reference windows; see the file comment)
+// ---- the multi-clip search wavefront (per-MB reference windows; see the file comment).  96
+// registers a thread: five 128-thread CTAs of the direct kind an SM (120: four, 1.68 ms a step of 24
+// clips against 1.66; 80: six, 1.91).
 template <bool TABLE, bool SMALL>
-__global__ void __maxnreg__(120) k_search_multi(const SearchParams* __restrict__ ps, const int* __restrict__ start,
+__global__ void __maxnreg__(96) k_search_multi(const SearchParams* __restrict__ ps, const int* __restrict__ start,
                                                 int nclips) {
-    search_body<false, TABLE, SMALL>(ps[batch_clip(start, nclips, blockIdx.x)]);
+    search_body<false, TABLE, SMALL, false>(ps[batch_clip(start, nclips, blockIdx.x)]);
 }
 
 static const void* search_multi_fn(SearchKind k) {
@@ -235,12 +237,12 @@ int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int tota
 int search_multi_kind(bool table, bool small) {
     return table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN;
 }
-bool search_multi_table(int kind) { return kind == SK_TABLE_SMALL || kind == SK_TABLE; }
+bool search_multi_predicts(int kind) { return search_fast(false, (SearchKind)kind); }
 
 int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* threads) {
     const void* fn = search_multi_fn((SearchKind)kind);
     const size_t sm = search_smem(max_sr, 0, false, (SearchKind)kind);
-    const int nt = search_threads(false);
+    const int nt = search_threads(search_fast(false, (SearchKind)kind));
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nt, sm);
     *smem = sm;

@@ -3214,6 +3214,15 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
                     kc[a].tab = nullptr;
                 }
                 pvar[a] = search_variant(e, t.table != 0);
+                if (search_multi_predicts(pvar[a])) {  // as submit_gpu's aq_in_search
+                    kc[a].predicted = 1;
+                    sps[a].pred = kc[a].pred;
+                    sps[a].varsum = e->varsum.as<uint2>();
+                    sps[a].lnv = kc[a].lnv;
+                    sps[a].logfix = kc[a].logfix;
+                    sps[a].nlog = kc[a].nlog;
+                    kc[a].rp.ref = kc[a].ref;  // chroma prediction in the residual
+                }
                 step_pmbs += (uint64_t)e->NMB;
             }
         }

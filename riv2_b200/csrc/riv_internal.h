@@ -165,6 +165,7 @@ struct BatchClip {
     float* lnv;
     const uint32_t* logfix;
     int nlog;
+    int predicted;      // the search launch makes the luma prediction and the ln variances
     ResidualParams rp;  // residual (steps from lnv for P-frames, intra tables for key frames)
     // deblock (db_level > 0): db_src -> db_dst
     int db_level, db_E, db_I, db_H;
@@ -192,7 +193,7 @@ int launch_batch_stage(int stage, const BatchLaunch& b, const BatchTune& t, int 
 // the SADs computed on the way.
 constexpr int SEARCH_KINDS = 4;
 int search_multi_kind(bool table, bool small);
-bool search_multi_table(int kind);
+bool search_multi_predicts(int kind);  // its launch makes the luma prediction and the ln variances
 int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* threads);
 int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total_ctas, int kind, size_t smem,
                         int threads, void* stream);

@@ -266,11 +266,10 @@ __device__ __forceinline__ void fill_chunk(uint8_t* band, int BWB, int WS, int c
 }
 
 
-// Per-MB window (DIRECT, no band): rows wy0 .. wy0 + WS - 1, columns fx0 .. fx0 + stride - 1 with
-// fx0 = x0 - MARGIN, a multiple of 16, in 16-byte chunks (cp.async; replicated borders by value).
-__host__ __device__ inline int search_window_stride(int sr) { return 16 + 2 * ((sr + 1 + 15) & ~15); }
-__device__ __forceinline__ void fill_window(uint8_t* win, int stride, int WS, int MARGIN, int fx0, int wy0,
-                                           const uint8_t* __restrict__ ref, int W, int H, int lane) {
+// A search window: rows wy0 .. wy0 + WS - 1, columns fx0 .. fx0 + stride - 1 (multiples of 16) in
+// 16-byte chunks (cp.async, past L1; replicated borders by value).
+__device__ __forceinline__ void fill_window(uint8_t* win, int stride, int WS, int fx0, int wy0,
+                                           const uint8_t* ref, int W, int H, int lane) {
     const int nc = stride >> 4;
     for (int i = lane; i < WS * nc; i += 32) {
         const int r = i / nc, c = i - r * nc, fx = fx0 + 16 * c;
@@ -986,15 +985,17 @@ __device__ __forceinline__ bool hand_put(unsigned long long* hand, volatile int*
     return true;
 }
 
+// nap: nanoseconds between polls, from the first on (0: poll 64 times, then every 16 ns)
 __device__ __forceinline__ bool hand_get(const unsigned long long* hand, int n, unsigned long long& w,
-                                         long long limit) {
+                                         long long limit, unsigned nap) {
     const volatile unsigned long long* h = hand + (n & (HAND_RING - 1));
     const unsigned long long want = (unsigned long long)((n + 1) & 0x7fff) << 49;
     unsigned long long v = *h;
     long long spins = 0;
     while ((v & ~((1ull << 49) - 1)) != want) {
         if (++spins > limit) return false;
-        if (spins > 64) __nanosleep(16);
+        if (nap != 0) __nanosleep(nap);
+        else if (spins > 64) __nanosleep(16);
         v = *h;
     }
     w = v;
@@ -1097,7 +1098,7 @@ __device__ __forceinline__ MbDecision decide_mb(const SearchParams& p, const MvT
 // the next row's mode warp reads (second half of p.rec) and the per-MB output.  None of this
 // feeds the search, so it runs beside the search chain instead of on it.
 __device__ __forceinline__ void mode_warp(const SearchParams& p, const unsigned long long* hand, volatile int* hand_done,
-                                       unsigned long long tagbits) {
+                                       unsigned long long tagbits, unsigned nap) {
     const int lane = threadIdx.x & 31;
     MbRec* rc = p.rec + (size_t)p.BW * p.BH;
     auto rec_cod = [](unsigned long long v) {
@@ -1113,7 +1114,7 @@ __device__ __forceinline__ void mode_warp(const SearchParams& p, const unsigned 
             unsigned long long hw = 0, vTR = 0;
             int st = 0;  // 0 ok, 1 wait expired, 2 the search warp gave up
             if (lane == 0) {
-                if (!hand_get(hand, n, hw, p.spin_limit)) st = 1;
+                if (!hand_get(hand, n, hw, p.spin_limit, nap)) st = 1;
                 else if (hw & HAND_FAIL) st = 2;
                 if (st == 0 && r > 0) {
                     if (bx == 0 && !rec_wait(rc + (size_t)(r - 1) * p.BW, tagbits, vT, p.spin_limit)) st = 1;
@@ -1554,7 +1555,7 @@ __global__ void k_wait_expiry(int which, const unsigned long long* rec, const un
         if (lane == 0) ok = wait_at_least(counter + blockIdx.x, 1u, limit);
     } else if (which == 2) {
         unsigned long long w = 0;
-        if (lane == 0) ok = hand_get(hand, 0, w, limit);
+        if (lane == 0) ok = hand_get(hand, 0, w, limit, 0);
     } else {
         ok = mbar_wait_warp(&bar, 0u, limit);
     }
@@ -1568,23 +1569,32 @@ int launch_wait_expiry(int which, const unsigned long long* rec, const unsigned*
     return (int)cudaGetLastError();
 }
 
-// Staging ring of the band+table search (LD_RING MBs ahead): per slot the MB's SAD-table row
-// (2*tstride bytes), its 16x16 current block and the previous frame's coded MV (4 bytes).
+// Staging ring of the loader (LD_RING MBs ahead): per slot the MB's SAD-table row (2*tstride
+// bytes), its 16x16 current block, the previous frame's coded MV (4 bytes) and, without a band, its
+// reference window (rows y0-sr-1 .. y0+16+sr, MARGIN columns on both sides).
 constexpr int LD_RING = 4;
-__host__ __device__ inline int ld_slot_bytes(int tstride) { return 2 * tstride + 256 + 16; }
+__host__ __device__ inline int search_window_stride(int sr) { return 16 + 2 * ((sr + 1 + 15) & ~15); }
+__host__ __device__ inline int ld_slot_bytes(int tstride, bool window, int sr) {
+    return 2 * tstride + 256 + 16 + (window ? (18 + 2 * sr) * search_window_stride(sr) + 16 : 0);
+}
 
-// The third warp of each row CTA (band + table instantiations): fills the MB-row reference
-// band once per row (one bulk copy per band row plus the replicated edge margins) and, up to
-// LD_RING MBs ahead of the search warp, each MB's table row, current block and temporal MV,
-// so that no copy is issued on the search chain.  ctl[0] = MBs the search warp has released,
-// ctl[1] = rows it has finished, ctl[2] = abort.
+// The third warp of each row CTA (where a loader runs): fills the MB-row reference band once per
+// row (one bulk copy per band row plus the replicated edge margins) and, up to LD_RING MBs ahead of
+// the search warp, each MB's table row, current block and temporal MV -- with RING, where there is
+// no band, its window too -- so that no copy is issued on the search chain.  ctl[0] = MBs the
+// search warp has released, ctl[1] = rows it has finished, ctl[2] = abort, ctl[3] / ctl[4] = rows /
+// MBs that the AQ warp has finished.
+// RING copies with cp.async (16 bytes a lane: a window is 126 of them at a search range of 12, too
+// many for row-wise bulk copies of 48 bytes); the slot's barrier then counts two arrivals a lane,
+// one when its copies have landed and one for what it stored itself.
 // row_live (optional): set once the first row's reference bands are ready, which stops the
 // CTA's helper worker groups from taking further tasks.
+template <bool RING>
 __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long long* fullb, unsigned long long* bandb,
                                             volatile int* ctl, uint8_t* slots, uint8_t* band, volatile int* row_live) {
     const int lane = threadIdx.x & 31;
     const int sr = p.sr, WS = 18 + 2 * sr, MARGIN = (sr + 1 + 15) & ~15, BWB = band_stride(p.W, sr);
-    const int SLOT = ld_slot_bytes(p.tstride);
+    const int SLOT = ld_slot_bytes(p.tstride, RING, sr);
     const unsigned tab_bytes = 2u * (unsigned)p.tstride;
     int n = 0, rows = 0;
     bool abort = false;
@@ -1601,7 +1611,7 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
     };
     for (int r = row_cta(p); r < p.BH && !abort; r += p.nrow_ctas) {
         const int wy0 = r * 16 - sr - 1;
-        if (rows > 0 && !(wait_ctl(1, rows) && (p.lnv == nullptr || wait_ctl(3, rows)))) { abort = true; break; }
+        if (!RING && rows > 0 && !(wait_ctl(1, rows) && (p.lnv == nullptr || wait_ctl(3, rows)))) { abort = true; break; }
         if (p.defer) {  // the previous frame's bands r-1 .. r+1 must be deblocked (written by workers)
             int ok = 1;
             if (lane == 0) {
@@ -1614,6 +1624,7 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
             if (!__shfl_sync(0xffffffffu, ok, 0)) { abort = true; break; }
         }
         if (row_live != nullptr && lane == 0) *row_live = 1;
+        if (!RING) {
         // ---- the band: rows wy0 .. wy0+WS-1 (edge-clamped), columns -MARGIN .. W+MARGIN-1
         for (int i = lane; i < WS; i += 32) {
             const int gy = min(max(wy0 + i, 0), p.H - 1);
@@ -1630,12 +1641,26 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
         __syncwarp();
         if (lane == 0) mbar_arrive_tx(bandb, (unsigned)(WS * p.W));
         else mbar_arrive(bandb);
+        }
         // ---- per-MB staging
         for (int bx = 0; bx < p.BW; bx++) {
             const int idx = r * p.BW + bx;
             const int s = n & (LD_RING - 1);
-            if (n >= LD_RING && !wait_ctl(0, n - LD_RING + 1)) { abort = true; break; }
+            if (n >= LD_RING && !(wait_ctl(0, n - LD_RING + 1) && (!RING || p.lnv == nullptr || wait_ctl(4, n - LD_RING + 1)))) {
+                abort = true;
+                break;
+            }
             uint8_t* slot = slots + (size_t)s * SLOT;
+            if (RING) {
+                if (lane < 16) cp_async16(slot + lane * 16, p.cur_y + (size_t)(r * 16 + lane) * p.W + bx * 16);
+                if (lane == 0) *(int*)(slot + 256) = p.prev_coded ? *(const int*)(p.prev_coded + 4 * (size_t)idx) : 0;
+                fill_window(slot + 272, search_window_stride(sr), WS, bx * 16 - MARGIN, wy0, p.ref_y, p.W, p.H, lane);
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sa32(fullb + s)) : "memory");
+                mbar_arrive(fullb + s);
+                __syncwarp();
+                n++;
+                continue;
+            }
             if (p.tflag != nullptr) {  // fused launch: wait until a table worker published this MB's row
                 int ok = 1;
                 if (lane == 0) {
@@ -1667,7 +1692,7 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
             long long spins = 0;
             while (!mbar_test(fullb + (k & (LD_RING - 1)), (unsigned)((k / LD_RING) & 1)) && ++spins <= p.spin_limit) {}
         }
-        if (rows > 0) {
+        if (!RING && rows > 0) {
             long long spins = 0;
             while (!mbar_test(bandb, (unsigned)((rows - 1) & 1)) && ++spins <= p.spin_limit) {}
         }
@@ -1675,19 +1700,20 @@ __device__ __forceinline__ void loader_warp(const SearchParams& p, unsigned long
     }
 }
 
-// The fourth warp of each row CTA (band + table instantiations, P-frames): for every MB the
+// The fourth warp of each row CTA (where a loader runs, P-frames): for every MB the
 // search warp hands over, in raster order, the luma motion-compensated prediction
-// (build_predicted, com/fast_motion.rs:103-352) from the row's reference band, where the
-// replicated edges give the same samples as the reference's clamped coordinates, and the
-// predicted-luma sums (sum, sum of squares) for the MB's variance (compute_aq_quant_steps,
-// res/residual.rs:116-153).  Chroma prediction is left to the residual kernel.  After each row
-// it sets ctl[3] = rows it has finished (the loader refills the band only after both the search
-// warp and this warp are done with it), computes the row's ln variances into lnv and publishes
-// row_done[r] = tag.
+// (build_predicted, com/fast_motion.rs:103-352) from the row's reference band (RING: the MB's
+// window, `band` = the loader's slots), where the replicated edges give the same samples as the
+// reference's clamped coordinates, and the predicted-luma sums (sum, sum of squares) for the MB's
+// variance (compute_aq_quant_steps, res/residual.rs:116-153).  Chroma prediction is left to the
+// residual kernel.  After each MB (RING) it sets ctl[4], after each row ctl[3], for the loader,
+// computes the row's ln variances into lnv and, for a fold in the launch, publishes row_done[r] = tag.
+template <bool RING>
 __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned long long* hand, volatile int* hand_done,
-                                        volatile int* ctl, const uint8_t* band, unsigned long long* bandb) {
+                                        volatile int* ctl, const uint8_t* band, unsigned long long* fullb,
+                                        unsigned long long* bandb, unsigned nap) {
     const int lane = threadIdx.x & 31;
-    const int sr = p.sr, MARGIN = (sr + 1 + 15) & ~15, BWB = band_stride(p.W, sr);
+    const int sr = p.sr, MARGIN = (sr + 1 + 15) & ~15, BWB = RING ? search_window_stride(sr) : band_stride(p.W, sr);
     const int W = p.W;
     uint8_t* PY = p.pred;
     const int yy = lane >> 1, xoff = (lane & 1) * 8;  // luma: row, 8-pixel half
@@ -1695,7 +1721,7 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
     for (int r = row_cta(p); r < p.BH; r += p.nrow_ctas) {
         const int y0 = r * 16, wy0 = y0 - sr - 1;
         // observe the band fill of this row (the loader refills only after this warp is done)
-        if (!mbar_wait_warp(bandb, (unsigned)(rows & 1), p.spin_limit)) {
+        if (!RING && !mbar_wait_warp(bandb, (unsigned)(rows & 1), p.spin_limit)) {
             if (lane == 0) atomicOr(p.status, ST_WAIT_TIMEOUT);
             return;
         }
@@ -1704,7 +1730,7 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
             unsigned long long hw = 0;
             int st = 0;
             if (lane == 0) {
-                if (!hand_get(hand, n, hw, p.spin_limit)) st = 1;
+                if (!hand_get(hand, n, hw, p.spin_limit, nap)) st = 1;
                 else if (hw & HAND_FAIL) st = 2;
                 else hand_done[1] = n + 1;
             }
@@ -1712,6 +1738,14 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
             if (st != 0) {
                 if (lane == 0 && st == 1) atomicOr(p.status, ST_WAIT_TIMEOUT);
                 return;
+            }
+            const uint8_t* org = band + MARGIN + x0;  // the band's or window's sample at column x0
+            if (RING) {  // the window's copies landed before the search warp used it; observe it here too
+                if (!mbar_wait_warp(fullb + (n & (LD_RING - 1)), (unsigned)((n / LD_RING) & 1), p.spin_limit)) {
+                    if (lane == 0) atomicOr(p.status, ST_WAIT_TIMEOUT);
+                    return;
+                }
+                org = band + (size_t)(n & (LD_RING - 1)) * ld_slot_bytes(p.tstride, true, sr) + 272 + MARGIN;
             }
             n++;
             hw = __shfl_sync(0xffffffffu, hw, 0);
@@ -1723,8 +1757,8 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
             unsigned s = 0, s2 = 0;
             {
                 const int byp = (2 * (y0 + yy) + mdy) >> 1;
-                const int c0 = x0 + xoff + (mdx >> 1);  // first integer column (floor)
-                const uint8_t* rp = band + (size_t)(byp - wy0) * BWB + MARGIN + c0;
+                const int c0 = xoff + (mdx >> 1);  // first integer column (floor)
+                const uint8_t* rp = org + (byp - wy0) * BWB + c0;
                 uint32_t A[2][3];  // bytes c0 .. c0+11 of rows byp, byp+1
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
@@ -1757,6 +1791,10 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
             }
             s = __reduce_add_sync(0xffffffffu, s);
             s2 = __reduce_add_sync(0xffffffffu, s2);
+            if (RING) {  // the window is read
+                __syncwarp();
+                if (lane == 0) ctl[4] = n;
+            }
             if (lane == 0) p.varsum[idx] = make_uint2(s, s2);
             if (lane == 0) RIV_GSTAMP(idx, 31);
         }
@@ -1785,9 +1823,11 @@ __device__ __forceinline__ void aq_warp(const SearchParams& p, const unsigned lo
                 if (i < p.BW) p.lnv[(size_t)r * p.BW + i] = l4[j];
             }
         }
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) st_release_u32(p.row_done + r, p.tag);
+        if (p.row_done != nullptr) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) st_release_u32(p.row_done + r, p.tag);
+        }
         rows++;
     }
 }
@@ -1891,17 +1931,20 @@ __device__ __forceinline__ void sad_parts(const RefView& v, int org, bool inside
     }
 }
 
-template <bool BAND, bool TABLE, bool SMALL>
+// Where several row CTAs share an SM their waiting mode and AQ warps look less often.
+constexpr unsigned SEARCH_NAP = 250;
+// WORKERS: the launch may be fused (worker CTAs, helper groups of the row CTAs).
+template <bool BAND, bool TABLE, bool SMALL, bool WORKERS>
 __device__ __forceinline__ void search_body(const SearchParams& p) {
-    // FAST (band + 32-bit costs or table): search chain, mode decision, loader and AQ warps.
-    // Otherwise the search warp stages its own data with cp.async and only the mode warp runs
-    // beside it.  DIRECT (32-bit costs, no table): the integer SADs are computed on the chain, four
+    // FAST (DIRECT, or band and table): search chain, mode decision, loader and AQ warps.  Otherwise
+    // the search warp stages its own data with cp.async and only the mode warp runs beside it.  RING:
+    // the loader brings each MB's window instead of the row's band.  DIRECT (32-bit costs, no table): the integer SADs are computed on the chain, four
     // positions at a time (8 lanes each).  1080p at search range 31: 0.99 ms a frame with the
     // previous frame's reconstruction in the launch, where one position at a time on 64-bit costs,
     // its prediction, AQ, residual and deblock in kernels of their own, took 1.60 ms.
-    constexpr bool FAST = BAND && (TABLE || SMALL), DIRECT = SMALL && !TABLE;
+    constexpr bool DIRECT = SMALL && !TABLE, FAST = (BAND && TABLE) || DIRECT, RING = DIRECT && !BAND;
     extern __shared__ __align__(16) uint8_t smem[];
-    if (FAST && p.fused && row_cta(p) >= p.nrow_ctas) {
+    if (FAST && WORKERS && p.fused && row_cta(p) >= p.nrow_ctas) {
         frame_worker(p, smem);
         return;
     }
@@ -1919,7 +1962,8 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     // other layouts: double-buffered current block and table row
     uint8_t* curbuf = after_hand;  // 2 x 256 bytes
     uint16_t* tabbuf = (uint16_t*)(curbuf + 512);   // TABLE: 2 x tstride entries
-    uint8_t* refmem = FAST ? slots + LD_RING * ld_slot_bytes(p.tstride)
+    const int SLOT = ld_slot_bytes(p.tstride, RING, p.sr);
+    uint8_t* refmem = FAST ? slots + LD_RING * SLOT
                            : curbuf + 512 + (TABLE ? 4 * p.tstride : 0);  // band or window (+16 bytes slack)
     const int side = 2 * p.sr + 1;
     const int lane = threadIdx.x & 31;
@@ -1927,7 +1971,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     const int WS = 18 + 2 * sr;
     const int MARGIN = (sr + 1 + 15) & ~15;
     const int BWB = band_stride(p.W, sr);
-    const int WSB = search_window_stride(sr);  // per-MB window (DIRECT, no band): row stride
+    const int WSB = search_window_stride(sr);  // RING: the window's row stride
     for (int i = threadIdx.x; i < 256; i += blockDim.x) bits[i] = p.mvbits[i];
     const int* nc32 = nc32s;
     if (SMALL)
@@ -1936,8 +1980,8 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     // Fused launch: threads 128-511 of a row CTA are worker groups 1-3 until the row starts
     // (region after the row layout: a live flag, then a 3-group worker region), and the
     // whole CTA joins the worker queue once its rows are done.
-    const bool helpers = FAST && p.fused && p.row_helpers;
-    uint8_t* pre = smem + (((size_t)(refmem - smem) + (size_t)WS * BWB + 16 + 15) & ~(size_t)15);
+    const bool helpers = FAST && WORKERS && p.fused && p.row_helpers;
+    uint8_t* pre = smem + (((size_t)(refmem - smem) + (RING ? 0 : (size_t)WS * BWB + 16) + 15) & ~(size_t)15);
     volatile int* row_live = (volatile int*)pre;
     uint8_t* preg = pre + 16;
     if (helpers) load_worker_bases(p, preg, threadIdx.x, blockDim.x);
@@ -1946,29 +1990,37 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
         hand_done[0] = 0;
         hand_done[1] = FAST && p.lnv != nullptr ? 0 : 0x3fffffff;  // no AQ warp: never waited for
         if (FAST) {
-            for (int i = 0; i < LD_RING; i++) mbar_init(fullb + i, 1);
+            for (int i = 0; i < LD_RING; i++) mbar_init(fullb + i, RING ? 64 : 1);
             mbar_init(bandb, 32);
-            ld_ctl[0] = ld_ctl[1] = ld_ctl[2] = ld_ctl[3] = 0;
+            for (int i = 0; i < 5; i++) ld_ctl[i] = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
     __syncthreads();
     const unsigned long long tagbits = (unsigned long long)(p.tag & 0xffffu) << 48;
+    const unsigned nap = WORKERS ? 0u : SEARCH_NAP;
+    // The role of this warp: search, mode, loader, AQ.  A warp's scheduler is its index modulo 4, so
+    // where several CTAs share an SM the roles rotate from CTA to CTA (CTAs 148 apart share an SM
+    // when the grid is larger): with the search warp first in each, one scheduler had all the chains
+    // (24 mixed clips, five CTAs an SM: 2.21 ms a step, 1.66 rotated; 1.95 for search and prediction
+    // without loader and AQ warps).
+    const int warp = (int)(threadIdx.x >> 5);
+    const int role = FAST && !WORKERS ? (warp + (int)(blockIdx.x / 148u)) & 3 : warp;
     auto roles = [&]() {
-    if (threadIdx.x >= 64) {
-        if (FAST && threadIdx.x < 96) {
-            loader_warp(p, fullb, bandb, ld_ctl, slots, refmem, helpers ? row_live : nullptr);
-            if (p.lnv != nullptr && row_cta(p) == 0) aq_fold(p, ld_ctl, fold_stage);
-        } else if (FAST && threadIdx.x < 128 && p.lnv != nullptr) {
-            aq_warp(p, hand, hand_done, ld_ctl, refmem, bandb);
-        } else if (helpers && threadIdx.x >= TW_GROUP) {
+    if (role >= 2) {
+        if (FAST && role == 2) {
+            loader_warp<RING>(p, fullb, bandb, ld_ctl, slots, refmem, helpers ? row_live : nullptr);
+            if (p.lnv != nullptr && p.row_done != nullptr && row_cta(p) == 0) aq_fold(p, ld_ctl, fold_stage);
+        } else if (FAST && role == 3 && p.lnv != nullptr) {
+            aq_warp<RING>(p, hand, hand_done, ld_ctl, RING ? slots : refmem, fullb, bandb, nap);
+        } else if (WORKERS && helpers && threadIdx.x >= TW_GROUP) {
             const int gid = threadIdx.x / TW_GROUP;
             worker_loop(p, preg, 3, gid - 1, gid, row_live);
         }
         return;
     }
-    if (threadIdx.x >= 32) {
-        mode_warp(p, hand, hand_done, tagbits);
+    if (role == 1) {
+        mode_warp(p, hand, hand_done, tagbits, nap);
         return;
     }
     int ln = 0;      // MBs taken from the loader (FAST)
@@ -2010,7 +2062,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
         int c_done = -1;
         auto c_hi = [&](int bx) { return (16 * bx + 16 + sr + MARGIN) >> 4; };
         if (FAST) {
-            if (!mbar_wait_warp(bandb, (unsigned)(lrows & 1), p.spin_limit)) {
+            if (!RING && !mbar_wait_warp(bandb, (unsigned)(lrows & 1), p.spin_limit)) {
                 if (lane == 0) {
                     atomicOr(p.status, ST_WAIT_TIMEOUT);
                     hand_put(hand, hand_done, hn, HAND_FAIL, p.spin_limit);
@@ -2022,7 +2074,6 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             for (int c = 0; c <= c_hi(0); c++) fill_chunk(refmem, BWB, WS, c, MARGIN, wy0, p.ref_y, p.W, p.H, lane);
             c_done = c_hi(0);
         }
-        if (DIRECT && !BAND) fill_window(refmem, WSB, WS, MARGIN, -MARGIN, wy0, p.ref_y, p.W, p.H, lane);
         if (!FAST) {
             if (lane < 16) cp_async16(curbuf + lane * 16, p.cur_y + (size_t)(y0 + lane) * p.W);
             if (TABLE)
@@ -2042,7 +2093,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             if (lane == 0) RIV_GSTAMP(idx, 16);
             // ---- FAST: wait for the loader's slot; otherwise prefetch MB bx+1 (columns, current
             // block, table row) and wait for MB bx's data
-            const uint8_t* lslot = slots + (size_t)(ln & (LD_RING - 1)) * ld_slot_bytes(p.tstride);
+            const uint8_t* lslot = slots + (size_t)(ln & (LD_RING - 1)) * SLOT;
             if (FAST) {
                 if (!mbar_wait_warp(fullb + (ln & (LD_RING - 1)), (unsigned)((ln / LD_RING) & 1), p.spin_limit)) {
                     if (lane == 0) {
@@ -2059,8 +2110,6 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                         fill_chunk(refmem, BWB, WS, c, MARGIN, wy0, p.ref_y, p.W, p.H, lane);
                     c_done = hi;
                 }
-                if (DIRECT && !BAND)
-                    fill_window(refmem + ((bx + 1) & 1) * (WS * WSB), WSB, WS, MARGIN, x0 + 16 - MARGIN, wy0, p.ref_y, p.W, p.H, lane);
                 RIV_STAMP(10);
                 if (lane < 16)
                     cp_async16(curbuf + ((bx + 1) & 1) * 256 + lane * 16, p.cur_y + (size_t)(y0 + lane) * p.W + x0 + 16);
@@ -2078,8 +2127,8 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
             if (BAND) {
                 view.org = refmem + x0 + MARGIN;
                 view.stride = BWB;
-            } else if (DIRECT) {  // per-MB window, filled one MB ahead
-                view.org = refmem + (bx & 1) * (WS * WSB) + MARGIN;
+            } else if (RING) {
+                view.org = lslot + 272 + MARGIN;
                 view.stride = WSB;
             } else {
                 // per-MB window (large search ranges / very wide frames): rows wy0.., cols x0-sr-1..
@@ -2516,7 +2565,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
                     }
                 }
             }
-            if (FAST) {  // the table row, current block and temporal MV are in registers now
+            if (FAST && !RING) {  // the table row, current block and temporal MV are in registers now
                 __syncwarp();
                 if (lane == 0) ld_ctl[0] = ln + 1;
                 ln++;
@@ -2576,6 +2625,11 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
 #pragma unroll
                     for (int q = 0; q < 9; q++) hpart[q] = (h ? hpart[q] : 0u) + __vsadu4(cw, v[q]);
                 }
+            }
+            if (RING) {  // the window too
+                __syncwarp();
+                if (lane == 0) ld_ctl[0] = ln + 1;
+                ln++;
             }
             long long best_sad;
             int bsx = 0, bsy = 0;
@@ -2663,7 +2717,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     }
     };
     roles();
-    if (helpers) {  // the row work is done: the whole CTA takes worker tasks
+    if (WORKERS && helpers) {  // the row work is done: the whole CTA takes worker tasks
         __syncthreads();
         if (threadIdx.x == 0) {
             for (int i = 0; i < LD_RING; i++) mbar_inval(fullb + i);
@@ -2686,7 +2740,7 @@ __global__ void __maxnreg__(120) k_search(SearchParams p) {
     if (tl != nullptr && threadIdx.x == 0) atomicCAS(tl, 0ull, (unsigned long long)gtimer());
     if (p.wq_next != nullptr && blockIdx.x == gridDim.x - 1)  // the next launch's queue words
         for (int i = threadIdx.x; i < p.wq_words; i += blockDim.x) p.wq_next[i] = 0u;
-    search_body<BAND, TABLE, SMALL>(p);
+    search_body<BAND, TABLE, SMALL, true>(p);
     if (tl != nullptr && (threadIdx.x & 31) == 0) atomicMax(tl + 1, (unsigned long long)gtimer());
 }
 
@@ -2699,14 +2753,14 @@ bool search_use_table(int sr) { return sr <= 15; }
 // worker tasks too until their row starts (2160 rows of MBs leave 13).
 constexpr int SEARCH_DIRECT_WORKERS = 8;
 enum SearchKind { SK_TABLE_SMALL, SK_TABLE, SK_DIRECT, SK_PLAIN };  // PLAIN: 64-bit costs, no table
-static bool search_fast(bool band, SearchKind k) { return band && k != SK_PLAIN; }
+static bool search_fast(bool band, SearchKind k) { return k == SK_DIRECT || (band && k != SK_PLAIN); }
 static size_t search_smem(int sr, int W, bool band, SearchKind k) {
     const bool table = k == SK_TABLE_SMALL || k == SK_TABLE;
     size_t ws = 18 + 2 * (size_t)sr;
-    size_t ref = band ? ws * (size_t)band_stride(W, sr) : k == SK_DIRECT ? 2 * ws * search_window_stride(sr) : ws * ws;
+    size_t ref = band ? ws * (size_t)band_stride(W, sr) : k == SK_DIRECT ? 0 : ws * ws;
     size_t head = 256 * sizeof(double) + 64 * 64 * 4 + HAND_RING * 8 + 16;
     const int stride = table ? sad_table_stride(sr) : 0;
-    if (search_fast(band, k)) return head + 64 + 1024 + LD_RING * (size_t)ld_slot_bytes(stride) + ref + 16;
+    if (search_fast(band, k)) return head + 64 + 1024 + LD_RING * (size_t)ld_slot_bytes(stride, !band, sr) + ref + 16;
     return head + 512 + 4 * (size_t)stride + ref + 16;
 }
 static int search_threads(bool fast) { return fast ? 128 : 64; }

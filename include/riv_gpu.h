@@ -314,6 +314,9 @@ riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uin
  * or a class it refuses: RIV_ERR_ENCODING_FAILED). */
 riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, uint32_t n, int intra, uint32_t max_symbols,
                                    uint8_t* out, size_t cap, size_t* len, int* on_gpu);
+/* Test hook (no reference counterpart): the rANS stream of n symbols (probability of a 0 in 1/256
+ * | bit << 8), coded in batches by the host (on_gpu == 0) or the GPU, as a batch's frames are. */
+riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_t* out, size_t cap, size_t* len);
 /* Test hook (host only, no reference counterpart): the decoder's DCT-coefficient decoder on one
  * frame's coefficient stream; n blocks of 384 i16 out, blocks with coded[b] == 0 are not in the
  * stream and stay zero; DC prediction when intra.  RIV_OK, or RIV_ERR_FRAME where the stream is

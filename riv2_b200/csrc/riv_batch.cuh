@@ -155,6 +155,21 @@ __global__ void __launch_bounds__(SY_MODEL_THREADS, 8) kb_sym_model(BatchLaunch 
                     BATCH_MODEL_CTAS * (SY_MODEL_THREADS / 32), threadIdx.x & 31);
 }
 
+// ---- rANS streams (riv_rans.cuh), a row of CTAs per clip
+__global__ void __launch_bounds__(32 * RA_WARPS) kb_rans(const BatchClip* __restrict__ clips) {
+    rans_cta(clips[blockIdx.y].rans, blockIdx.x);
+}
+__global__ void __launch_bounds__(RA_GATHER) kb_rans_gather(const BatchClip* __restrict__ clips) {
+    const RansFrame& f = clips[blockIdx.y].rans;
+    rans_gather_cta(f, blockIdx.x, (f.nside + RA_SIDE - 1) / RA_SIDE);
+}
+int launch_batch_rans(const BatchClip* clips, int nclips, unsigned max_cap, int max_nside, void* stream) {
+    const int nb = rans_batches(max_cap);
+    kb_rans<<<dim3((nb + RA_WARPS - 1) / RA_WARPS, nclips), 32 * RA_WARPS, 0, (cudaStream_t)stream>>>(clips);
+    kb_rans_gather<<<dim3(nb + rans_side_ctas(max_nside), nclips), RA_GATHER, 0, (cudaStream_t)stream>>>(clips);
+    return (int)cudaGetLastError();
+}
+
 // ---- the multi-clip search wavefront (per-MB reference windows; see the file comment).  96
 // registers a thread: five 128-thread CTAs of the direct kind an SM (120: four, 1.68 ms a step of 24
 // clips against 1.66; 80: six, 1.91).

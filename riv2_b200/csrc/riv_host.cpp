@@ -355,6 +355,9 @@ struct Job {
     int prev_buf = 0;
     int ck = 0;             // double-buffer parity of the frame's buffers
     bool sym = false;       // its symbols were made on the GPU (riv_symbols.cuh)
+    bool rans = false;      // and its rANS batches coded there (riv_rans.cuh)
+    const uint8_t* res_stream = nullptr;  // that stream, in the slot's pinned buffer
+    size_t res_len = 0;
     uint32_t count = 0;
     std::future<void> fut, fut_mv, fut_prep, fut_asm;
     std::vector<uint8_t> res_bytes, mv_bytes;
@@ -519,6 +522,13 @@ static riv_status validate(const riv_config& c, std::string& msg) {  // enc/conf
     return RIV_OK;
 }
 
+// A slot's buffers: the device's stacks (or packed coefficients) with RansFrame::info behind them,
+// and the pinned copy of these or of the rANS stream.
+static size_t rans_info_at(const riv_encoder* e) {
+    return (std::max((size_t)e->NMB * 384 * 2, (size_t)e->sym_cap * 2) + 255) & ~(size_t)255;
+}
+static size_t packed_bytes(const riv_encoder* e) { return std::max((size_t)e->NMB * 384 * 2, rans_max_bytes(e->sym_cap)); }
+
 static void setup_device(riv_encoder* e) {
     const riv_config& c = e->cfg;
     CK(cudaSetDevice(c.device));
@@ -665,12 +675,12 @@ static void setup_device(riv_encoder* e) {
     for (auto& s : e->slots) {
         s.rgb.alloc(std::max(rgb_bytes, e->yuv_bytes));
         s.dside.alloc((size_t)N * 4);
-        s.dpacked.alloc(std::max((size_t)N * 384 * 2, (size_t)e->sym_cap * 2));
+        s.dpacked.alloc(rans_info_at(e) + rans_info_bytes(e->sym_cap));
         s.dpeobs.alloc((size_t)N * 3);
         s.side.alloc((size_t)N * 4);
-        s.packed.alloc((size_t)N * 384 * 2);
+        s.packed.alloc(packed_bytes(e));
         s.peobs.alloc((size_t)N * 3);
-        s.hdr.alloc(16);
+        s.hdr.alloc(32);
         CK(cudaEventCreateWithFlags(&s.ev_h2d, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&s.ev_gpu, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&s.ev_d2h, cudaEventDisableTiming));
@@ -746,6 +756,21 @@ static SymFrame sym_frame(riv_encoder* e, int ck, bool intra, Slot& s) {
     f.peobs = s.dpeobs.as<uint8_t>();
     f.hdr = s.hdr.dev<uint32_t>();
     return f;
+}
+
+// The buffers of launch_batch_rans for the frame whose symbols f holds.
+static RansFrame rans_frame(riv_encoder* e, SymFrame& f, Slot& s) {
+    RansFrame r{};
+    r.stack = f.stack;
+    r.info = (uint4*)(s.dpacked.as<uint8_t>() + rans_info_at(e));
+    f.nsym = (uint32_t*)r.info;
+    r.side = f.side;
+    r.nside = e->NMB;
+    r.out_cap = (unsigned)std::min<size_t>(packed_bytes(e), 0xfffffff0u);
+    r.out = s.packed.as<uint8_t>();
+    r.side_out = s.side.as<uint32_t>();
+    r.out_bytes = f.hdr + 4;
+    return r;
 }
 
 // The first copy of a frame's rANS stacks to the host: whole batches, as many bytes as the last
@@ -1259,10 +1284,18 @@ static riv_status retire(riv_encoder* e, Job& j) {
         CK(cudaMemcpyAsync(s.peobs.p, s.dpeobs.p, (size_t)e->NMB * 3, cudaMemcpyDeviceToHost, e->R));
         CK(cudaStreamSynchronize(e->R));
     }
-    // what the host coder reads: whole rANS batches, or the truncated blocks
-    const size_t coef_bytes = j.sym ? (nsym + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH * 2 : (size_t)hdr[1] * 2;
+    const bool coded = j.sym && j.rans;  // the GPU coded the stream too
+    if (coded && nsym > 0) {
+        if (hdr[4] == SYM_FAIL) return fail(e, RIV_ERR_ENCODING_FAILED, "coefficient stream larger than its buffer");
+        j.res_stream = s.packed.as<uint8_t>();
+        j.res_len = hdr[4];
+    }
+    // what the host reads: the stream, whole rANS batches, or the truncated blocks
+    const size_t coef_bytes = coded ? j.res_len : j.sym ? (nsym + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH * 2 : (size_t)hdr[1] * 2;
     const uint16_t* stacks = s.packed.as<uint16_t>();
-    if (j.sym && coef_bytes > (size_t)e->NMB * 384 * 2) {  // more than the pinned buffer holds (rare: high-quality key frames)
+    if (coded) {
+        s.prefetched = 0;
+    } else if (j.sym && coef_bytes > packed_bytes(e)) {  // more than the pinned buffer holds (rare: high-quality key frames)
         j.big_stacks.resize(coef_bytes / 2);
         CK(cudaMemcpyAsync(j.big_stacks.data(), s.dpacked.p, coef_bytes, cudaMemcpyDeviceToHost, e->R));
         CK(cudaStreamSynchronize(e->R));
@@ -1273,7 +1306,7 @@ static riv_status retire(riv_encoder* e, Job& j) {
         CK(cudaStreamSynchronize(e->R));
     }
     // next frames of this type: copy 25% + 64 KiB more than this frame needed
-    (j.sym ? e->sym_guess : e->coef_guess)[j.type - 1] = coef_bytes + coef_bytes / 4 + 65536;
+    if (!coded) (j.sym ? e->sym_guess : e->coef_guess)[j.type - 1] = coef_bytes + coef_bytes / 4 + 65536;
     e->d2h_bytes += (uint64_t)e->NMB * (j.sym ? 4 : 7) + 16 + std::max(coef_bytes, s.prefetched);
     float t[NSTAGE + 1] = {0};
     if (!j.xev) CK(cudaEventSynchronize(s.ev_recon));  // the D2H did not wait for the deblock
@@ -1368,6 +1401,14 @@ static riv_status retire(riv_encoder* e, Job& j) {
     // extra work then competes with the frames beside it).
     // Frames whose symbols the GPU modelled need only their rANS batches coded.
     const bool newest = e->draining && &j == &e->jobs.back();
+    if (coded) {
+        std::promise<void> done;
+        done.set_value();
+        j.fut = done.get_future();
+        j.state = 1;
+        e->host_ms[1] += now_ms() - t0;
+        return RIV_OK;
+    }
     if (j.sym) {
         j.fut = e->pool->submit([jp, ep, stacks, nsym, newest] {
             double d0 = now_ms();
@@ -1415,13 +1456,15 @@ static riv_status write_job(riv_encoder* e, Job& j) {
     e->host_ms[5] += w0 - b0;
     const riv_config& c = e->cfg;
     std::vector<uint8_t> rec;
-    rec.reserve(32 + j.mv_bytes.size() + j.res_bytes.size());
+    const uint8_t* res = j.res_stream ? j.res_stream : j.res_bytes.data();
+    const size_t res_len = j.res_stream ? j.res_len : j.res_bytes.size();
+    rec.reserve(32 + j.mv_bytes.size() + res_len);
     put_le(rec, j.ts, 8);
     if (j.type == 1) {
         rec.push_back(1);
         rec.push_back(c.intra_quality);
-        put_le(rec, j.res_bytes.size(), 4);
-        rec.insert(rec.end(), j.res_bytes.begin(), j.res_bytes.end());
+        put_le(rec, res_len, 4);
+        rec.insert(rec.end(), res, res + res_len);
     } else {
         rec.push_back(2);
         rec.push_back(c.inter_quality);
@@ -1430,13 +1473,13 @@ static riv_status write_job(riv_encoder* e, Job& j) {
         rec.push_back(0);
         put_le(rec, j.mv_bytes.size(), 4);
         rec.insert(rec.end(), j.mv_bytes.begin(), j.mv_bytes.end());
-        put_le(rec, j.res_bytes.size(), 4);
-        rec.insert(rec.end(), j.res_bytes.begin(), j.res_bytes.end());
+        put_le(rec, res_len, 4);
+        rec.insert(rec.end(), res, res + res_len);
     }
     j.stats.total_bytes = (uint32_t)rec.size();
     j.stats.mv_bytes = (uint32_t)j.mv_bytes.size();
-    j.stats.residual_bytes = (uint32_t)j.res_bytes.size();
-    j.stats.resi_rans = j.type == 2 ? (int64_t)j.res_bytes.size() : -1;
+    j.stats.residual_bytes = (uint32_t)res_len;
+    j.stats.resi_rans = j.type == 2 ? (int64_t)res_len : -1;
     if (j.type != 2) j.stats.resi_raw = -1;
     if (e->wr.write(e->wr.user, rec.data(), rec.size()) != 0) return fail(e, RIV_ERR_IO, "writer.write failed");
     e->host_ms[4] += now_ms() - w0;
@@ -2462,6 +2505,64 @@ riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, u
     return RIV_OK;
 }
 
+riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_t* out, size_t cap, size_t* len) {
+    if ((n > 0 && !symbols) || !len) return RIV_ERR_FRAME;
+    entropy_init();
+    const size_t nb = ((size_t)n + SYM_BATCH - 1) / SYM_BATCH;
+    std::vector<uint16_t> st(nb * SYM_BATCH);
+    for (size_t k = 0; k < n; k++) st[k / SYM_BATCH * SYM_BATCH + (SYM_BATCH - 1 - k % SYM_BATCH)] = symbols[k];
+    std::vector<uint8_t> stream;
+    struct Bufs {
+        DevBuf stack, info, side;
+        MappedBuf out;
+        ~Bufs() {
+            for (DevBuf* b : {&stack, &info, &side}) b->release();
+            out.release();
+        }
+    } B;
+    try {
+        if (!on_gpu) {
+            ThreadPool pool(2);
+            BatchSubmit sub = [&pool](std::function<void()> g) { return pool.submit(std::move(g)); };
+            if (auto w = encode_stacks_async(st.data(), n, stream, sub)) w->collect();
+        } else {
+            const unsigned room = (unsigned)st.size();
+            const size_t bytes = (rans_max_bytes(room) + 15) & ~(size_t)15;
+            RansFrame f{};
+            B.stack.alloc(st.size() * 2);
+            B.info.alloc(rans_info_bytes(room));
+            B.side.alloc((size_t)n * 4);
+            B.out.alloc(bytes + 16 + (size_t)n * 4);
+            CK(cudaMemcpy(B.stack.p, st.data(), st.size() * 2, cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(B.info.p, &n, 4, cudaMemcpyHostToDevice));
+            std::vector<uint32_t> side(n);
+            for (uint32_t k = 0; k < n; k++) side[k] = k * 2654435761u;
+            CK(cudaMemcpy(B.side.p, side.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
+            f.stack = B.stack.as<uint16_t>();
+            f.info = B.info.as<uint4>();
+            f.side = B.side.as<uint32_t>();
+            f.nside = (int)n;
+            f.out = B.out.dev<uint8_t>();
+            f.out_cap = (unsigned)bytes;
+            f.out_bytes = B.out.dev<uint32_t>() + bytes / 4;
+            f.side_out = f.out_bytes + 4;
+            CK(launch_rans(f, std::max(room, 1u), nullptr));
+            CK(cudaDeviceSynchronize());
+            const uint8_t* h = B.out.host<uint8_t>();
+            const uint32_t got = *(const uint32_t*)(h + bytes);
+            if (got == SYM_FAIL || memcmp(h + bytes + 16, side.data(), (size_t)n * 4) != 0) return RIV_ERR_ENCODING_FAILED;
+            stream.assign(h, h + got);
+        }
+    } catch (const CudaError&) {
+        return RIV_ERR_CUDA;
+    } catch (const std::exception&) {
+        return RIV_ERR_ENCODING_FAILED;
+    }
+    *len = stream.size();
+    if (out && cap) memcpy(out, stream.data(), std::min(cap, stream.size()));
+    return RIV_OK;
+}
+
 riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uint32_t threads, uint8_t* out, size_t cap,
                                size_t* len) {
     if ((n > 0 && !blocks) || !len) return RIV_ERR_FRAME;
@@ -2935,10 +3036,11 @@ struct riv_batch {
         uint64_t mbs = 0, pmbs = 0;
     } tpend[2];
     int tpar = 0;
-    // step descriptors: pinned staging (double-buffered), one device copy
+    // step descriptors: pinned staging and device copies, both double-buffered
     HostBuf hdesc[2];
     cudaEvent_t ev_desc[2] = {};
-    DevBuf ddesc;
+    DevBuf ddesc[2];              // the rANS kernels of a step read theirs while the next step's is filled
+    cudaEvent_t ev_ddesc[2] = {};
     size_t off_sp = 0, off_start = 0, off_sstart = 0, desc_bytes = 0;
     int dpar = 0;
     int max_sr = 0;
@@ -2953,7 +3055,7 @@ struct riv_batch {
     int tune_n[3][TUNE_NCAND] = {};      // all-P-frame steps measured per candidate
     uint64_t steps = 0, frames = 0, mbs = 0, launches = 0, timed = 0;
     double stage_us[BT_NSTAGE + 1] = {};  // sums over timed steps (last: whole step)
-    uint64_t h2d_bytes = 0, d2h_bytes = 0;
+    uint64_t h2d_bytes = 0;
     // host milliseconds: [0] making room (earlier records of a clip written before its next
     // frame), [1] descriptors and launches, [2] copies back and step bookkeeping, [3] advancing
     // the clips' pipelines after the step, [4] finish
@@ -3088,7 +3190,8 @@ static void batch_collect(riv_encoder* e, Job& j, int src, const void* frame, cu
     }
     k.sym = sym_frame(e, ck, j.type == 1, s);
     k.sym.status = e->status.as<unsigned>();
-    j.sym = true;
+    k.rans = rans_frame(e, k.sym, s);
+    j.sym = j.rans = true;
     e->ref_cur = nxt;
     e->has_ref = true;
     e->last_par = ck;
@@ -3265,10 +3368,12 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
             CK(cudaEventRecord(b->ev_h2d, b->Hs));
             CK(cudaStreamWaitEvent(B, b->ev_h2d, 0));
         }
-        CK(cudaMemcpyAsync(b->ddesc.p, hd, b->desc_bytes, cudaMemcpyHostToDevice, B));
-        CK(cudaEventRecord(b->ev_desc[b->dpar], B));
+        const int dpar = b->dpar;
         b->dpar ^= 1;
-        const uint8_t* dd = b->ddesc.as<uint8_t>();
+        CK(cudaStreamWaitEvent(B, b->ev_ddesc[dpar], 0));
+        CK(cudaMemcpyAsync(b->ddesc[dpar].p, hd, b->desc_bytes, cudaMemcpyHostToDevice, B));
+        CK(cudaEventRecord(b->ev_desc[dpar], B));
+        const uint8_t* dd = b->ddesc[dpar].as<uint8_t>();
         BatchLaunch L{(const BatchClip*)dd, (const int*)(dd + b->off_start), m};
         cudaEvent_t* evt = b->ev_t[b->tpar];
         auto mark = [&](int k) {
@@ -3300,17 +3405,19 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         const double h1 = now_ms();
         b->host_ms[0] += room;
         b->host_ms[1] += h1 - h0 - room;
-        // ---- copies back: side info and a bounded prefix of the rANS stacks per clip
+        // ---- on C, beside the next step: the rANS streams, written to the slots' pinned buffers
+        // with the side info
         cudaEvent_t xev = b->ev_step[b->steps % b->ev_step.size()];
         CK(cudaStreamWaitEvent(b->C, b->ev_gpu, 0));
+        unsigned max_cap = 0;
+        int max_nmb = 0;
         for (int a = 0; a < m; a++) {
-            riv_encoder* e = b->clips[act[a]];
-            Slot& s = e->slots[jobs[a]->slot];
-            const int N = e->NMB;
-            CK(cudaMemcpyAsync(s.side.p, s.dside.p, (size_t)N * 4, cudaMemcpyDeviceToHost, b->C));
-            copy_stacks(e, *jobs[a], s, b->C);
-            b->d2h_bytes += (uint64_t)N * 4 + s.prefetched;
+            max_cap = std::max(max_cap, b->clips[act[a]]->sym_cap);
+            max_nmb = std::max(max_nmb, b->clips[act[a]]->NMB);
         }
+        CK(launch_batch_rans((const BatchClip*)dd, m, max_cap, max_nmb, b->C));
+        b->launches += 2;
+        CK(cudaEventRecord(b->ev_ddesc[dpar], b->C));
         CK(cudaEventRecord(xev, b->C));
         if (src == 0) {
             for (int a = 0; a < m; a++) {
@@ -3424,6 +3531,8 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
         for (int k = 0; k < 2; k++) {
             CK(cudaEventCreateWithFlags(&b->ev_desc[k], cudaEventDisableTiming));
             CK(cudaEventRecord(b->ev_desc[k], b->B));
+            CK(cudaEventCreateWithFlags(&b->ev_ddesc[k], cudaEventDisableTiming));
+            CK(cudaEventRecord(b->ev_ddesc[k], b->C));
         }
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
         b->off_sp = al((size_t)n * sizeof(BatchClip));
@@ -3434,7 +3543,7 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
             b->hdesc[k].alloc(b->desc_bytes);
             memset(b->hdesc[k].p, 0, b->desc_bytes);
         }
-        b->ddesc.alloc(b->desc_bytes);
+        for (int k = 0; k < 2; k++) b->ddesc[k].alloc(b->desc_bytes);
         int dev = 0, nsm = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -3511,11 +3620,12 @@ void riv_batch_free(riv_batch* b) {
             if (b->ev_t[q][k]) cudaEventDestroy(b->ev_t[q][k]);
     for (int k = 0; k < 2; k++) {
         if (b->ev_desc[k]) cudaEventDestroy(b->ev_desc[k]);
+        if (b->ev_ddesc[k]) cudaEventDestroy(b->ev_ddesc[k]);
         b->hdesc[k].release();
+        b->ddesc[k].release();
     }
     if (b->ev_h2d) cudaEventDestroy(b->ev_h2d);
     if (b->ev_gpu) cudaEventDestroy(b->ev_gpu);
-    b->ddesc.release();
     if (b->B) cudaStreamDestroy(b->B);
     if (b->C) cudaStreamDestroy(b->C);
     if (b->Hs) cudaStreamDestroy(b->Hs);
@@ -3556,7 +3666,8 @@ riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us
         c7[3] = b->launches;
         c7[4] = b->timed;
         c7[5] = b->h2d_bytes;
-        c7[6] = b->d2h_bytes;
+        c7[6] = 0;
+        for (const riv_encoder* e : b->clips) c7[6] += e->d2h_bytes;
     }
     if (stage_us10)
         for (int s = 0; s <= BT_NSTAGE; s++) stage_us10[s] = b->timed ? b->stage_us[s] / (double)b->timed : 0.0;

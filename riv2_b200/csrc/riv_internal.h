@@ -144,6 +144,18 @@ struct SymFrame {
     uint8_t* peobs;
     uint32_t* hdr;    // mapped host words: coded MBs, coefficients, [2] = *status (not nullptr), symbols
     const unsigned* status;
+    uint32_t* nsym;   // not nullptr: the symbols once more, on the device
+};
+// One frame's rANS batches coded on the GPU (riv_rans.cuh).
+struct RansFrame {
+    uint16_t* stack;      // SymFrame's; overwritten
+    uint4* info;          // [0].x = SymFrame::nsym's word, then per batch: words, the two states
+    const uint32_t* side; // nside words, copied to side_out
+    int nside;
+    unsigned out_cap;     // bytes of `out`
+    uint8_t* out;         // pinned host memory, as are side_out and out_bytes
+    uint32_t* side_out;
+    uint32_t* out_bytes;  // the stream's bytes; SYM_FAIL: no stacks
 };
 
 // ---- multi-clip steps (riv_batch): one launch per stage over every clip of the step.
@@ -172,7 +184,8 @@ struct BatchClip {
     const uint8_t* db_src;
     uint8_t* db_dst;
     const uint8_t* db_mask;
-    SymFrame sym;  // symbols into the slot's buffers
+    SymFrame sym;    // symbols into the slot's buffers
+    RansFrame rans;  // and their stream into its pinned ones
 };
 enum BatchStage { BS_CONVERT, BS_TABLE, BS_PREDICT, BS_AQSUM, BS_RESIDUAL, BS_DEBLOCK, BS_SCAN, BS_PACK, BS_N };
 // Tile shapes of a step (chosen by the batch's autotuner; the output does not depend on them).
@@ -188,6 +201,8 @@ struct BatchLaunch {
     int nclips;
 };
 int batch_ctas_host(int stage, const BatchClip& k, const BatchTune& t);
+// The rANS streams and side info of a step's clips (caps: the largest SymFrame::cap and nside).
+int launch_batch_rans(const BatchClip* clips, int nclips, unsigned max_cap, int max_nside, void* stream);
 int launch_batch_stage(int stage, const BatchLaunch& b, const BatchTune& t, int total_ctas, int max_sr, void* stream);
 // Kinds of multi-clip search launches: 64- or 32-bit costs, with an exhaustive SAD table or with
 // the SADs computed on the way.
@@ -245,6 +260,9 @@ int deblock_scratch_address(void** out);
 int launch_symbols(const SymFrame& f, void* stream);
 // Bytes of a frame's cnt, tot, occ, ustate and work; with f, lays them out at p (256-byte aligned).
 size_t sym_workspace(SymFrame* f, int nmb, unsigned cap, void* p);
+int launch_rans(const RansFrame& f, unsigned cap, void* stream);
+size_t rans_info_bytes(unsigned cap);  // of RansFrame::info
+size_t rans_max_bytes(unsigned cap);   // the longest stream of cap symbols
 // libm device helpers exposed for the exhaustive check
 int launch_libm_eval(int which, const float* in, float* out, size_t n, const uint32_t* fix, int nfix, void* stream);
 // Learned-proposal form of the P-frame search and mode decision (riv_kernels.cu): lmv holds 8

@@ -3721,6 +3721,7 @@ int deblock_scratch_address(void** out) { return (int)cudaGetSymbolAddress(out, 
 // K8: side info and coefficient symbols of a frame reconstructed outside a search launch.
 // ---------------------------------------------------------------------------------
 #include "riv_symbols.cuh"
+#include "riv_rans.cuh"
 
 // Multi-clip launches of the stages above (riv_batch).
 #include "riv_batch.cuh"

@@ -5,7 +5,7 @@
 // with one of 427 adaptive models that start fresh every frame.  A model's probability at each
 // of its symbols depends only on the bits it saw before, so the list can be made block-parallel
 // and the models can run beside one another; what stays serial is the rANS state of each
-// 16386-symbol batch, which the host codes from the (probability, bit) stacks left here.  The
+// 16386-symbol batch, which riv_rans.cuh or the host codes from the (probability, bit) stacks left here.  The
 // stacks are laid out as the host's writer fills them: batch k / 16386, newest symbol first.
 //
 //   k_sym_count   one warp per SY_MBS macroblocks: symbols per model, coded MBs, coefficients
@@ -217,6 +217,7 @@ __device__ __forceinline__ void sym_scan_rows(const SymFrame& f, int group) {
             f.hdr[0] = coded;
             f.hdr[1] = coefs;
             f.hdr[3] = ok ? syms : SYM_FAIL;
+            if (f.nsym != nullptr) *f.nsym = ok ? syms : SYM_FAIL;
             if (f.status != nullptr) f.hdr[2] = *(volatile const unsigned*)f.status;
         }
     }

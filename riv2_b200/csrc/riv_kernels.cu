@@ -856,6 +856,320 @@ __device__ __forceinline__ void residual_mb(const ResidualParams& p, int nmb, in
                sT16, sT16t, R, RT, S.aant[0], Q + 256, S.predc);
 }
 
+// ---- two MBs by one warp: lane 16 h + r owns row (then column) r of MB h's luma and row r & 7 of its
+// chroma plane r >> 3, a whole 1-D transform at a time, in registers.
+//
+// The 64-thread form above is bound by its instructions and shared-memory reads: a basis row and a
+// data word per four products.  Here a transform's inputs are registers and its basis constant-bank
+// operands, the symmetry of the basis (T[15 - i][j] = +-T[i][j], and again in the even half) leaves 88
+// products of 256, and the warp needs no barrier.  Sums are the same integers: all arithmetic is
+// modulo 2^32, and every partial sum of a result that fits is recovered exactly.
+// 24 mixed clips (78,456 MBs): 405 -> 200 us; what is left is mostly the quantiser's divisions and
+// roundings, 24 a lane, at half the issue rate.
+constexpr int RP_LP = 20, RP_CP = 12;  // rows of 16 / 8 words, 16-byte steps that visit all banks
+struct __align__(16) ResPair {
+    int32_t L[2][16 * RP_LP + 16];          // the second MB half the banks further
+    int32_t C[2][2][8 * RP_CP + 8];         // chroma planes
+};
+static_assert(sizeof(ResPair::L[0]) % 16 == 0 && sizeof(ResPair::C[0][0]) % 16 == 0, "16-byte rows");
+
+// o[j] = (sum_i d[i] T[i][j] + 2^17) >> 18
+__device__ __forceinline__ void fdct16(const int32_t (&d)[16], int32_t (&o)[16]) {
+    uint32_t s[8], t[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        s[i] = (uint32_t)d[i] + (uint32_t)d[15 - i];
+        t[i] = (uint32_t)d[i] - (uint32_t)d[15 - i];
+    }
+    uint32_t s2[4], t2[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        s2[i] = s[i] + s[7 - i];
+        t2[i] = s[i] - s[7 - i];
+    }
+    const uint32_t s3[2] = {s2[0] + s2[3], s2[1] + s2[2]}, t3[2] = {s2[0] - s2[3], s2[1] - s2[2]};
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const int n = j & 1 ? 8 : j & 2 ? 4 : 2;
+        uint32_t a = 1u << 17;
+#pragma unroll
+        for (int i = 0; i < n; i++) a += (j & 1 ? t[i] : j & 2 ? t2[i] : j & 4 ? t3[i] : s3[i]) * (uint32_t)c_T16[i * 16 + j];
+        o[j] = (int32_t)a >> 18;
+    }
+}
+// o[x] = (sum_j c[j] T[x][j] + 2^17) >> 18
+__device__ __forceinline__ void idct16(const int32_t (&c)[16], int32_t (&o)[16]) {
+    auto part = [&](int x, int j0, int step) {
+        uint32_t a = 0;
+#pragma unroll
+        for (int j = j0; j < 16; j += step) a += (uint32_t)c[j] * (uint32_t)c_T16[x * 16 + j];
+        return a;
+    };
+    uint32_t e[8];
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+        const uint32_t p = part(x, 0, 8) + (1u << 17), q = part(x, 4, 8);
+        e[x] = p + q;
+        e[3 - x] = p - q;
+    }
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+        const uint32_t p = e[x], q = part(x, 2, 4);
+        e[x] = p + q;
+        e[7 - x] = p - q;
+    }
+#pragma unroll
+    for (int x = 0; x < 8; x++) {
+        const uint32_t q = part(x, 1, 2);
+        o[x] = (int32_t)(e[x] + q) >> 18;
+        o[15 - x] = (int32_t)(e[x] - q) >> 18;
+    }
+}
+__device__ __forceinline__ void fdct8(const int32_t (&d)[8], int32_t (&o)[8]) {
+    uint32_t s[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        s[i] = (uint32_t)d[i] + (uint32_t)d[7 - i];
+        t[i] = (uint32_t)d[i] - (uint32_t)d[7 - i];
+    }
+    const uint32_t s2[2] = {s[0] + s[3], s[1] + s[2]}, t2[2] = {s[0] - s[3], s[1] - s[2]};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        uint32_t a = 1u << 17;
+#pragma unroll
+        for (int i = 0; i < (j & 1 ? 4 : 2); i++) a += (j & 1 ? t[i] : j & 2 ? t2[i] : s2[i]) * (uint32_t)c_T8[i * 8 + j];
+        o[j] = (int32_t)a >> 18;
+    }
+}
+// A lane's row into shared memory and back as its column, or the other way round (the warp's other
+// lanes do the same; P words a row).
+template <int N, int P>
+__device__ __forceinline__ void rows_to_cols(int32_t* S, int r, int32_t (&v)[N]) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; k += 4) *(int4*)(S + r * P + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = S[k * P + r];
+}
+template <int N, int P>
+__device__ __forceinline__ void cols_to_rows(int32_t* S, int r, int32_t (&v)[N]) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; k++) S[k * P + r] = v[k];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; k += 4) {
+        const int4 q = *(const int4*)(S + r * P + k);
+        v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+    }
+}
+__device__ __forceinline__ int byte_of(const uint32_t* w, int k) { return (int)((w[k >> 2] >> (8 * (k & 3))) & 255u); }
+// f32_to_i16_sat(roundf(f)): the conversion gives 0 for a NaN and the ends of int's range beyond them.
+__device__ __forceinline__ int round_i16(float f) { return min(max(__float2int_rz(roundf(f)), -32768), 32767); }
+// Four samples of prediction + residual, clamped to 0 .. 255.
+__device__ __forceinline__ uint32_t add_clamped(uint32_t base, const int32_t* r) {
+    uint32_t lo, hi;
+    const int a = (int)(base & 255u) + r[0], b = (int)((base >> 8) & 255u) + r[1];
+    const int c = (int)((base >> 16) & 255u) + r[2], d = (int)(base >> 24) + r[3];
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(d), "r"(c), "r"(0));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(lo) : "r"(b), "r"(a), "r"(hi));
+    return lo;
+}
+__device__ __forceinline__ uint32_t pack16(int a, int b) { return __byte_perm((uint32_t)a, (uint32_t)b, 0x5410); }
+
+// MBs mb0 and mb0 + 1 (where it exists); results as residual_mb's.
+__device__ __forceinline__ void residual_pair(const ResidualParams& p, int nmb, int mb0, int lane, ResPair& S) {
+    const int h = lane >> 4, r = lane & 15, cp = r >> 3, cr = r & 7;
+    const bool ok = mb0 + h < nmb;
+    const int mb = ok ? mb0 + h : mb0;
+    const int W = p.W, H = p.H, CW = W / 2, CH = H / 2;
+    const int bx = mb % p.BW, by = mb / p.BW;
+    const bool intra = p.intra != 0;
+    int32_t *SL = S.L[h], *SC = S.C[h][cp];
+    const size_t yi = (size_t)(by * 16 + r) * W + bx * 16;
+    const size_t chroma = (size_t)W * H + (cp == 0 ? 0 : (size_t)CW * CH);
+    const size_t ci = chroma + (size_t)(by * 8 + cr) * CW + bx * 8;
+    int16_t* co = p.coeffs + (size_t)mb * 384;
+
+    // inputs and the chroma prediction (as residual_mb's), a row of each
+    const uint4 cw = *(const uint4*)(p.cur + yi);
+    const uint2 ccw = *(const uint2*)(p.cur + ci);
+    uint4 pw = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
+    uint32_t pc[2] = {0x80808080u, 0x80808080u};
+    if (!intra) {
+        pw = *(const uint4*)(p.pred + yi);
+        if (p.ref != nullptr) {
+            const MbOut m = p.mb[mb];
+            const int mdx = m.raw[0] * 2 + m.raw[2], mdy = m.raw[1] * 2 + m.raw[3];
+            const int sx0 = bx * 16 + (mdx >> 1), sy0 = by * 16 + (mdy >> 1);
+            const bool copy = ((mdx | mdy) & 1) == 0 && sx0 >= 0 && sy0 >= 0 && sx0 + 15 < W && sy0 + 15 < H;
+            const uint8_t* Rp = p.ref + chroma;
+            if (copy) {  // aligned words that hold the 8 samples, none beyond them
+                const uint8_t* src = Rp + (size_t)(sy0 / 2 + cr) * CW + sx0 / 2;
+                const unsigned off = (unsigned)((size_t)src & 3u);
+                const uint32_t* a = (const uint32_t*)(src - off);
+                const uint32_t w0 = a[0], w1 = a[1], w2 = off != 0u ? a[2] : 0u;
+                pc[0] = __funnelshift_r(w0, w1, 8 * off);
+                pc[1] = __funnelshift_r(w1, w2, 8 * off);
+            } else {
+                pc[0] = pc[1] = 0u;
+                const int yh = 2 * (by * 8 + cr) + (mdy >> 1);
+#pragma unroll 4
+                for (int k = 0; k < 8; k++) {
+                    const uint32_t s = (uint32_t)sample_round(Rp, CW, CH, 2 * (bx * 8 + k) + (mdx >> 1), yh) << (8 * (k & 3));
+                    if (k < 4) pc[0] |= s;
+                    else pc[1] |= s;
+                }
+            }
+        } else {
+            const uint2 q = *(const uint2*)(p.pred + ci);
+            pc[0] = q.x;
+            pc[1] = q.y;
+        }
+    }
+    float qsv = 0.0f;
+    bool skip = false;
+    if (!intra) {
+        if (p.lnv != nullptr) {  // AQ step (compute_aq_quant_steps, res/residual.rs:154-167)
+            const float off = __fmul_rn(0.8f, __fsub_rn(p.lnv[mb], p.lnv[nmb]));
+            qsv = __fmul_rn(p.aq_base, glibc_exp2f(__fdiv_rn(off, 6.0f), p.expfix, p.nexp));
+            if (ok && r == 0) p.qs_out[mb] = qsv;
+        } else {
+            qsv = p.qs[mb];
+        }
+        skip = p.mb[mb].rdo_skip != 0;  // never transformed: residual 0, recon = prediction
+    }
+    auto copy_pred = [&]() {  // recon = prediction, coefficients zero
+        *(uint4*)(p.recon + yi) = pw;
+        *(uint2*)(p.recon + ci) = make_uint2(pc[0], pc[1]);
+        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+        *(uint4*)(co + r * 16) = z;
+        *(uint4*)(co + r * 16 + 8) = z;
+        *(uint4*)(co + 256 + cp * 64 + cr * 8) = z;
+        if (r == 0) {
+            p.opt_skip[mb] = 1;
+            const int8_t* c = p.mb[mb].coded;
+            p.fmask[mb] = (c[0] | c[1] | c[2] | c[3]) != 0;
+            p.eobs[3 * mb] = p.eobs[3 * mb + 1] = p.eobs[3 * mb + 2] = 0;
+        }
+    };
+    if (__all_sync(0xffffffffu, skip || !ok)) {
+        if (ok) copy_pred();
+        return;
+    }
+    int32_t v[16], c[8];
+    {
+        const uint32_t a[4] = {cw.x, cw.y, cw.z, cw.w}, b[4] = {pw.x, pw.y, pw.z, pw.w}, ca[2] = {ccw.x, ccw.y};
+        int32_t d[16], dc[8];
+#pragma unroll
+        for (int k = 0; k < 16; k++) d[k] = byte_of(a, k) - byte_of(b, k);
+#pragma unroll
+        for (int k = 0; k < 8; k++) dc[k] = byte_of(ca, k) - byte_of(pc, k);
+        fdct16(d, v);
+        fdct8(dc, c);
+    }
+    rows_to_cols<16, RP_LP>(SL, r, v);
+    rows_to_cols<8, RP_CP>(SC, cr, c);
+    {
+        int32_t o[16], oc[8];
+        fdct16(v, o);
+        fdct8(c, oc);
+        cols_to_rows<16, RP_LP>(SL, r, o);
+        cols_to_rows<8, RP_CP>(SC, cr, oc);
+        // quantisation
+        if (intra) {
+            const uint4 y0 = *(const uint4*)(p.intra_ytab + r * 16), y1 = *(const uint4*)(p.intra_ytab + r * 16 + 8);
+            const uint4 ct = *(const uint4*)(p.intra_ctab + cr * 8);
+            const uint32_t yt[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w}, cq[4] = {ct.x, ct.y, ct.z, ct.w};
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const int q = max((int)((yt[k >> 1] >> (16 * (k & 1))) & 0xffffu), 1);
+                v[k] = round_i16(__fdiv_rn(__int2float_rn(o[k]), (float)q));
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int q = max((int)((cq[k >> 1] >> (16 * (k & 1))) & 0xffffu), 1);
+                c[k] = round_i16(__fdiv_rn(__int2float_rn(oc[k]), (float)q));
+            }
+        } else {
+            auto quant = [&](int32_t x) {
+                const float q = __fdiv_rn(__int2float_rn(x), qsv);
+                return fabsf(q) < p.dead_zone ? 0 : round_i16(q);
+            };
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = quant(o[k]);
+#pragma unroll
+            for (int k = 0; k < 8; k++) c[k] = quant(oc[k]);
+        }
+    }
+    // last non-zero index per plane block (0 when all zero)
+    int ly = -1, lc = -1;
+#pragma unroll
+    for (int k = 0; k < 16; k++) ly = v[k] != 0 ? k : ly;
+#pragma unroll
+    for (int k = 0; k < 8; k++) lc = c[k] != 0 ? k : lc;
+    const unsigned my = __ballot_sync(0xffffffffu, ly >= 0) >> (16 * h) & 0xffffu, mc = __ballot_sync(0xffffffffu, lc >= 0) >> (16 * h) & 0xffffu;
+    const int ry = 31 - __clz((int)(my | 1u)), ru = 31 - __clz((int)((mc & 255u) | 1u)), rv = 31 - __clz((int)((mc >> 8) | 1u));
+    const int ey = my ? 16 * ry : 0, eu = mc & 255u ? 8 * ru : 0, ev = mc >> 8 ? 8 * rv : 0;
+    const int ky = __shfl_sync(0xffffffffu, ly, 16 * h + ry), ku = __shfl_sync(0xffffffffu, lc, 16 * h + ru), kv = __shfl_sync(0xffffffffu, lc, 16 * h + 8 + rv);
+    const bool copied = !intra && (skip || (my | mc) == 0u);  // or all zero after quantisation: optimized skip
+    if (!copied && ok) {
+        *(uint4*)(co + r * 16) = make_uint4(pack16(v[0], v[1]), pack16(v[2], v[3]), pack16(v[4], v[5]), pack16(v[6], v[7]));
+        *(uint4*)(co + r * 16 + 8) = make_uint4(pack16(v[8], v[9]), pack16(v[10], v[11]), pack16(v[12], v[13]), pack16(v[14], v[15]));
+        *(uint4*)(co + 256 + cp * 64 + cr * 8) = make_uint4(pack16(c[0], c[1]), pack16(c[2], c[3]), pack16(c[4], c[5]), pack16(c[6], c[7]));
+        if (r == 0) {
+            p.eobs[3 * mb] = (uint8_t)(ey + max(ky, 0));
+            p.eobs[3 * mb + 1] = (uint8_t)(eu + max(ku, 0));
+            p.eobs[3 * mb + 2] = (uint8_t)(ev + max(kv, 0));
+            p.opt_skip[mb] = 0;
+            p.fmask[mb] = 1;
+        }
+    }
+    if (copied && ok) copy_pred();
+    if (__all_sync(0xffffffffu, copied || !ok)) return;
+    // dequantisation, inverse transforms and reconstruction (inverse_mb's arithmetic)
+    {
+        int32_t d[16], o[16];
+        if (intra) {
+            const uint4 y0 = *(const uint4*)(p.intra_ytab + r * 16), y1 = *(const uint4*)(p.intra_ytab + r * 16 + 8);
+            const uint32_t yt[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+            for (int k = 0; k < 16; k++) d[k] = v[k] * max((int)((yt[k >> 1] >> (16 * (k & 1))) & 0xffffu), 1);
+        } else {
+            const int32_t qfp = f32_to_i32_sat(roundf(__fmul_rn(qsv, 16384.0f)));
+#pragma unroll
+            for (int k = 0; k < 16; k++) d[k] = wadd(wmul(v[k], qfp), 8192) >> 14;
+        }
+        idct16(d, o);
+        rows_to_cols<16, RP_LP>(SL, r, o);
+        idct16(o, d);
+        cols_to_rows<16, RP_LP>(SL, r, d);
+        if (!copied && ok)  // (14 bits are left of a residual: inverse_mb's clamp to 16 never applies)
+            *(uint4*)(p.recon + yi) = make_uint4(add_clamped(pw.x, d), add_clamped(pw.y, d + 4), add_clamped(pw.z, d + 8), add_clamped(pw.w, d + 12));
+    }
+    {
+        int32_t s[8], o[8];
+        if (intra) {
+            const uint4 ct = *(const uint4*)(p.intra_ctab + cr * 8);
+            const uint32_t cq[4] = {ct.x, ct.y, ct.z, ct.w};
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] = c[k] * max((int)((cq[k >> 1] >> (16 * (k & 1))) & 0xffffu), 1);
+        } else {
+            float qr = roundf(qsv);
+            qr = qr < 1.0f ? 1.0f : qr;
+            const int32_t qa = qr >= 65535.0f ? 65535 : (int32_t)qr;
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] = c[k] * qa;
+        }
+        aan_1d(s, o, 512, 10);
+        rows_to_cols<8, RP_CP>(SC, cr, o);
+        aan_1d(o, s, 65536, 17);
+        cols_to_rows<8, RP_CP>(SC, cr, s);
+        if (!copied && ok) *(uint2*)(p.recon + ci) = make_uint2(add_clamped(pc[0], s), add_clamped(pc[1], s + 4));
+    }
+}
+
 __device__ __forceinline__ int c128(int x) { return min(max(x, -128), 127); }
 __device__ __forceinline__ void filter_line(int* px, int E, int I, int Hv) {
     int p3 = px[0], p2 = px[1], p1 = px[2], p0 = px[3], q0 = px[4], q1 = px[5], q2 = px[6], q3 = px[7];
@@ -3549,7 +3863,8 @@ int launch_aq(const uint2* varsum, int n, float base, const uint32_t* logfix, in
 // res/residual.rs:520-752).  Intra: pixel-128, JPEG-derived matrices, no dead zone
 // (res/residual.rs:267-388, dct16.rs:420-560, dct8.rs:142-196).
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_residual(ResidualParams p, int nmb) {
+// 64 threads an MB.
+__global__ void __launch_bounds__(64 * RS_MB) k_residual(ResidualParams p, int nmb) {
     __shared__ __align__(16) int32_t sT16[256], sT16t[256], sT8[64];
     __shared__ __align__(16) ResSmem S[RS_MB];
     const int tid = threadIdx.x;
@@ -3561,6 +3876,13 @@ __global__ void __launch_bounds__(256) k_residual(ResidualParams p, int nmb) {
     const int mb = blockIdx.x * RS_MB + g;
     if (mb >= nmb) return;
     residual_mb(p, nmb, mb, u, g + 1, S[g], sT16, sT16t, sT8);
+}
+// A warp for two.
+constexpr int RP_MB = 4;  // MBs of a CTA
+__global__ void __launch_bounds__(16 * RP_MB, 12) k_residual_pairs(ResidualParams p, int nmb) {
+    __shared__ ResPair S[RP_MB / 2];
+    const int w = threadIdx.x >> 5, mb = blockIdx.x * RP_MB + 2 * w;
+    if (mb < nmb) residual_pair(p, nmb, mb, threadIdx.x & 31, S[w]);
 }
 
 // Decoder reconstruction (res/residual.rs:815-887 intra, :889-1079 inter): the decoded
@@ -3620,7 +3942,12 @@ int launch_reconstruct(const int16_t* coeffs, const uint8_t* pred, const uint8_t
 }
 
 int launch_residual(const ResidualParams& p, int nmb, void* stream) {
-    k_residual<<<(nmb + RS_MB - 1) / RS_MB, 64 * RS_MB, 0, (cudaStream_t)stream>>>(p, nmb);
+    // A warp's transforms take longer than four warps' shares of them: below one CTA of pairs an SM the
+    // form with more threads is quicker (CIF 7.5 against 8.4 us), above it the pairs (640x368 9.5
+    // against 8.5, 1080p 39 against 20, 4K 138 against 60).
+    constexpr int RES_PAIRS_MIN = 148 * RP_MB;
+    if (nmb < RES_PAIRS_MIN) k_residual<<<(nmb + RS_MB - 1) / RS_MB, 64 * RS_MB, 0, (cudaStream_t)stream>>>(p, nmb);
+    else k_residual_pairs<<<(nmb + RP_MB - 1) / RP_MB, 16 * RP_MB, 0, (cudaStream_t)stream>>>(p, nmb);
     return (int)cudaGetLastError();
 }
 

@@ -204,7 +204,8 @@ riv_status riv_batch_set_tune(riv_batch* b, const riv_batch_tune* t);
 riv_status riv_batch_get_tune(const riv_batch* b, riv_batch_tune* t, int* tuned);
 /* c7 = {steps, frames, MBs, kernel launches, timed steps, host->device bytes, device->host
  * bytes}; stage_us10 = mean GPU microseconds per timed step: conversion, SAD tables, search,
- * prediction, AQ mean, residual, deblock, scan, pack, whole step.  Either may be NULL. */
+ * prediction, AQ mean, residual, deblock, symbol counts, symbols and models, whole step (the rANS
+ * batches run beside the next step and are not in it).  Either may be NULL. */
 riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us10);
 /* Cumulative host milliseconds: [0] waiting for a clip's earlier records before its next
  * frame (pipeline full), [1] descriptors and launches, [2] copies back and bookkeeping,

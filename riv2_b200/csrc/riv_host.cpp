@@ -2,7 +2,7 @@
 // kernel sequence, the frame pipeline and the host entropy stage.
 //
 // Per P-frame (one CUDA stream):  rgb->yuv -> search/mode wavefront -> predict+variance
-// -> AQ -> residual/DCT/quant/recon -> deblock -> compaction; a copy stream brings the
+// -> AQ -> residual/DCT/quant/recon -> deblock -> coefficient symbols; a copy stream brings the
 // per-MB side info and the coded MBs' coefficients back; the host runs the motion-vector
 // rANS coder (ordered, contexts persist across frames), the DCT-coefficient rANS coder
 // (fresh contexts per frame, so frames code in parallel on a thread pool) and writes the
@@ -322,7 +322,7 @@ struct MappedBuf {
     T* dev() const { return (T*)d; }
 };
 
-// Per-frame timing events: Y = input stream, S = main chain, K = compaction stream.
+// Per-frame timing events: Y = input stream, S = main chain, K = symbol stream.
 constexpr int NPAR = 3;  // rotation depth of the per-frame device buffers
 constexpr uint64_t TIMING_SAMPLE = 8;  // pipelined frames carry stage timing events one in this many
 enum { EV_START, EV_YUV, EV_S0, EV_TABLE, EV_SEARCH, EV_PRED, EV_AQ, EV_RES, EV_DEBLOCK, EV_K0, EV_COMPACT, EV_NET0, EV_NET1, EV_N };
@@ -343,7 +343,7 @@ struct Job {
     uint64_t index = 0, ts = 0;
     int type = 0, slot = 0;
     int state = 0;  // 0 submitted, 1 entropy running
-    bool tail_done = true;  // compaction and copies enqueued (false while the frame is pending)
+    bool tail_done = true;  // symbols (or compaction) and copies enqueued (false while the frame is pending)
     bool deferred = false;  // reconstructed inside the next P-frame's search launch
     bool timed = false;     // stage timing events recorded for this frame
     // multi-clip step (riv_batch): one event marks the step's GPU work and copies done, in
@@ -387,7 +387,7 @@ struct riv_encoder {
     int W = 0, H = 0, BW = 0, BH = 0, NMB = 0;
     size_t yuv_bytes = 0;
     cudaStream_t S = nullptr, C = nullptr, Hs = nullptr;  // main chain, device->host, host->device
-    cudaStream_t Y = nullptr, K = nullptr;                // input conversion, compaction
+    cudaStream_t Y = nullptr, K = nullptr;                // input conversion, coefficient symbols
     // what a frame's first copy left out, copied once the frame is done: on C it would wait for
     // the copies of every later frame in flight
     cudaStream_t R = nullptr;
@@ -3419,7 +3419,7 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
         };
         auto stage = [&](int s, int tb) {
             CK(launch_batch_stage(s, L, t, tot[s], b->max_sr, B));
-            if (tot[s] > 0) b->launches++;
+            if (tot[s] > 0) b->launches += s == BS_SCAN ? 2 : s == BS_PACK ? 3 : 1;
             mark(tb);
         };
         mark(TB_START);

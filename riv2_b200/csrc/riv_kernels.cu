@@ -3064,7 +3064,7 @@ __global__ void __maxnreg__(120) k_search(SearchParams p) {
 int sad_table_stride(int sr) { return ((2 * sr + 1) * (2 * sr + 1) + 7) & ~7; }
 bool search_use_table(int sr) { return sr <= 15; }
 // A fused launch without a table needs fewer CTAs beside the rows: the row CTAs' spare warps take
-// worker tasks too until their row starts (2160 rows of MBs leave 13).
+// worker tasks too until their row starts (frames of 2160 pixel rows leave 13).
 constexpr int SEARCH_DIRECT_WORKERS = 8;
 enum SearchKind { SK_TABLE_SMALL, SK_TABLE, SK_DIRECT, SK_PLAIN };  // PLAIN: 64-bit costs, no table
 static bool search_fast(bool band, SearchKind k) { return k == SK_DIRECT || (band && k != SK_PLAIN); }

@@ -203,7 +203,8 @@ riv_status riv_batch_set_tune(riv_batch* b, const riv_batch_tune* t);
 /* The shapes in use; *tuned = 0 still tuning, 1 chosen by the autotuner, 2 fixed. */
 riv_status riv_batch_get_tune(const riv_batch* b, riv_batch_tune* t, int* tuned);
 /* c7 = {steps, frames, MBs, kernel launches, timed steps, host->device bytes, device->host
- * bytes}; stage_us10 = mean GPU microseconds per timed step: conversion, SAD tables, search,
+ * bytes}; stage_us10 = mean GPU microseconds per timed step: waiting for the conversion (which
+ * runs beside the step before), SAD tables, search,
  * prediction, AQ mean, residual, deblock, symbol counts, symbols and models, whole step (the rANS
  * batches run beside the next step and are not in it).  Either may be NULL. */
 riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us10);

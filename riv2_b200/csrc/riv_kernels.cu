@@ -2253,7 +2253,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     // FAST (DIRECT, or band and table): search chain, mode decision, loader and AQ warps.  Otherwise
     // the search warp stages its own data with cp.async and only the mode warp runs beside it.  RING:
     // the loader brings each MB's window instead of the row's band.  DIRECT (32-bit costs, no table): the integer SADs are computed on the chain, four
-    // positions at a time (8 lanes each).  1080p at search range 31: 0.99 ms a frame with the
+    // positions at a time (8 lanes each).  1080p at search range 31: 0.78 ms a frame with the
     // previous frame's reconstruction in the launch, where one position at a time on 64-bit costs,
     // its prediction, AQ, residual and deblock in kernels of their own, took 1.60 ms.
     constexpr bool DIRECT = SMALL && !TABLE, FAST = (BAND && TABLE) || DIRECT, RING = DIRECT && !BAND;
@@ -3142,9 +3142,9 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         pl.grid = pl.nrow = BH < per_sm * nsm ? BH : per_sm * nsm;
         return cudaSuccess;
     };
-    // A table wherever there is one: its chain is 1100 cycles a MB shorter (at 2160 rows a table
-    // kernel, the search, the residual and the deblock take 1.9 ms a frame, a fused direct launch
-    // 2.4 ms; at 1080 rows 0.63 ms against 0.99).
+    // A table wherever there is one: its chain is shorter (at 2160 rows a table kernel, the search,
+    // the residual and the deblock take 1.57 ms a frame, a fused direct launch 1.84-1.94 ms; at 1080
+    // rows 0.55 ms against 0.79-0.87).
     e = plan(table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN, *out);
     return (int)e;
 }

@@ -248,7 +248,9 @@ int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* 
     const void* fn = search_multi_fn((SearchKind)kind);
     const size_t sm = search_smem(max_sr, 0, false, (SearchKind)kind);
     const int nt = search_threads(search_fast(false, (SearchKind)kind));
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    int room = 0;
+    cudaError_t e = open_smem(fn, &room);
+    if (e == cudaSuccess && sm > (size_t)room) e = cudaErrorInvalidValue;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nt, sm);
     *smem = sm;
     *threads = nt;

@@ -3088,6 +3088,20 @@ static const void* search_fn(bool band, SearchKind k) {
     }
 }
 
+// Lets launches of a kernel ask for as much shared memory as a CTA may have (`room`).  The limit belongs
+// to the kernel and not to an encoder: set to one encoder's own size, it made a larger encoder's next
+// launch fail as soon as a smaller one had been made.
+static cudaError_t open_smem(const void* fn, int* room) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, fn);
+    if (e != cudaSuccess) return e;
+    *room = optin - (int)a.sharedSizeBytes;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, *room);
+}
+
 int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) {
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -3096,7 +3110,9 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
     if (e != cudaSuccess) return (int)e;
     const void* fn = nullptr;
     auto resident = [&](size_t sm, int nthreads, int* per_sm) {
-        cudaError_t r = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        int room = 0;
+        cudaError_t r = open_smem(fn, &room);
+        if (r == cudaSuccess && sm > (size_t)room) r = cudaErrorInvalidValue;
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nthreads, sm);
         return r;
     };

@@ -681,7 +681,9 @@ int nn_gemm(const void* A, int lda, const void* B, int ldb, void* D, int ldd, co
     const int stage = (128 * bk * 2 + ntile * bk * 2 + 1023) & ~1023;
     const size_t smem = 1024 + (size_t)GEMM_STAGES * stage + 256;
     const void* fn = bk == 64 ? (const void*)k_nn_gemm<64> : (const void*)k_nn_gemm<32>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit of the widest tile (256 columns): it belongs to the kernel, and another thread's product
+    // may be launched between this call and the launch below
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 1280 + GEMM_STAGES * 384 * bk * 2);
     if (e != cudaSuccess) return (int)e;
     dim3 grid((M + 127) / 128, splits, N / ntile);
     if (bk == 64)

@@ -3088,6 +3088,15 @@ static const void* search_fn(bool band, SearchKind k) {
     }
 }
 
+// Shared memory a CTA may have on this architecture.
+constexpr size_t SEARCH_SMEM_CTA = (size_t)227 * 1024;
+// The kind without a table: the direct one where a CTA holds its band or ring of windows (a ring up to a
+// search range of 101: 232,416 bytes; 102 asks for 234,336 and 127 for 317,152), else the plain one,
+// which holds one window (93 KB at 127) and one position at a time.
+static SearchKind untabled_kind(int sr, int W, bool band, bool small) {
+    return small && search_smem(sr, W, band, SK_DIRECT) <= SEARCH_SMEM_CTA ? SK_DIRECT : SK_PLAIN;
+}
+
 // Lets launches of a kernel ask for as much shared memory as a CTA may have (`room`).  The limit belongs
 // to the kernel and not to an encoder: set to one encoder's own size, it made a larger encoder's next
 // launch fail as soon as a smaller one had been made.
@@ -3133,7 +3142,7 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
             // row CTAs' helper region (live flag + three worker groups) after the row layout,
             // where the per-CTA maximum allows it
             const size_t with_helpers = ((sm + 15) & ~(size_t)15) + 16 + (size_t)worker_region_bytes(3);
-            const bool helpers = with_helpers <= (size_t)227 * 1024;
+            const bool helpers = with_helpers <= SEARCH_SMEM_CTA;
             const size_t need = helpers ? with_helpers : sm;
             const size_t smf = need > (size_t)116 * 1024 ? need : (size_t)116 * 1024;
             cudaError_t r = resident(smf, 4 * 128, &per_sm);
@@ -3161,8 +3170,8 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
     // A table wherever there is one: its chain is shorter (at 2160 rows a table kernel, the search,
     // the residual and the deblock take 1.57 ms a frame, a fused direct launch 1.84-1.94 ms; at 1080
     // rows 0.55 ms against 0.79-0.87).
-    e = plan(table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN, *out);
-    return (int)e;
+    const SearchKind untabled = untabled_kind(sr, W, use_band(SK_DIRECT), small);
+    return (int)plan(table ? (small ? SK_TABLE_SMALL : SK_TABLE) : untabled, *out);
 }
 
 int launch_search(const SearchParams& p, const SearchPlan& plan, void* stream) {

@@ -41,3 +41,24 @@ def test_batches_of_two_ranges():
         b.finish()
         b.close()
         assert wr.into_inner() == _oracle(oc, f)
+
+
+def _encode(gc, frames):
+    from riv2_b200 import encoder as E
+    wr = E.VecWriter()
+    enc = E.Encoder.new(gc, wr)
+    for t, f in enumerate(frames):
+        enc.encode_frame(E.Frame(f, gc.display_width, gc.display_height, 20 * t))
+    enc.finish()
+    enc.close()
+    return wr.into_inner()
+
+
+@pytest.mark.parametrize("depth", [0, 4])
+@pytest.mark.parametrize("w,h,sr", [(640, 48, 96), (640, 48, 101), (640, 48, 102), (640, 64, 127), (1920, 32, 127)])
+def test_widest_ranges(w, h, sr, depth):
+    """Both sides of the range above which four windows no longer fit (101), where the band does not
+    either."""
+    frames = _frames(w, h, 3, w + sr)
+    gc, oc = _configs(w, h, sr, depth)
+    assert _encode(gc, frames) == _oracle(oc, frames)

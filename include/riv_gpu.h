@@ -316,6 +316,10 @@ riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uin
  * or a class it refuses: RIV_ERR_ENCODING_FAILED). */
 riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, uint32_t n, int intra, uint32_t max_symbols,
                                    uint8_t* out, size_t cap, size_t* len, int* on_gpu);
+/* Test hook (no reference counterpart): the search launch that an encoder of this storage size gets with
+ * 32-bit (small != 0) or 64-bit costs: out7 = {SAD table, loader warps, band, fused, CTAs of MB rows, all
+ * CTAs, bytes of shared memory a CTA}. */
+riv_status riv_test_search_plan(uint32_t w, uint32_t h, uint32_t search_range, int small, int32_t* out7);
 /* Test hook (no reference counterpart): the rANS stream of n symbols (probability of a 0 in 1/256
  * | bit << 8), coded in batches by the host (on_gpu == 0) or the GPU, as a batch's frames are. */
 riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_t* out, size_t cap, size_t* len);

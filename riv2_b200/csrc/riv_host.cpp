@@ -2513,6 +2513,15 @@ riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, u
     return RIV_OK;
 }
 
+riv_status riv_test_search_plan(uint32_t w, uint32_t h, uint32_t search_range, int small, int32_t* out7) {
+    if (w == 0 || h == 0 || w % 16 || h % 16 || search_range > 127 || !out7) return RIV_ERR_INVALID_CONFIG;
+    SearchPlan p{};
+    if (search_plan((int)search_range, (int)w, (int)h / 16, search_use_table((int)search_range), small != 0, &p)) return RIV_ERR_CUDA;
+    const int v[7] = {p.table, p.fast, p.band, p.fused, p.nrow, p.grid, (int)p.smem};
+    for (int k = 0; k < 7; k++) out7[k] = v[k];
+    return RIV_OK;
+}
+
 riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_t* out, size_t cap, size_t* len) {
     if ((n > 0 && !symbols) || !len) return RIV_ERR_FRAME;
     entropy_init();

@@ -228,6 +228,7 @@ struct SearchPlan {
     const void* fn;
     bool fast;   // loader and AQ warps (prediction and AQ in the launch)
     bool table;  // searches an exhaustive SAD table
+    bool band;   // each CTA holds its MB row's reference band
     bool fused;
     bool helpers;  // fused: row CTAs' spare threads and finished row CTAs take worker tasks
     int grid, nrow, threads;

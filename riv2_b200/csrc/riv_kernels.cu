@@ -3090,6 +3090,12 @@ static const void* search_fn(bool band, SearchKind k) {
 
 // Shared memory a CTA may have on this architecture.
 constexpr size_t SEARCH_SMEM_CTA = (size_t)227 * 1024;
+// Whether a CTA holds its row's band.  Without one the direct kind fetches a window for every MB: up to
+// all a CTA may have, as its loader's slots come on top of a band that other kinds hold in 200 KB
+// (640x360 at search range 96: 204 KB; 0.30 ms a frame with the band, 0.96 with windows).
+static bool search_band(int sr, int W, SearchKind k) {
+    return search_smem(sr, W, true, k) <= (k == SK_DIRECT ? SEARCH_SMEM_CTA : SEARCH_SMEM_MAX);
+}
 // The kind without a table: the direct one where a CTA holds its band or ring of windows (a ring up to a
 // search range of 101: 232,416 bytes; 102 asks for 234,336 and 127 for 317,152), else the plain one,
 // which holds one window (93 KB at 127) and one position at a time.
@@ -3125,7 +3131,7 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, nthreads, sm);
         return r;
     };
-    auto use_band = [&](SearchKind k) { return search_smem(sr, W, true, k) <= SEARCH_SMEM_MAX; };
+    auto use_band = [&](SearchKind k) { return search_band(sr, W, k); };
     // The plan of one kind: fused when it can be, else one CTA per MB row (as many as fit).
     // fused: one CTA per SM (the shared-memory request rules out a second), rows first, workers on
     // the SMs the rows leave free; a table's MBs need at least 32 of those.
@@ -3137,6 +3143,7 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         pl.fn = fn;
         pl.fast = search_fast(band, k);
         pl.table = tab;
+        pl.band = band;
         int per_sm = 0;
         if (pl.fast) {
             // row CTAs' helper region (live flag + three worker groups) after the row layout,

@@ -122,7 +122,7 @@ EXPORTED_SYMBOLS = (
     "riv_stage_rgb_to_yuv", "riv_stage_deblock", "riv_stage_libm", "riv_libm_fixup_counts", "riv_dct_tables",
     "riv_debug_frame_state", "riv_counters", "riv_host_times", "riv_stage_deblock_noalloc",
     "riv_decoder_new", "riv_decoder_info", "riv_decode_frame_yuv", "riv_decode_frame_rgb", "riv_decoder_current_frame",
-    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_encode_gpu", "riv_test_dct_decode", "riv_test_rans", "riv_test_mv_encode",
+    "riv_decoder_last_error", "riv_decoder_free", "riv_test_dct_encode", "riv_test_dct_encode_gpu", "riv_test_dct_decode", "riv_test_rans", "riv_test_search_plan", "riv_test_mv_encode",
     "riv_test_mv_decode", "riv_test_delta_bias", "riv_test_worker_queue", "riv_test_libm_range",
     "riv_stage_predict", "riv_stage_residual", "riv_test_wait_expiry", "riv_encoder_set_proposal",
     "riv_learned_counters", "riv_test_mv_encode_threads",
@@ -695,6 +695,15 @@ def dct_encode_gpu(blocks: np.ndarray, intra: bool, skip: Optional[np.ndarray] =
     if st != 0:
         raise _ERRORS.get(st, EncodeError)(f"riv_test_dct_encode_gpu failed (status {st})")
     return out[:n.value].tobytes(), bool(g.value)
+
+
+def search_plan(w: int, h: int, search_range: int, small: bool = True) -> dict:
+    """The search launch of an encoder of this storage size (test hook)."""
+    v = (C.c_int32 * 7)()
+    st = lib().riv_test_search_plan(w, h, search_range, int(small), v)
+    if st != 0:
+        raise _ERRORS.get(st, EncodeError)(f"riv_test_search_plan failed (status {st})")
+    return dict(zip(("table", "loader", "band", "fused", "row_ctas", "ctas", "smem"), list(v)))
 
 
 def rans_stream(symbols: np.ndarray, on_gpu: bool) -> bytes:

@@ -62,3 +62,12 @@ def test_widest_ranges(w, h, sr, depth):
     frames = _frames(w, h, 3, w + sr)
     gc, oc = _configs(w, h, sr, depth)
     assert _encode(gc, frames) == _oracle(oc, frames)
+
+
+@pytest.mark.parametrize("w,h,sr", [(640, 368, 98), (960, 544, 73), (1920, 1088, 36)])
+def test_band_kept(w, h, sr):
+    """The widest ranges at which a row's band fits 200 KB without a loader: it is kept with the
+    loader's slots on top."""
+    from riv2_b200 import encoder as E
+    p = E.search_plan(w, h, sr)
+    assert p["band"] and p["loader"] and not p["table"]

@@ -178,8 +178,8 @@ static const void* search_multi_fn(SearchKind k) {
     }
 }
 
-static size_t batch_stage_smem(int s, int max_sr) {
-    if (s == BS_TABLE) return sad_table_smem(max_sr);
+static size_t batch_stage_smem(int s, int table_sr) {
+    if (s == BS_TABLE) return sad_table_smem(table_sr);
     if (s == BS_AQSUM) return 8192 * sizeof(float);
     return 0;
 }
@@ -197,20 +197,14 @@ static int batch_stage_threads(int s, const BatchTune& t) {
 
 int batch_ctas_host(int s, const BatchClip& k, const BatchTune& t) { return batch_ctas(s, k, t); }
 
-int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int total, int max_sr, void* stream) {
+int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int total, int table_sr, void* stream) {
     if (total <= 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t sm = batch_stage_smem(s, max_sr);
+    const size_t sm = batch_stage_smem(s, table_sr);
     const int nt = batch_stage_threads(s, t);
     switch (s) {
         case BS_CONVERT: kb_convert<<<total, nt, 0, st>>>(b); break;
-        case BS_TABLE:
-            if (sm > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(kb_table, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-                if (e != cudaSuccess) return (int)e;
-            }
-            kb_table<<<total, nt, sm, st>>>(b);
-            break;
+        case BS_TABLE: kb_table<<<total, nt, sm, st>>>(b); break;
         case BS_PREDICT: kb_predict<<<total, nt, 0, st>>>(b); break;
         case BS_AQSUM: kb_aqsum<<<total, nt, sm, st>>>(b); break;
         case BS_RESIDUAL:
@@ -239,8 +233,8 @@ int launch_batch_stage(int s, const BatchLaunch& b, const BatchTune& t, int tota
     return (int)cudaGetLastError();
 }
 
-int search_multi_kind(bool table, bool small) {
-    return table ? (small ? SK_TABLE_SMALL : SK_TABLE) : small ? SK_DIRECT : SK_PLAIN;
+int search_multi_kind(bool table, bool small, int sr) {
+    return table ? (small ? SK_TABLE_SMALL : SK_TABLE) : untabled_kind(sr, 0, false, small);
 }
 bool search_multi_predicts(int kind) { return search_fast(false, (SearchKind)kind); }
 

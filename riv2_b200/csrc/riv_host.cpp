@@ -418,6 +418,7 @@ struct riv_encoder {
     unsigned sym_cap = 0;               // symbols a frame may have there, and its slot's stacks
     DevBuf mvbits, logfix, expfix, ytab, ctab, newcost, newcost32;
     bool small_costs = false;
+    int multi_kind = 0;     // in a batch: its kind of search without a SAD table
     bool table_ok = false;  // exhaustive SAD table + packed argmin usable (costs < 2^59)
     int ref_cur = 0, coded_cur = 0;
     bool has_ref = false, has_prev_mvs = false;
@@ -3061,7 +3062,7 @@ struct riv_batch {
     cudaEvent_t ev_ddesc[2] = {};
     size_t off_sp = 0, off_start = 0, off_sstart = 0, desc_bytes = 0;
     int dpar = 0;
-    int max_sr = 0;
+    int table_sr = 0;  // the largest search range among the clips that have a SAD table
     // search capacity per kind of launch (search_multi_kind)
     int cap[SEARCH_KINDS] = {}, sthreads[SEARCH_KINDS] = {};
     size_t ssmem[SEARCH_KINDS] = {};
@@ -3084,7 +3085,46 @@ struct riv_batch {
 
 namespace {
 
-static int search_variant(const riv_encoder* e, bool table) { return search_multi_kind(table && e->table_ok, e->small_costs); }
+// The clip's kind of search in a step: from its SAD table (where it has one and the step's shapes
+// say so), or the kind riv_batch_new chose for it.
+static int search_variant(const riv_encoder* e, bool table) {
+    return table && e->table_ok ? search_multi_kind(true, e->small_costs, 0) : e->multi_kind;
+}
+
+// Each clip's kind without a table, and the launch of every kind that some clip uses, sized by the largest
+// search range among those clips.  A step may hold a frame of every clip, so each kind's CTAs must be
+// at least as many as its clips.  A ring of windows leaves two CTAs an SM up to a search range of 63
+// and one above; where that is too few (more than 148 clips) the clips of the widest ranges search with
+// the plain kind, two CTAs an SM at any range.
+static void batch_search_kinds(riv_batch* b, int nsm) {
+    auto size_kind = [&](int v, bool table) {  // how many clips use it
+        int n = 0, sr = -1;
+        for (const riv_encoder* e : b->clips) {
+            if (search_variant(e, table) != v) continue;
+            n++;
+            sr = std::max(sr, (int)e->cfg.search_range);
+        }
+        b->cap[v] = 0;
+        if (n == 0) return n;
+        int per_sm = 0;
+        CK(search_multi_capacity(v, sr, &per_sm, &b->ssmem[v], &b->sthreads[v]));
+        b->cap[v] = per_sm * nsm;
+        return n;
+    };
+    for (riv_encoder* e : b->clips) e->multi_kind = search_multi_kind(false, e->small_costs, e->cfg.search_range);
+    const int direct = search_multi_kind(false, true, 0), plain = search_multi_kind(false, false, 0);
+    while (size_kind(direct, false) > b->cap[direct]) {
+        int sr = 0;
+        for (const riv_encoder* e : b->clips)
+            if (e->multi_kind == direct) sr = std::max(sr, (int)e->cfg.search_range);
+        for (riv_encoder* e : b->clips)
+            if (e->multi_kind == direct && e->cfg.search_range == sr) e->multi_kind = plain;
+    }
+    size_kind(plain, false);
+    for (int small = 0; small < 2; small++) size_kind(search_multi_kind(true, small != 0, 0), true);
+    for (const riv_encoder* e : b->clips)
+        if (e->table_ok) b->table_sr = std::max(b->table_sr, (int)e->cfg.search_range);
+}
 
 // Row CTAs of each clip of one search launch: about proportional to its MBs, at least one, at
 // most its MB rows, `total` in all (>= the number of clips).
@@ -3433,11 +3473,11 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
             if (timed) CK(cudaEventRecord(evt[k], B));
         };
         auto stage = [&](int s, int tb) {
-            CK(launch_batch_stage(s, L, t, tot[s], b->max_sr, B));
+            CK(launch_batch_stage(s, L, t, tot[s], b->table_sr, B));
             if (tot[s] > 0) b->launches += s == BS_SCAN ? 2 : s == BS_PACK ? 3 : 1;
             mark(tb);
         };
-        CK(launch_batch_stage(BS_CONVERT, L, t, tot[BS_CONVERT], b->max_sr, b->V));
+        CK(launch_batch_stage(BS_CONVERT, L, t, tot[BS_CONVERT], b->table_sr, b->V));
         if (tot[BS_CONVERT] > 0) b->launches++;
         CK(cudaEventRecord(b->ev_conv, b->V));
         mark(TB_START);
@@ -3573,7 +3613,6 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
             e->mv_submit = [mp](std::function<void()> f) { return mp->submit(std::move(f)); };
             e->rans_parts = (int)std::max(2u, hw / 2) + 1;
             b->clips.push_back(e);
-            b->max_sr = std::max(b->max_sr, (int)c.search_range);
             maxcap = std::max(maxcap, e->slots.size());
         }
         CK(cudaStreamCreateWithFlags(&b->B, cudaStreamNonBlocking));
@@ -3606,11 +3645,7 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
         int dev = 0, nsm = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        for (int v = 0; v < SEARCH_KINDS; v++) {
-            int per_sm = 0;
-            CK(search_multi_capacity(v, b->max_sr, &per_sm, &b->ssmem[v], &b->sthreads[v]));
-            b->cap[v] = per_sm * nsm;
-        }
+        batch_search_kinds(b, nsm);
         CK(cudaStreamSynchronize(b->B));
     } catch (const CudaError& ce) {
         fprintf(stderr, "riv_batch_new: %s: %s\n", ce.where, cudaGetErrorString(ce.e));

@@ -203,11 +203,12 @@ struct BatchLaunch {
 int batch_ctas_host(int stage, const BatchClip& k, const BatchTune& t);
 // The rANS streams and side info of a step's clips (caps: the largest SymFrame::cap and nside).
 int launch_batch_rans(const BatchClip* clips, int nclips, unsigned max_cap, int max_nside, void* stream);
-int launch_batch_stage(int stage, const BatchLaunch& b, const BatchTune& t, int total_ctas, int max_sr, void* stream);
+// table_sr: the largest search range among the clips that have a SAD table.
+int launch_batch_stage(int stage, const BatchLaunch& b, const BatchTune& t, int total_ctas, int table_sr, void* stream);
 // Kinds of multi-clip search launches: 64- or 32-bit costs, with an exhaustive SAD table or with
 // the SADs computed on the way.
 constexpr int SEARCH_KINDS = 4;
-int search_multi_kind(bool table, bool small);
+int search_multi_kind(bool table, bool small, int sr);  // of a clip
 bool search_multi_predicts(int kind);  // its launch makes the luma prediction and the ln variances
 int search_multi_capacity(int kind, int max_sr, int* per_sm, size_t* smem, int* threads);
 int launch_search_multi(const SearchParams* dparams, const int* dstart, int nclips, int total_ctas, int kind, size_t smem,

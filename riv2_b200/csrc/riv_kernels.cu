@@ -383,11 +383,7 @@ size_t sad_table_smem(int sr) {
 int launch_sad_table(const uint8_t* ref, const uint8_t* cur, int W, int H, int sr, uint16_t* tab, int tstride,
                      void* stream) {
     int BW = W / 16, n = BW * (H / 16);
-    size_t sm = sad_table_smem(sr);
-    if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_sad_table, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return (int)e;
-    }
+    size_t sm = sad_table_smem(sr);  // 3.2 KB at the largest range that has a table
     k_sad_table<<<n, 128, sm, (cudaStream_t)stream>>>(ref, cur, W, H, BW, sr, tab, tstride);
     return (int)cudaGetLastError();
 }

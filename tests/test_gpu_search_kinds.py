@@ -71,3 +71,24 @@ def test_band_kept(w, h, sr):
     from riv2_b200 import encoder as E
     p = E.search_plan(w, h, sr)
     assert p["band"] and p["loader"] and not p["table"]
+
+
+@pytest.mark.parametrize("table", [0, 1])
+@pytest.mark.parametrize("clips", [[(352, 64, 101), (64, 64, 12)], [(352, 64, 102), (64, 64, 12), (48, 32, 31)], [(64, 64, 127)],
+                                   [(16, 16, 64)] * 149, [(16, 16, 64)] * 147 + [(32, 32, 16)] * 10])
+def test_batch_of_wide_ranges(clips, table):
+    """Ranges beyond a ring of four windows (101), and more clips than such rings fit the GPU at once
+    (148 from a range of 64 on)."""
+    from riv2_b200 import encoder as E
+    from riv2_b200.batch import Batch
+    cfgs = {c: _configs(*c, 2) for c in set(clips)}
+    frames = {c: _frames(c[0], c[1], 3, sum(c)) for c in cfgs}
+    writers = [E.VecWriter() for _ in clips]
+    b = Batch.new([cfgs[c][0] for c in clips], writers)
+    b.set_tune(100, 4, 128, table)
+    for t in range(3):
+        b.encode_step([frames[c][t] for c in clips], [20 * t] * len(clips))
+    b.finish()
+    b.close()
+    want = {c: _oracle(cfgs[c][1], frames[c]) for c in cfgs}
+    assert all(w.into_inner() == want[c] for w, c in zip(writers, clips))

@@ -166,7 +166,7 @@ int launch_batch_rans(const BatchClip* clips, int nclips, unsigned max_cap, int 
 template <bool TABLE, bool SMALL>
 __global__ void __maxnreg__(96) k_search_multi(const SearchParams* __restrict__ ps, const int* __restrict__ start,
                                                 int nclips) {
-    search_body<false, TABLE, SMALL, false>(ps[batch_clip(start, nclips, blockIdx.x)]);
+    search_body<false, TABLE, SMALL, true>(ps[batch_clip(start, nclips, blockIdx.x)]);
 }
 
 static const void* search_multi_fn(SearchKind k) {

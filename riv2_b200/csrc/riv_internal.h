@@ -82,7 +82,6 @@ struct SearchParams {
     long long* prof;  // optional: RIV_PROF_WORDS words per MB (phase stamps, hexagon rounds), nullptr = off
     int nrow_ctas;    // CTAs that own MB rows (row stride); the rest of the grid are table workers
     int cta0;         // first CTA of this clip in a multi-clip launch (0 for a single clip)
-    int fused;        // the grid's CTAs beyond the row CTAs are workers
     int row_helpers;  // row CTAs run worker groups before their row starts and after it ends
     unsigned* tflag;  // fused table: per-MB flag = tag once its table row is written; nullptr = precomputed
     // Prediction and AQ inside the search launch (band + table instantiations): nullptr lnv =
@@ -222,9 +221,9 @@ enum StatusBits : unsigned {
 // Launchers (riv_kernels.cu).  All are asynchronous on `stream`.
 int launch_rgb_to_yuv(const uint8_t* rgb, int dw, int dh, uint8_t* yuv, int W, int H, void* stream, bool beside = false);
 int launch_yuv_to_rgb(const uint8_t* yuv, int W, int H, int dw, int dh, uint8_t* rgb, void* stream);
-// Launch plan of the search wavefront (chosen once per encoder).  fused: the SAD table (if any) and
-// the previous frame's reconstruction are worked on inside the same cooperative launch by
-// `grid - nrow` worker CTAs.
+// Launch plan of the search wavefront (chosen once per encoder).  fused: the SAD table and the
+// previous frame's reconstruction are worked on inside the same cooperative launch by `grid - nrow`
+// worker CTAs.
 struct SearchPlan {
     const void* fn;
     bool fast;   // loader and AQ warps (prediction and AQ in the launch)

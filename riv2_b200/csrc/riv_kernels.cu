@@ -1524,12 +1524,11 @@ __device__ __forceinline__ bool wait_at_least(const unsigned* c, unsigned target
     return true;
 }
 // The rows / bands MB row r depends on before its reference samples may be read: the
-// previous frame's deblocked bands (or its residual rows when it has no deblock) that its search
-// window of sr + 1 rows above and below touches, r-1 .. r+1 up to a search range of 15.
+// previous frame's deblocked bands r-1 .. r+1 (or its residual rows when it has no deblock), which
+// hold its search window of sr + 1 rows above and below: fused launches have a table, sr <= 15.
 __device__ __forceinline__ bool wait_ref_rows(const SearchParams& p, int r, int tiles_per_band) {
     if (!p.defer) return true;
-    const int k = (p.sr + 16) >> 4;
-    for (int b = max(r - k, 0); b <= min(r + k, p.BH - 1); b++) {
+    for (int b = max(r - 1, 0); b <= min(r + 1, p.BH - 1); b++) {
         const bool ok = p.db_level > 0 ? wait_at_least(p.wq + 1 + p.BH + b, (unsigned)tiles_per_band, p.spin_limit)
                                        : wait_at_least(p.wq + 1 + b, (unsigned)p.BW, p.spin_limit);
         if (!ok) return false;
@@ -2241,20 +2240,21 @@ __device__ __forceinline__ void sad_parts(const RefView& v, int org, bool inside
     }
 }
 
-// Where several row CTAs share an SM their waiting mode and AQ warps look less often.
+// Where several row CTAs share an SM (MULTI) their waiting mode and AQ warps look less often.
 constexpr unsigned SEARCH_NAP = 250;
-// WORKERS: the launch may be fused (worker CTAs, helper groups of the row CTAs).
-template <bool BAND, bool TABLE, bool SMALL, bool WORKERS>
+template <bool BAND, bool TABLE, bool SMALL, bool MULTI>
 __device__ __forceinline__ void search_body(const SearchParams& p) {
     // FAST (DIRECT, or band and table): search chain, mode decision, loader and AQ warps.  Otherwise
     // the search warp stages its own data with cp.async and only the mode warp runs beside it.  RING:
-    // the loader brings each MB's window instead of the row's band.  DIRECT (32-bit costs, no table): the integer SADs are computed on the chain, four
-    // positions at a time (8 lanes each).  1080p at search range 31: 0.78 ms a frame with the
-    // previous frame's reconstruction in the launch, where one position at a time on 64-bit costs,
-    // its prediction, AQ, residual and deblock in kernels of their own, took 1.60 ms.
+    // the loader brings each MB's window instead of the row's band.  DIRECT (32-bit costs, no table):
+    // the integer SADs are computed on the chain, four positions at a time (8 lanes each).  1080p at
+    // search range 31: 0.78 ms a frame, where one position at a time on 64-bit costs, with prediction
+    // and AQ in kernels of their own, took 1.60 ms.  WORKERS: the launch may be fused (worker CTAs,
+    // helper groups of the row CTAs).
     constexpr bool DIRECT = SMALL && !TABLE, FAST = (BAND && TABLE) || DIRECT, RING = DIRECT && !BAND;
+    constexpr bool WORKERS = BAND && TABLE && !MULTI;
     extern __shared__ __align__(16) uint8_t smem[];
-    if (FAST && WORKERS && p.fused && row_cta(p) >= p.nrow_ctas) {
+    if (WORKERS && p.tflag != nullptr && row_cta(p) >= p.nrow_ctas) {
         frame_worker(p, smem);
         return;
     }
@@ -2290,7 +2290,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     // Fused launch: threads 128-511 of a row CTA are worker groups 1-3 until the row starts
     // (region after the row layout: a live flag, then a 3-group worker region), and the
     // whole CTA joins the worker queue once its rows are done.
-    const bool helpers = FAST && WORKERS && p.fused && p.row_helpers;
+    const bool helpers = WORKERS && p.tflag != nullptr && p.row_helpers;
     uint8_t* pre = smem + (((size_t)(refmem - smem) + (RING ? 0 : (size_t)WS * BWB + 16) + 15) & ~(size_t)15);
     volatile int* row_live = (volatile int*)pre;
     uint8_t* preg = pre + 16;
@@ -2308,14 +2308,14 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     }
     __syncthreads();
     const unsigned long long tagbits = (unsigned long long)(p.tag & 0xffffu) << 48;
-    const unsigned nap = WORKERS ? 0u : SEARCH_NAP;
+    const unsigned nap = MULTI ? SEARCH_NAP : 0u;
     // The role of this warp: search, mode, loader, AQ.  A warp's scheduler is its index modulo 4, so
     // where several CTAs share an SM the roles rotate from CTA to CTA (CTAs 148 apart share an SM
     // when the grid is larger): with the search warp first in each, one scheduler had all the chains
     // (24 mixed clips, five CTAs an SM: 2.21 ms a step, 1.66 rotated; 1.95 for search and prediction
     // without loader and AQ warps).
     const int warp = (int)(threadIdx.x >> 5);
-    const int role = FAST && !WORKERS ? (warp + (int)(blockIdx.x / 148u)) & 3 : warp;
+    const int role = FAST && MULTI ? (warp + (int)(blockIdx.x / 148u)) & 3 : warp;
     auto roles = [&]() {
     if (role >= 2) {
         if (FAST && role == 2) {
@@ -3050,7 +3050,7 @@ __global__ void __maxnreg__(120) k_search(SearchParams p) {
     if (tl != nullptr && threadIdx.x == 0) atomicCAS(tl, 0ull, (unsigned long long)gtimer());
     if (p.wq_next != nullptr && blockIdx.x == gridDim.x - 1)  // the next launch's queue words
         for (int i = threadIdx.x; i < p.wq_words; i += blockDim.x) p.wq_next[i] = 0u;
-    search_body<BAND, TABLE, SMALL, true>(p);
+    search_body<BAND, TABLE, SMALL, false>(p);
     if (tl != nullptr && (threadIdx.x & 31) == 0) atomicMax(tl + 1, (unsigned long long)gtimer());
 }
 
@@ -3059,9 +3059,6 @@ __global__ void __maxnreg__(120) k_search(SearchParams p) {
 // on the chain (32-bit costs).
 int sad_table_stride(int sr) { return ((2 * sr + 1) * (2 * sr + 1) + 7) & ~7; }
 bool search_use_table(int sr) { return sr <= 15; }
-// A fused launch without a table needs fewer CTAs beside the rows: the row CTAs' spare warps take
-// worker tasks too until their row starts (frames of 2160 pixel rows leave 13).
-constexpr int SEARCH_DIRECT_WORKERS = 8;
 enum SearchKind { SK_TABLE_SMALL, SK_TABLE, SK_DIRECT, SK_PLAIN };  // PLAIN: 64-bit costs, no table
 static bool search_fast(bool band, SearchKind k) { return k == SK_DIRECT || (band && k != SK_PLAIN); }
 static size_t search_smem(int sr, int W, bool band, SearchKind k) {
@@ -3128,9 +3125,12 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         return r;
     };
     auto use_band = [&](SearchKind k) { return search_band(sr, W, k); };
-    // The plan of one kind: fused when it can be, else one CTA per MB row (as many as fit).
-    // fused: one CTA per SM (the shared-memory request rules out a second), rows first, workers on
-    // the SMs the rows leave free; a table's MBs need at least 32 of those.
+    // The plan of one kind: fused when it has a table and can be, else one CTA per MB row (as many as
+    // fit).  fused: one CTA per SM (the shared-memory request rules out a second), rows first, workers
+    // on the SMs the rows leave free; a table's MBs need at least 32 of those.  The direct kind is not:
+    // a fused launch's frames took as long (range 31, 8 in flight: 0.79 ms at 1080p, 0.78 unfused;
+    // 0.27 and 0.28 at 640x360; 1.76 and 1.64 at 4K) and its 148 CTAs keep every other encoder off the
+    // GPU (four of 640x360: 0.25 ms a frame, 0.12 unfused; three of 1080p: 0.80 and 0.41).
     auto plan = [&](SearchKind k, SearchPlan& pl) -> cudaError_t {
         const bool band = use_band(k), tab = k == SK_TABLE_SMALL || k == SK_TABLE;
         const size_t sm = search_smem(sr, W, band, k);
@@ -3141,7 +3141,7 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         pl.table = tab;
         pl.band = band;
         int per_sm = 0;
-        if (pl.fast) {
+        if (pl.fast && tab) {
             // row CTAs' helper region (live flag + three worker groups) after the row layout,
             // where the per-CTA maximum allows it
             const size_t with_helpers = ((sm + 15) & ~(size_t)15) + 16 + (size_t)worker_region_bytes(3);
@@ -3152,8 +3152,8 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
             if (r != cudaSuccess) return r;
             const int total = per_sm * nsm;
             const int nrow = BH < total ? BH : total;
-            const size_t gsm = tab ? ((size_t)sad_table_smem(sr) + 15) & ~(size_t)15 : 0;
-            if (per_sm == 1 && total - nrow >= (tab ? 32 : SEARCH_DIRECT_WORKERS) && 4 * gsm <= smf) {
+            const size_t gsm = ((size_t)sad_table_smem(sr) + 15) & ~(size_t)15;
+            if (per_sm == 1 && total - nrow >= 32 && 4 * gsm <= smf) {
                 pl.fused = true;
                 pl.helpers = helpers;
                 pl.threads = 4 * 128;  // row CTAs use four warps; workers four groups of 128
@@ -3170,9 +3170,9 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
         pl.grid = pl.nrow = BH < per_sm * nsm ? BH : per_sm * nsm;
         return cudaSuccess;
     };
-    // A table wherever there is one: its chain is shorter (at 2160 rows a table kernel, the search,
-    // the residual and the deblock take 1.57 ms a frame, a fused direct launch 1.84-1.94 ms; at 1080
-    // rows 0.55 ms against 0.79-0.87).
+    // A table wherever there is one: its chain is shorter.  Range 12, 8 frames in flight, ms a frame with
+    // a table and without: 0.64 and 0.88 at 1080p (fused), 0.91 and 1.15 at 1920x1904 (29 SMs left: not
+    // fused), 1.65 and 2.04 at 3840x2160.
     const SearchKind untabled = untabled_kind(sr, W, use_band(SK_DIRECT), small);
     return (int)plan(table ? (small ? SK_TABLE_SMALL : SK_TABLE) : untabled, *out);
 }
@@ -3180,7 +3180,6 @@ int search_plan(int sr, int W, int BH, bool table, bool small, SearchPlan* out) 
 int launch_search(const SearchParams& p, const SearchPlan& plan, void* stream) {
     SearchParams q = p;
     q.nrow_ctas = plan.nrow;
-    q.fused = plan.fused ? 1 : 0;
     q.row_helpers = plan.fused && plan.helpers ? 1 : 0;
     if (!plan.fused) q.tflag = nullptr;
     void* args[] = {&q};

@@ -92,3 +92,39 @@ def test_batch_of_wide_ranges(clips, table):
     b.close()
     want = {c: _oracle(cfgs[c][1], frames[c]) for c in cfgs}
     assert all(w.into_inner() == want[c] for w, c in zip(writers, clips))
+
+
+@pytest.mark.parametrize("w,h", [(16, 16), (640, 368), (1920, 1088), (3840, 2160)])
+@pytest.mark.parametrize("sr", [16, 31, 63])
+def test_direct_launch_leaves_the_gpu_to_others(w, h, sr):
+    """Without a table a launch has the CTAs of its macroblock rows and no others."""
+    from riv2_b200 import encoder as E
+    p = E.search_plan(w, h, sr)
+    assert not p["fused"] and p["ctas"] == p["row_ctas"] <= h // 16
+
+
+@pytest.mark.parametrize("sr", [12, 16, 31])
+def test_encoders_side_by_side(sr):
+    """Four encoders of different sizes, each on a thread of its own, depth 0 and frames in flight."""
+    import threading
+
+    from riv2_b200 import encoder as E
+    runs = []
+    for k, (w, h) in enumerate([(352, 288), (96, 64), (640, 368), (208, 112)]):
+        gc, oc = _configs(w, h, sr, 4 * (k % 2))
+        wr = E.VecWriter()
+        runs.append((E.Encoder.new(gc, wr), wr, oc, _frames(w, h, 5, w + sr)))
+
+    def work(enc, oc, frames):
+        for t, f in enumerate(frames):
+            enc.encode_frame(E.Frame(f, oc.display_width, oc.display_height, 20 * t))
+        enc.finish()
+
+    threads = [threading.Thread(target=work, args=(enc, oc, f)) for enc, _, oc, f in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for enc, wr, oc, f in runs:
+        enc.close()
+        assert wr.into_inner() == _oracle(oc, f)

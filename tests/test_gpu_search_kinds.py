@@ -128,3 +128,42 @@ def test_encoders_side_by_side(sr):
     for enc, wr, oc, f in runs:
         enc.close()
         assert wr.into_inner() == _oracle(oc, f)
+
+
+def test_learned_encoders_side_by_side():
+    """Four encoders of the learned form on threads of their own write what one alone writes (their
+    products are of different widths, launched by the threads at the same time)."""
+    import os
+    import threading
+
+    import riv2_b200
+    from riv2_b200 import encoder as E
+    from riv2_b200 import proposal as P
+    params = P.load_params(os.path.join(os.path.dirname(riv2_b200.__file__), "weights", "proposal.bin"))
+    frames = _frames(352, 288, 24, 7)
+
+    def start():
+        gc = _configs(352, 288, 12, 4)[0].with_encode_form(1)
+        wr = E.VecWriter()
+        enc = E.Encoder.new(gc, wr)
+        enc.set_proposal(params)
+        return enc, wr
+
+    def work(enc):
+        for t, f in enumerate(frames):
+            enc.encode_frame(E.Frame(f, 352, 288, 20 * t))
+        enc.finish()
+
+    alone, alone_wr = start()
+    work(alone)
+    alone.close()
+    runs = [start() for _ in range(4)]
+    threads = [threading.Thread(target=work, args=(enc,)) for enc, _ in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    want = alone_wr.into_inner()
+    for enc, wr in runs:
+        enc.close()
+        assert wr.into_inner() == want

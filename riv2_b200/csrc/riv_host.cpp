@@ -3028,7 +3028,7 @@ constexpr int BT_BOUNDS = BS_N + 3;  // timing marks: start, then one after each
 enum { TB_START, TB_CONVERT, TB_TABLE, TB_SEARCH, TB_PREDICT, TB_AQSUM, TB_RESIDUAL, TB_DEBLOCK, TB_SCAN, TB_PACK };
 constexpr int BT_NSTAGE = 9;  // convert, table, search, predict, aq mean, residual, deblock, scan, pack
 // Autotuner candidates (one dimension per timed stage; the streams do not depend on them).
-// The search has six candidates (CTA share x SAD table or not, timed as table + search stages),
+// The search has six candidates (CTA share x SAD table or not, timed as table, search and prediction),
 // the residual and the deblock three each (cycled twice as often).
 constexpr int TUNE_NCAND = 6;
 constexpr int TUNE_ROWS_PCT[TUNE_NCAND] = {100, 75, 50, 100, 75, 50};
@@ -3271,6 +3271,14 @@ static BatchTune batch_step_tune(riv_batch* b, bool& tuning, int& cand) {
     return t;
 }
 
+// The stage times that decide one dimension of the shapes (0 search, 1 residual, 2 deblock); ms: the
+// times between the TB_ marks.  A search from tables needs them made first and the prediction after,
+// which the direct kind makes on the way.
+static float tune_score(int dim, const float* ms) {
+    if (dim == 0) return ms[TB_TABLE - 1] + ms[TB_SEARCH - 1] + ms[TB_PREDICT - 1];
+    return dim == 1 ? ms[TB_RESIDUAL - 1] : ms[TB_DEBLOCK - 1];
+}
+
 // Stage times of the timed step held by timing set `par` (if any): accumulated, and fed to the
 // autotuner when that step ran candidate shapes.  Waits for that step's work to end.
 static void batch_read_times(riv_batch* b, int par) {
@@ -3287,9 +3295,9 @@ static void batch_read_times(riv_batch* b, int par) {
     if (!t.tuning || b->tuned || b->fixed) return;
     if (t.pmbs == t.mbs && t.pmbs > 0) {  // P-frames only: comparable steps
         const int c3 = t.cand % 3;
-        b->tune_us[0][t.cand] += 1000.0 * (ms[1] + ms[2]) / (double)t.pmbs;  // SAD table + search
-        b->tune_us[1][c3] += 1000.0 * ms[5] / (double)t.mbs;                 // residual
-        b->tune_us[2][c3] += 1000.0 * ms[6] / (double)t.mbs;                 // deblock
+        b->tune_us[0][t.cand] += 1000.0 * tune_score(0, ms) / (double)t.pmbs;
+        b->tune_us[1][c3] += 1000.0 * tune_score(1, ms) / (double)t.mbs;
+        b->tune_us[2][c3] += 1000.0 * tune_score(2, ms) / (double)t.mbs;
         b->tune_n[0][t.cand]++;
         b->tune_n[1][c3]++;
         b->tune_n[2][c3]++;
@@ -3769,6 +3777,12 @@ riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us
     }
     if (stage_us10)
         for (int s = 0; s <= BT_NSTAGE; s++) stage_us10[s] = b->timed ? b->stage_us[s] / (double)b->timed : 0.0;
+    return RIV_OK;
+}
+
+riv_status riv_test_batch_tune_score(int dim, const float* stage9, float* score) {
+    if (dim < 0 || dim > 2 || !stage9 || !score) return RIV_ERR_INVALID_CONFIG;
+    *score = tune_score(dim, stage9);
     return RIV_OK;
 }
 

@@ -140,7 +140,7 @@ def test_learned_encoders_side_by_side():
     from riv2_b200 import encoder as E
     from riv2_b200 import proposal as P
     params = P.load_params(os.path.join(os.path.dirname(riv2_b200.__file__), "weights", "proposal.bin"))
-    frames = _frames(352, 288, 24, 7)
+    frames = _frames(352, 288, 12, 7) * 2
 
     def start():
         gc = _configs(352, 288, 12, 4)[0].with_encode_form(1)

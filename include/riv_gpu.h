@@ -203,10 +203,11 @@ riv_status riv_batch_set_tune(riv_batch* b, const riv_batch_tune* t);
 /* The shapes in use; *tuned = 0 still tuning, 1 chosen by the autotuner, 2 fixed. */
 riv_status riv_batch_get_tune(const riv_batch* b, riv_batch_tune* t, int* tuned);
 /* c7 = {steps, frames, MBs, kernel launches, timed steps, host->device bytes, device->host
- * bytes}; stage_us10 = mean GPU microseconds per timed step: waiting for the conversion (which
- * runs beside the step before), SAD tables, search,
- * prediction, AQ mean, residual, deblock, symbol counts, symbols and models, whole step (the rANS
- * batches run beside the next step and are not in it).  Either may be NULL. */
+ * bytes}; stage_us10 = mean GPU microseconds per timed step: conversion, SAD tables, search,
+ * prediction, AQ mean, residual, deblock, symbol counts, symbols and models, whole step.  The
+ * conversion runs beside the step before, so the whole step, from the end of that one, holds only
+ * what is left of it; the rANS batches run beside the next step and are in none.  Either may be
+ * NULL. */
 riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us10);
 /* Cumulative host milliseconds: [0] waiting for a clip's earlier records before its next
  * frame (pipeline full), [1] descriptors and launches, [2] copies back and bookkeeping,

@@ -22,6 +22,7 @@ import numpy as np
 from . import encoder as E
 
 U8P = C.POINTER(C.c_uint8)
+# of riv_batch_counters: "scan" is the symbol counts, "pack" the symbols and models
 STAGES = ["convert", "sad_table", "search", "predict", "aq_mean", "residual", "deblock", "scan", "pack", "step"]
 
 

@@ -3049,6 +3049,7 @@ struct riv_batch {
     // stage timing marks of timed steps, two sets: a step's marks are read one timed step later
     // (or at the end), so that reading them rarely waits for the GPU
     cudaEvent_t ev_t[2][BT_BOUNDS] = {};
+    cudaEvent_t ev_tc[2][2] = {};  // around the conversion, on its own stream
     struct TimedStep {
         bool pending = false, tuning = false;
         int cand = 0;
@@ -3288,7 +3289,8 @@ static void batch_read_times(riv_batch* b, int par) {
     cudaEvent_t* ev = b->ev_t[par];
     CK(cudaEventSynchronize(ev[TB_PACK]));
     float ms[BT_NSTAGE + 1] = {0};
-    for (int s = 0; s < BT_NSTAGE; s++) CK(cudaEventElapsedTime(&ms[s], ev[s], ev[s + 1]));
+    for (int s = 1; s < BT_NSTAGE; s++) CK(cudaEventElapsedTime(&ms[s], ev[s], ev[s + 1]));
+    CK(cudaEventElapsedTime(&ms[0], b->ev_tc[par][0], b->ev_tc[par][1]));
     CK(cudaEventElapsedTime(&ms[BT_NSTAGE], ev[TB_START], ev[TB_PACK]));
     for (int s = 0; s <= BT_NSTAGE; s++) b->stage_us[s] += 1000.0 * ms[s];
     b->timed++;
@@ -3485,8 +3487,10 @@ static riv_status batch_step(riv_batch* b, int src, const void* const* frames, c
             if (tot[s] > 0) b->launches += s == BS_SCAN ? 2 : s == BS_PACK ? 3 : 1;
             mark(tb);
         };
+        if (timed) CK(cudaEventRecord(b->ev_tc[b->tpar][0], b->V));
         CK(launch_batch_stage(BS_CONVERT, L, t, tot[BS_CONVERT], b->table_sr, b->V));
         if (tot[BS_CONVERT] > 0) b->launches++;
+        if (timed) CK(cudaEventRecord(b->ev_tc[b->tpar][1], b->V));
         CK(cudaEventRecord(b->ev_conv, b->V));
         mark(TB_START);
         CK(cudaStreamWaitEvent(B, b->ev_conv, 0));
@@ -3634,6 +3638,8 @@ riv_status riv_batch_new(const riv_config* cfgs, const riv_writer_vtable* writer
         for (auto& ev : b->ev_step) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         for (int q = 0; q < 2; q++)
             for (int k = 0; k < BT_BOUNDS; k++) CK(cudaEventCreate(&b->ev_t[q][k]));
+        for (int q = 0; q < 2; q++)
+            for (int k = 0; k < 2; k++) CK(cudaEventCreate(&b->ev_tc[q][k]));
         for (int k = 0; k < 2; k++) {
             CK(cudaEventCreateWithFlags(&b->ev_desc[k], cudaEventDisableTiming));
             CK(cudaEventRecord(b->ev_desc[k], b->B));
@@ -3722,6 +3728,9 @@ void riv_batch_free(riv_batch* b) {
     for (int q = 0; q < 2; q++)
         for (int k = 0; k < BT_BOUNDS; k++)
             if (b->ev_t[q][k]) cudaEventDestroy(b->ev_t[q][k]);
+    for (int q = 0; q < 2; q++)
+        for (int k = 0; k < 2; k++)
+            if (b->ev_tc[q][k]) cudaEventDestroy(b->ev_tc[q][k]);
     for (int k = 0; k < 2; k++) {
         if (b->ev_desc[k]) cudaEventDestroy(b->ev_desc[k]);
         if (b->ev_ddesc[k]) cudaEventDestroy(b->ev_ddesc[k]);

@@ -2531,10 +2531,10 @@ riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_
     for (size_t k = 0; k < n; k++) st[k / SYM_BATCH * SYM_BATCH + (SYM_BATCH - 1 - k % SYM_BATCH)] = symbols[k];
     std::vector<uint8_t> stream;
     struct Bufs {
-        DevBuf stack, info, side;
+        DevBuf stack, info, side, clip;
         MappedBuf out;
         ~Bufs() {
-            for (DevBuf* b : {&stack, &info, &side}) b->release();
+            for (DevBuf* b : {&stack, &info, &side, &clip}) b->release();
             out.release();
         }
     } B;
@@ -2564,7 +2564,11 @@ riv_status riv_test_rans(const uint16_t* symbols, uint32_t n, int on_gpu, uint8_
             f.out_cap = (unsigned)bytes;
             f.out_bytes = B.out.dev<uint32_t>() + bytes / 4;
             f.side_out = f.out_bytes + 4;
-            CK(launch_rans(f, std::max(room, 1u), nullptr));
+            BatchClip k{};  // as a step of one clip
+            k.rans = f;
+            B.clip.alloc(sizeof(k));
+            CK(cudaMemcpy(B.clip.p, &k, sizeof(k), cudaMemcpyHostToDevice));
+            CK(launch_batch_rans(B.clip.as<BatchClip>(), 1, std::max(room, 1u), f.nside, nullptr));
             CK(cudaDeviceSynchronize());
             const uint8_t* h = B.out.host<uint8_t>();
             const uint32_t got = *(const uint32_t*)(h + bytes);

@@ -261,7 +261,6 @@ int deblock_scratch_address(void** out);
 int launch_symbols(const SymFrame& f, void* stream);
 // Bytes of a frame's cnt, tot, occ, ustate and work; with f, lays them out at p (256-byte aligned).
 size_t sym_workspace(SymFrame* f, int nmb, unsigned cap, void* p);
-int launch_rans(const RansFrame& f, unsigned cap, void* stream);
 size_t rans_info_bytes(unsigned cap);  // of RansFrame::info
 size_t rans_max_bytes(unsigned cap);   // the longest stream of cap symbols
 // libm device helpers exposed for the exhaustive check

@@ -185,18 +185,9 @@ __device__ __forceinline__ void rans_gather_cta(const RansFrame& f, int cta, int
     }
 }
 
-__global__ void __launch_bounds__(32 * RA_WARPS) k_rans(RansFrame f) { rans_cta(f, blockIdx.x); }
-__global__ void __launch_bounds__(RA_GATHER) k_rans_gather(RansFrame f, int side_ctas) { rans_gather_cta(f, blockIdx.x, side_ctas); }
-
 static inline int rans_batches(unsigned cap) { return (int)((cap + SYM_BATCH - 1u) / SYM_BATCH); }
 static inline int rans_side_ctas(int nside) { return (nside + RA_SIDE - 1) / RA_SIDE; }
 size_t rans_info_bytes(unsigned cap) { return (size_t)(1 + rans_batches(cap)) * sizeof(uint4); }
 // A symbol grows its state by 8 bits and log2(1 + 1 / 256) at most (a state is 2^8 f or more when its
 // symbol of frequency f is coded).
 size_t rans_max_bytes(unsigned cap) { return (size_t)cap + cap / 512 + 16 * (size_t)rans_batches(cap); }
-int launch_rans(const RansFrame& f, unsigned cap, void* stream) {
-    const int nb = rans_batches(cap), ns = rans_side_ctas(f.nside);
-    k_rans<<<(nb + RA_WARPS - 1) / RA_WARPS, 32 * RA_WARPS, 0, (cudaStream_t)stream>>>(f);
-    k_rans_gather<<<nb + ns, RA_GATHER, 0, (cudaStream_t)stream>>>(f, ns);
-    return (int)cudaGetLastError();
-}

@@ -136,11 +136,15 @@ def test_learned_encoders_side_by_side():
     import os
     import threading
 
+    import numpy as np
+    import torch
+
     import riv2_b200
     from riv2_b200 import encoder as E
     from riv2_b200 import proposal as P
     params = P.load_params(os.path.join(os.path.dirname(riv2_b200.__file__), "weights", "proposal.bin"))
-    frames = _frames(352, 288, 12, 7) * 2
+    frames = torch.from_numpy(np.stack(_frames(352, 288, 8, 7))).cuda()
+    torch.cuda.synchronize()
 
     def start():
         gc = _configs(352, 288, 12, 4)[0].with_encode_form(1)
@@ -150,8 +154,8 @@ def test_learned_encoders_side_by_side():
         return enc, wr
 
     def work(enc):
-        for t, f in enumerate(frames):
-            enc.encode_frame(E.Frame(f, 352, 288, 20 * t))
+        for t in range(160):
+            enc.encode_frame_device(frames[t % 8].data_ptr(), 20 * t)
         enc.finish()
 
     alone, alone_wr = start()
@@ -167,3 +171,45 @@ def test_learned_encoders_side_by_side():
     for enc, wr in runs:
         enc.close()
         assert wr.into_inner() == want
+
+
+# 64-bit costs, with a table (ranges up to 15) and without, each with a band and (3856 columns) a window:
+# the usual weight with the 32-bit kinds switched off, weights whose costs pass 2^27 and 2^58 (no table),
+# and a negative one (no table either)
+WEIGHTS = [("0", 0.49), ("1", 1e7), ("1", 1e17), ("1", -0.49)]
+
+
+def _weighted(w, h, sr, depth, weight):
+    gc, oc = _configs(w, h, sr, depth)
+    oc.rdo_lambda_mult = weight
+    return gc.with_rdo_lambda_mult(weight), oc
+
+
+@pytest.mark.parametrize("small,weight", WEIGHTS)
+@pytest.mark.parametrize("w,h,sr", [(352, 288, 12), (3856, 32, 15), (352, 288, 31), (3856, 32, 31)])
+@pytest.mark.parametrize("depth", [0, 4])
+def test_wide_costs(w, h, sr, depth, small, weight, monkeypatch):
+    monkeypatch.setenv("RIV_SEARCH_SMALL", small)
+    frames = _frames(w, h, 4, w + sr)
+    gc, oc = _weighted(w, h, sr, depth, weight)
+    assert _encode(gc, frames) == _oracle(oc, frames)
+
+
+@pytest.mark.parametrize("table", [0, 1])
+def test_batch_of_wide_costs(table):
+    """Every kind of search in one step."""
+    from riv2_b200 import encoder as E
+    from riv2_b200.batch import Batch
+    clips = [(352, 288, 12, 1e7), (352, 288, 12, 0.49), (100, 70, 31, 1e7), (208, 112, 31, 0.49), (64, 48, 7, 1e17),
+             (64, 48, 12, -0.49)]
+    cfgs = [_weighted(w, h, sr, 2, k) for w, h, sr, k in clips]
+    frames = [_frames(w, h, 4, w + sr) for w, h, sr, _ in clips]
+    writers = [E.VecWriter() for _ in clips]
+    b = Batch.new([g for g, _ in cfgs], writers)
+    b.set_tune(100, 4, 128, table)
+    for t in range(4):
+        b.encode_step([f[t] for f in frames], [20 * t] * len(clips))
+    b.finish()
+    b.close()
+    for (_, oc), f, wr in zip(cfgs, frames, writers):
+        assert wr.into_inner() == _oracle(oc, f)

@@ -73,3 +73,15 @@ def test_refused_class_and_full_stacks_go_to_the_host_coder():
     skip[1] = 1  # not coded: nothing to refuse
     got, on_gpu = E.dct_encode_gpu(b, False, skip)
     assert on_gpu and got == E.dct_encode_host(b[skip == 0], False)
+
+
+@pytest.mark.parametrize("intra", [False, True])
+@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 31, 32, 33, 47, 49])
+def test_part_and_cta_edges(n, intra):
+    """A part is two macroblocks (a warp's), a CTA eight parts."""
+    b = _blocks(n, 0.4, 2.0, 100 + n)
+    skip = None if intra else (np.random.default_rng(n).random(n) < 0.3).astype(np.uint8)
+    coded = b if intra else b[skip == 0]
+    want = E.dct_encode_host(coded, intra) if len(coded) else b""
+    got, on_gpu = E.dct_encode_gpu(b, intra, skip, max_symbols=n * 384 * 27)
+    assert on_gpu and got == want

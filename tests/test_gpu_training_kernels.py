@@ -112,3 +112,18 @@ def test_colsum(rows, n, ld):
     want = 1.0 + z[:, :n].double().sum(0)
     # f32 sums: at most `rows` roundings of 2^-24 of the sum of magnitudes
     assert bool(((out.double() - want).abs() <= (1.0 + z[:, :n].double().abs().sum(0)) * rows * 2.0 ** -24 + 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("rows,n,ld", [(1, 32, 32), (513, 32, 32), (1000, 100, 128), (5003, 100, 128), (70001, 32, 32),
+                                       (296 * 512, 32, 32), (296 * 512 + 37, 32, 32), (589824, 32, 32)])
+def test_colsum_is_exact_for_small_integers(rows, n, ld):
+    """Values in -3 .. 3 sum exactly in f32 in any order: a lost or doubled row shows.  296 * 512 rows is
+    where the CTAs reach their largest number (16 bytes a load), 296 * 16 with single elements."""
+    torch, L, dev = _env()
+    g = torch.Generator(device="cpu").manual_seed(rows)
+    z = torch.randint(-3, 4, (rows, ld), generator=g).to(torch.bfloat16).to(dev)
+    z[-1] = 3.0
+    out = torch.ones(n, device=dev)
+    assert L.riv_nn_colsum(z.data_ptr(), ld, C.c_longlong(rows), n, out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out.double(), 1.0 + z[:, :n].double().sum(0))

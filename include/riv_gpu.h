@@ -317,6 +317,9 @@ riv_status riv_test_dct_encode(const int16_t* blocks, uint32_t n, int intra, uin
  * or a class it refuses: RIV_ERR_ENCODING_FAILED). */
 riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, uint32_t n, int intra, uint32_t max_symbols,
                                    uint8_t* out, size_t cap, size_t* len, int* on_gpu);
+/* Test hook (host only, no reference counterpart): the symbols that the GPU codes of a frame of nmb
+ * macroblocks, and the sum of n counts as its kernels form a frame's total. */
+riv_status riv_test_symbol_room(uint64_t nmb, const uint32_t* counts, uint32_t n, uint32_t* room, uint32_t* total);
 /* Test hook (host only, no reference counterpart): what the batch autotuner compares candidates by, of
  * one step's nine stage times (order of riv_batch_counters): dim 0 search, 1 residual, 2 deblock. */
 riv_status riv_test_batch_tune_score(int dim, const float* stage9, float* score);

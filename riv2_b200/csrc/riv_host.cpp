@@ -665,9 +665,7 @@ static void setup_device(riv_encoder* e) {
     deblock_thresholds(e->inter_level, false, e->inter_E, e->inter_I, e->inter_H);
     e->intra_level = deblock_level(quant_step(c.intra_quality));
     deblock_thresholds(e->intra_level, true, e->intra_E, e->intra_I, e->intra_H);
-    // Symbols made on the GPU: room for 512 a macroblock (a key frame at quality 95 of a noisy
-    // 1080p clip has 470, a P-frame 25 to 130); a frame with more goes to the host coder.
-    e->sym_cap = (unsigned)(((size_t)N * 512 + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH);
+    e->sym_cap = sym_room((size_t)N);
     e->sym_mem.alloc(sym_workspace(nullptr, N, e->sym_cap, nullptr));
     // pipeline slots
     int nslots = std::max(1u, c.pipeline_depth);
@@ -2461,7 +2459,7 @@ riv_status riv_test_dct_encode_gpu(const int16_t* blocks, const uint8_t* skip, u
     std::vector<uint8_t> stream;
     try {
         SymFrame f{};
-        f.cap = (unsigned)(((max_symbols ? (size_t)max_symbols : (size_t)n * 512) + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH);
+        f.cap = max_symbols ? (unsigned)(((size_t)max_symbols + SYM_BATCH - 1) / SYM_BATCH * SYM_BATCH) : sym_room(n);
         B.co.alloc((size_t)n * 384 * 2);
         B.sk.alloc(n);
         B.eo.alloc((size_t)n * 3);
@@ -3790,6 +3788,14 @@ riv_status riv_batch_counters(const riv_batch* b, uint64_t* c7, double* stage_us
     }
     if (stage_us10)
         for (int s = 0; s <= BT_NSTAGE; s++) stage_us10[s] = b->timed ? b->stage_us[s] / (double)b->timed : 0.0;
+    return RIV_OK;
+}
+
+riv_status riv_test_symbol_room(uint64_t nmb, const uint32_t* counts, uint32_t n, uint32_t* room, uint32_t* total) {
+    if ((n > 0 && !counts) || !room || !total) return RIV_ERR_FRAME;
+    *room = sym_room((size_t)nmb);
+    *total = 0;
+    for (uint32_t k = 0; k < n; k++) *total = sym_add(*total, counts[k]);
     return RIV_OK;
 }
 

@@ -125,6 +125,19 @@ constexpr int SYM_WORK_WORDS = SYM_TAB + 2 * 427;
 constexpr unsigned SYM_UNIT = 128;          // symbols of a model whose probabilities one warp computes
 constexpr unsigned SYM_OCC_SLACK = (SYM_UNIT - 1) * 427;  // each model's list starts on a unit
 constexpr unsigned SYM_FAIL = 0xffffffffu;  // header word 3: the host coder takes the frame
+// Symbols that the GPU codes of a frame: 512 a macroblock (a key frame at quality 95 of a noisy 1080p
+// clip has 470, a P-frame 25 to 130), in whole batches, and no more than the 31 bits of a stack position
+// in SymFrame::occ tell apart; a frame with more goes to the host coder.
+inline unsigned sym_room(size_t nmb) {
+    const size_t want = (nmb * 512 + SYM_BATCH - 1) / SYM_BATCH, most = 0x7fffffffu / SYM_BATCH;
+    return (unsigned)((want < most ? want : most) * SYM_BATCH);
+}
+// Sums of symbol counts stop at 2^32 - 1, more than any room (a frame of half a million macroblocks can have
+// more: a wrapped total would pass for one that fits).
+__host__ __device__ inline unsigned sym_add(unsigned a, unsigned b) {
+    const unsigned s = a + b;
+    return s < a ? 0xffffffffu : s;
+}
 struct SymFrame {
     const uint8_t* opt_skip;
     const uint8_t* eobs;

@@ -192,7 +192,7 @@ __device__ __forceinline__ void sym_scan_rows(const SymFrame& f, int group) {
     unsigned* c = f.tot + row;
     unsigned sum = 0;
 #pragma unroll 16
-    for (int p = p0; p < p1; p++) sum += c[(size_t)p * SYM_ROWS];
+    for (int p = p0; p < p1; p++) sum = sym_add(sum, c[(size_t)p * SYM_ROWS]);
     sums[w][lane] = sum;
     __syncthreads();
     if (w == 0) {
@@ -200,7 +200,7 @@ __device__ __forceinline__ void sym_scan_rows(const SymFrame& f, int group) {
         for (int q = 0; q < 32; q++) {
             const unsigned x = sums[q][lane];
             sums[q][lane] = run;
-            run += x;
+            run = sym_add(run, x);
         }
         unsigned b = 0;
         if (row < SY_MODELS) {

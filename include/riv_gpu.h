@@ -150,7 +150,8 @@ riv_status riv_last_recon(riv_encoder* enc, uint8_t* y, uint8_t* u, uint8_t* v);
  * frame at pipeline_depth 0 or with per-frame stats, else one in 8), microseconds: [0] rgb->yuv
  * [1] integer-SAD table (plain form) or proposal network (learned form) [2] search/mode
  * (the wavefront, or the learned forms' parallel search + mode decision) [3] predict [4] aq
- * [5] residual [6] deblock [7] compact [8] total */
+ * [5] residual [6] deblock [7] coefficient symbols (within [2] where the next frame's search
+ * launch packs the blocks for the host's coder) [8] total */
 riv_status riv_last_kernel_times(riv_encoder* enc, float* us9);
 
 /* Cumulative counters since riv_encoder_new: us9 = per-stage GPU time summed over all
@@ -172,7 +173,7 @@ riv_status riv_host_times(riv_encoder* enc, double* ms6);
  * encoded together one step at a time.  A step takes at most one frame per clip; its GPU work
  * is one launch per stage over every clip of the step (conversion, SAD tables, the search --
  * one cooperative launch in which each clip's CTAs run its MB rows as a wavefront --,
- * prediction, AQ mean, residual, deblock, compaction), so the clips fill the SMs that one
+ * prediction, AQ mean, residual, deblock, symbols, rANS), so the clips fill the SMs that one
  * clip's wavefront leaves idle; each clip's entropy coding and records then run as in
  * riv_encode_frame, on thread pools the clips share.  Every clip's stream is byte-identical
  * to what riv_encoder_new + riv_encode_frame + riv_finish write for that clip alone.

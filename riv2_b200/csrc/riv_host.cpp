@@ -303,8 +303,8 @@ struct HostBuf {
     T* as() const { return (T*)p; }
 };
 
-// Pinned host memory mapped into the device address space: kernels write the frame's
-// side info and compacted coefficients straight into it.
+// Pinned host memory mapped into the device address space: kernels write a frame's header words
+// straight into it.
 struct MappedBuf {
     void* h = nullptr;
     void* d = nullptr;
@@ -326,7 +326,7 @@ struct MappedBuf {
 constexpr int NPAR = 3;  // rotation depth of the per-frame device buffers
 constexpr uint64_t TIMING_SAMPLE = 8;  // pipelined frames carry stage timing events one in this many
 enum { EV_START, EV_YUV, EV_S0, EV_TABLE, EV_SEARCH, EV_PRED, EV_AQ, EV_RES, EV_DEBLOCK, EV_K0, EV_COMPACT, EV_NET0, EV_NET1, EV_N };
-static const int NSTAGE = 8;  // rgb->yuv, table, search, predict, aq, residual, deblock, compact (+ total)
+static const int NSTAGE = 8;  // rgb->yuv, table, search, predict, aq, residual, deblock, symbols (+ total)
 
 struct Slot {
     // frame output on the device; dpacked: rANS stacks, or truncated coefficient blocks
@@ -392,7 +392,7 @@ struct riv_encoder {
     // the copies of every later frame in flight
     cudaStream_t R = nullptr;
     // cross-stream reuse guards: cur[k] free (its residual is done), mbout[k] and the
-    // coefficient buffers free (their compaction is done)
+    // coefficient buffers free (their symbols are made, or their blocks packed)
     cudaEvent_t ev_cur_free[NPAR] = {}, ev_mbout_free[NPAR] = {}, ev_coef_free[NPAR] = {};
     // the last search launch: input conversion waits for it, so that it never holds SMs the
     // next cooperative search launch needs
@@ -820,7 +820,7 @@ static void reconstruct_now(riv_encoder* e, Job& j, const ResidualParams& rp, in
                             const uint8_t* mask, uint8_t* recon) {
     Slot& s = e->slots[j.slot];
     cudaStream_t S = e->S;
-    CK(cudaStreamWaitEvent(S, e->ev_coef_free[j.ck], 0));  // compaction of the frame NPAR back
+    CK(cudaStreamWaitEvent(S, e->ev_coef_free[j.ck], 0));  // tail of the frame NPAR back
     e->launches += 1 + (level > 0 ? 1 : 0);
     CK(launch_residual(rp, e->NMB, S));
     mark(e, j, EV_RES, S);
@@ -916,10 +916,10 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
     MbOut* mbo = e->mboutb[ck].as<MbOut>();
     const bool defer_this = j.type == 2 && e->defer_ok;
     if (j.type == 1) flush_pending(e);  // key frames reconstruct immediately
-    // kernels per frame: rgb->yuv, (search, predict, 3 x aq), residual, deblock, scan + pack
+    // kernels per frame counted here: rgb->yuv, (table, search, predict, 3 x aq)
     const int p_launches = e->learned ? (c.encode_form == RIV_FORM_LEARNED ? 8 : 0) + 3
                                       : 1 + (e->splan.table && !e->splan.fused ? 1 : 0) + (e->splan.fast ? 0 : 4);
-    e->launches += (src == 2 ? 0 : 1) + (j.type == 2 ? p_launches : 0);  // + residual / deblock / compaction below
+    e->launches += (src == 2 ? 0 : 1) + (j.type == 2 ? p_launches : 0);  // + residual, deblock and symbols where they are launched
     if (src == 0) e->h2d_bytes += (uint64_t)c.display_width * c.display_height * 3;
     if (src == 2) e->h2d_bytes += e->yuv_bytes;
     // ---- input conversion on Y, overlapping the previous frame's main chain; cur[ck] is
@@ -1012,8 +1012,8 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
         // coded MVs of this frame become next frame's temporal predictors
         const int cn = e->coded_cur ^ 1;
         sp.coded_out = e->coded[cn].as<int8_t>();
-        // prediction, variances and ln inside the search launch (plain fused form), or inside the
-        // learned forms' parallel search (their launch also folds the mean)
+        // prediction, variances and ln inside the search launch: the kinds with a loader, or the
+        // learned forms' parallel search (either launch also folds the mean)
         const bool aq_in_search = e->splan.fast || e->learned;
         if (aq_in_search) {  // prediction, variances and ln inside the search launch
             sp.pred = e->predb[ck].as<uint8_t>();
@@ -1041,10 +1041,10 @@ static void submit_gpu(riv_encoder* e, Job& j, int src, const void* a, const voi
             sp.c_packed = ps.dpacked.as<int16_t>();
             sp.c_peobs = ps.dpeobs.as<uint8_t>();
             sp.c_hdr = ps.hdr.dev<uint32_t>();
-            CK(cudaStreamWaitEvent(S, e->ev_coef_free[e->pend.ck], 0));  // compaction of the frame NPAR back
+            CK(cudaStreamWaitEvent(S, e->ev_coef_free[e->pend.ck], 0));  // tail of the frame NPAR back
         }
         e->pend.active = false;
-        CK(cudaStreamWaitEvent(S, e->ev_mbout_free[ck], 0));  // compaction of the frame NPAR back
+        CK(cudaStreamWaitEvent(S, e->ev_mbout_free[ck], 0));  // tail of the frame NPAR back
         if (e->learned) {
             CK((cudaError_t)launch_learned(sp, c.encode_form == RIV_FORM_LEARNED ? e->nn_o[nbuf].as<float>() : nullptr,
                                            (int)c.proposal_margin, 2.2f, e->lmv.p, e->lcount.as<unsigned>(),

@@ -84,7 +84,7 @@ struct SearchParams {
     int cta0;         // first CTA of this clip in a multi-clip launch (0 for a single clip)
     int row_helpers;  // row CTAs run worker groups before their row starts and after it ends
     unsigned* tflag;  // fused table: per-MB flag = tag once its table row is written; nullptr = precomputed
-    // Prediction and AQ inside the search launch (band + table instantiations): nullptr lnv =
+    // Prediction and AQ inside the search launch (where a loader runs): nullptr lnv =
     // done by the separate predict / AQ kernels.
     uint8_t* pred;             // planar YUV prediction out
     uint2* varsum;             // per MB (sum, sum of squares) of the predicted luma

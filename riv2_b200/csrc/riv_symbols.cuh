@@ -527,8 +527,13 @@ __global__ void __launch_bounds__(SY_MODEL_THREADS, 8) k_sym_model(SymFrame f) {
 }
 
 static inline int sym_part_ctas(int nmb) { return (nmb + SY_MBS * SY_WARPS - 1) / (SY_MBS * SY_WARPS); }
-// CTAs of the units of a frame: a warp takes about two when a macroblock has 64 modelled symbols
-static inline int sym_model_ctas(int nmb) { return std::max(1, std::min(8 * 148, nmb / 16)); }
+// CTAs of the units of a frame: a warp takes about two when a macroblock has 64 modelled symbols.  Every
+// model that occurs has a unit, however small the frame, so no fewer than a warp a model (by macroblocks
+// alone a 64x48 key frame had one CTA for its 300 units, and 132 us a frame in flight went to 80).
+static inline int sym_model_ctas(int nmb) {
+    constexpr int warps = SY_MODEL_THREADS / 32;
+    return std::max((SY_MODELS + warps - 1) / warps, std::min(8 * 148, nmb / 16));
+}
 
 size_t sym_workspace(SymFrame* f, int nmb, unsigned cap, void* p) {
     size_t at = 0;

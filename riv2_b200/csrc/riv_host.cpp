@@ -416,6 +416,7 @@ struct riv_encoder {
     DevBuf lcindex, lcoffset;  // the search launch's compaction scan
     DevBuf sym_mem;                     // working memory of launch_symbols (one frame at a time, in stream order)
     unsigned sym_cap = 0;               // symbols a frame may have there, and its slot's stacks
+    int sym_min = 0;                    // frames of fewer macroblocks go to the host's coder (setup_device)
     DevBuf mvbits, logfix, expfix, ytab, ctab, newcost, newcost32;
     bool small_costs = false;
     int multi_kind = 0;     // in a batch: its kind of search without a SAD table
@@ -666,6 +667,14 @@ static void setup_device(riv_encoder* e) {
     e->intra_level = deblock_level(quant_step(c.intra_quality));
     deblock_thresholds(e->intra_level, true, e->intra_E, e->intra_I, e->intra_H);
     e->sym_cap = sym_room((size_t)N);
+    // On frames of few macroblocks the host lists and models symbols in less time than the symbol kernels'
+    // launches take.  ms a frame with the host's coder and with the kernels; nothing in flight: 0.271 and 0.284
+    // at 24 macroblocks, 0.317 and 0.299 at 48; in flight, where the host's threads take several frames at once
+    // and the kernels one: 0.068 and 0.074-0.097 at 99, 0.085 and 0.078 at 150 (parallel form; the plain form's
+    // P-frames are packed by their search launches), key frames only 0.083 and 0.125 at 240, 0.106 and 0.080 at 396.
+    const bool all_key = c.keyframe_mode == RIV_KEYFRAME_ALL_INTRA ||
+                         (c.keyframe_mode == RIV_KEYFRAME_FIXED && c.keyframe_interval == 1);
+    e->sym_min = c.pipeline_depth <= 1 ? 40 : all_key ? 320 : 128;
     e->sym_mem.alloc(sym_workspace(nullptr, N, e->sym_cap, nullptr));
     // pipeline slots
     int nslots = std::max(1u, c.pipeline_depth);
@@ -792,9 +801,11 @@ static void frame_tail(riv_encoder* e, Job& j, bool compacted = false) {
     mark(e, j, EV_K0, K);
     j.sym = false;
     if (!compacted) {
-        e->launches += 5;
-        CK(launch_symbols(sym_frame(e, ck, j.type == 1, s), K));
-        j.sym = true;
+        SymFrame f = sym_frame(e, ck, j.type == 1, s);
+        j.sym = N >= e->sym_min;
+        if (!j.sym) f.cap = 0;  // blocks packed for the host coder
+        e->launches += j.sym ? 5 : 3;
+        CK(launch_symbols(f, K));
     }
     CK(cudaEventRecord(e->ev_coef_free[ck], K));
     CK(cudaEventRecord(e->ev_mbout_free[ck], K));
@@ -1553,7 +1564,7 @@ static riv_status pump(riv_encoder* e, bool block_front, bool block_write) {
 // kernels would delay it) and behind the first tail's copies (their stacks take the packed blocks'
 // place): 16 frames of 1080p took 13.3 ms without, 11.7 ms with this.
 static void retail_last_frames(riv_encoder* e) {
-    if (!e->pend.active) return;
+    if (!e->pend.active || e->NMB < e->sym_min) return;
     for (auto& j : e->jobs) {
         if (j.index + NPAR <= e->pend.index || j.state != 0 || !j.tail_done || !j.deferred || j.sym) continue;
         Slot& s = e->slots[j.slot];

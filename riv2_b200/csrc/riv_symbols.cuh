@@ -556,11 +556,13 @@ size_t sym_workspace(SymFrame* f, int nmb, unsigned cap, void* p) {
     }
     return at;
 }
+// With no room (cap 0) the blocks are packed for the host coder.
 int launch_symbols(const SymFrame& f, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     k_sym_count<<<sym_part_ctas(f.nmb), 32 * SY_WARPS, 0, st>>>(f);
     k_sym_scan<<<SYM_ROWS / 32, 1024, 0, st>>>(f);
     k_sym_emit<<<sym_part_ctas(f.nmb), 32 * SY_WARPS, 0, st>>>(f);
+    if (f.cap == 0) return (int)cudaGetLastError();
     k_sym_chain<<<SY_MODELS, SY_CHAIN_THREADS, 0, st>>>(f);
     k_sym_model<<<sym_model_ctas(f.nmb), SY_MODEL_THREADS, 0, st>>>(f);
     return (int)cudaGetLastError();

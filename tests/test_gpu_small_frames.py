@@ -1,0 +1,31 @@
+"""Frames of few macroblocks: which coder lists and models their coefficients, at both sides of each line
+(40 with nothing in flight, 128 with frames in flight, 320 for key frames only), streams against the
+oracle."""
+import pytest
+
+from test_gpu_search_direct import _configs, _frames, _oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,depth,interval,on_gpu", [
+    (16, 16, 0, 1000, False), (208, 48, 0, 1000, False), (160, 64, 0, 1000, True), (208, 48, 1, 1, False),
+    (160, 64, 1, 1, True), (2032, 16, 4, 1000, False), (256, 128, 4, 1000, True), (464, 176, 4, 1, False),
+    (320, 256, 4, 1, True), (64, 48, 8, 3, False)])
+def test_route_and_stream(w, h, depth, interval, on_gpu):
+    from riv2_b200 import encoder as E
+    gc, oc = _configs(w, h, 16, depth)
+    gc = gc.with_keyframe_interval(E.KeyframeInterval.fixed(interval))
+    oc.keyframe_interval = interval
+    frames = _frames(w, h, 7, w + h)
+    wr = E.VecWriter()
+    enc = E.Encoder.new(gc, wr)
+    for t, f in enumerate(frames):
+        enc.encode_frame(E.Frame(f, w, h, 20 * t))
+    enc.finish()
+    launches = enc.counters()["launches"]
+    enc.close()
+    assert wr.into_inner() == _oracle(oc, frames)
+    # conversion, residual, deblock; a search; the five symbol kernels, or three that pack the blocks
+    keys = -(-7 // interval)
+    assert launches == 7 * (8 if on_gpu else 6) + (7 - keys)

@@ -155,6 +155,7 @@ struct SymFrame {
     int16_t* packed;  // when the host coder takes the frame: truncated blocks and their EOBs
     uint8_t* peobs;
     uint32_t* hdr;    // mapped host words: coded MBs, coefficients, [2] = *status (not nullptr), symbols
+                      // (SYM_FAIL: host coder), [5] = their number in either case
     const unsigned* status;
     uint32_t* nsym;   // not nullptr: the symbols once more, on the device
 };

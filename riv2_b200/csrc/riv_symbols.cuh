@@ -217,6 +217,7 @@ __device__ __forceinline__ void sym_scan_rows(const SymFrame& f, int group) {
             f.hdr[0] = coded;
             f.hdr[1] = coefs;
             f.hdr[3] = ok ? syms : SYM_FAIL;
+            f.hdr[5] = syms;
             if (f.nsym != nullptr) *f.nsym = ok ? syms : SYM_FAIL;
             if (f.status != nullptr) f.hdr[2] = *(volatile const unsigned*)f.status;
         }

@@ -213,3 +213,51 @@ def test_batch_of_wide_costs(table):
     b.close()
     for (_, oc), f, wr in zip(cfgs, frames, writers):
         assert wr.into_inner() == _oracle(oc, f)
+
+
+@pytest.mark.parametrize("w,h,sr", [(1136, 2400, 31), (1360, 2400, 64)])
+def test_more_rows_than_ctas(w, h, sr):
+    """150 macroblock rows on one CTA an SM: the last rows are a CTA's second, with a band and with a ring."""
+    from riv2_b200 import encoder as E
+    p = E.search_plan(w, h, sr)
+    assert p["row_ctas"] < h // 16 and p["band"] == (sr == 31) and not p["table"]
+    frames = _frames(w, h, 3, w + sr)
+    gc, oc = _configs(w, h, sr, 4)
+    assert _encode(gc, frames) == _oracle(oc, frames)
+
+
+# zero-MV threshold, predictor threshold, weight of the MV costs
+STOPS = [(800, 0, 0.49), (0, 1500, 0.49), (3000, 6000, 0.49), (0, 0, 0.0), (500, 900, 0.0)]
+
+
+def _stops(w, h, sr, depth, zero, predictor, weight):
+    gc, oc = _weighted(w, h, sr, depth, weight)
+    oc.me_zero_mv_threshold, oc.me_predictor_threshold = zero, predictor
+    return gc._with(me_zero_mv_threshold=zero, me_predictor_threshold=predictor), oc
+
+
+@pytest.mark.parametrize("zero,predictor,weight", STOPS)
+@pytest.mark.parametrize("w,h,sr", [(352, 288, 12), (357, 131, 16), (352, 288, 31), (3856, 32, 31), (640, 48, 102)])
+def test_early_stops_and_free_vectors(w, h, sr, zero, predictor, weight):
+    """Searches that end at the zero MV or at a predictor, and MV costs of 0."""
+    frames = _frames(w, h, 4, w + sr)
+    gc, oc = _stops(w, h, sr, 4, zero, predictor, weight)
+    assert _encode(gc, frames) == _oracle(oc, frames)
+
+
+@pytest.mark.parametrize("table", [0, 1])
+def test_batch_early_stops_and_free_vectors(table):
+    from riv2_b200 import encoder as E
+    from riv2_b200.batch import Batch
+    clips = [(352, 288, 12) + s for s in STOPS] + [(100, 70, 31) + s for s in STOPS]
+    cfgs = [_stops(w, h, sr, 2, *s) for w, h, sr, *s in clips]
+    frames = [_frames(w, h, 4, w + sr) for w, h, sr, *_ in clips]
+    writers = [E.VecWriter() for _ in clips]
+    b = Batch.new([g for g, _ in cfgs], writers)
+    b.set_tune(75, 8, 64, table)
+    for t in range(4):
+        b.encode_step([f[t] for f in frames], [20 * t] * len(clips))
+    b.finish()
+    b.close()
+    for (_, oc), f, wr in zip(cfgs, frames, writers):
+        assert wr.into_inner() == _oracle(oc, f)
